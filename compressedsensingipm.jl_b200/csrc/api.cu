@@ -96,20 +96,6 @@ static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in
     }
 }
 
-// Solver-order plane map: (re, im, kind, src) of the planes i = 0 and i = M1,
-// entry (p*N3 + k)*N2 + j, with re / im as solver-order tail indices.
-static __global__ void plane_map_kernel(Geom g, int4* __restrict__ pm) {
-    const int64_t per = (int64_t)g.n2 * g.n3;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < 2 * per;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int p = (int)(idx / per);
-        const int64_t r = idx - p * per;
-        const int k = (int)(r / g.n2), j = (int)(r % g.n2);
-        const MapEntry e = decode(g, p ? g.m1 : 0, j, k);
-        pm[idx] = make_int4((int)sol_tail(g, e.re), e.kind == KIND_VERT ? -1 : (int)sol_tail(g, e.im), e.kind, e.src);
-    }
-}
-
 cudaError_t to_solver_order(const Geom& g, const double* ref, double* sol, cudaStream_t st) {
     solver_order_kernel<true><<<ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st>>>(g, ref, sol);
     return cudaGetLastError();
@@ -477,25 +463,17 @@ int profile_impl(csipm_handle h, FftOperator<T>& op, const T* x, T* D, T* q, int
         return CSIPM_OK;
     };
     int r = 0;
-    if (g.dim == 1 && op.l1P) {
+    if (g.dim == 1) {
         const double M = (double)g.m1;
-        r = timeit([&] { return l1d_first(op, x, nullptr, st); }, 2 * w * N + cw * M,
+        r = timeit([&] { return l1d_first(op, x, nullptr, st); }, w * N + cw * M,
                    f32 ? "fp32 1D lines: gather+C2R+inverse" : "1D lines: gather+C2R+inverse");
         if (r) return r;
         r = timeit([&] { return mask ? l1d_row<T, IN_SPEC, OUT_SPEC, true>(op, ra.scale, nullptr, nullptr, nullptr, st)
                                      : l1d_row<T, IN_SPEC, OUT_SPEC, false>(op, ra.scale, nullptr, nullptr, nullptr, st); },
                    2 * cw * M + maskb, f32 ? "fp32 1D rows: inverse+mask+forward" : "1D rows: inverse+mask+forward");
         if (r) return r;
-        r = timeit([&] { return l1d_lines_forward(op, nullptr, st); }, 2 * cw * M,
-                   f32 ? "fp32 1D lines: forward" : "1D lines: forward");
-        if (r) return r;
-        r = timeit([&] { return l1d_post(op, ecg, nullptr, st); }, 2 * cw * M + 3 * w * N,
-                   f32 ? "fp32 1D R2C+scatter+CG" : "1D R2C+scatter+CG");
-        if (r) return r;
-    } else if (g.dim == 1) {
-        r = timeit([&] { return mask ? run_row<T, IN_GATHER, OUT_SCATTER, true>(op, ra, x, ecg, st)
-                                     : run_row<T, IN_GATHER, OUT_SCATTER, false>(op, ra, x, ecg, st); },
-                   4 * w * N + maskb, f32 ? "fp32 row: gather+FFT+scatter+CG" : "row: gather+C2R+mask+R2C+scatter+CG");
+        r = timeit([&] { return l1d_last(op, ecg, nullptr, st); }, cw * M + 3 * w * N,
+                   f32 ? "fp32 1D lines: R2C+scatter+CG" : "1D lines: forward+R2C+scatter+CG");
         if (r) return r;
     } else {
         // the product's order: beta-side passes along dim 2 (solver-order
@@ -513,8 +491,8 @@ int profile_impl(csipm_handle h, FftOperator<T>& op, const T* x, T* D, T* q, int
                        2 * cw * Nh, f32 ? "fp32 inverse dim3" : "inverse dim3");
             if (r) return r;
         }
-        r = timeit([&] { return mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, (const double*)nullptr, none, st)
-                                     : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, (const double*)nullptr, none, st); },
+        r = timeit([&] { return mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, st)
+                                     : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, st); },
                    2 * cw * Nh + maskb, f32 ? "fp32 row: C2R+mask+R2C dim1" : "row: C2R+mask+R2C dim1");
         if (r) return r;
         if (g.dim == 3) {
@@ -1005,15 +983,7 @@ int csipm_create(const csipm_problem* prob, const csipm_options* opt_in, csipm_h
     if (e != cudaSuccess) return bail(CSIPM_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e));
     if (h->opt.layout == 0 && solver_order_ok(h->op64) && (!mixed || solver_order_ok(h->op32))) {
         if (!h->alloc(&h->bs, n_)) return bail(CSIPM_ERR_OOM, h->err);
-        // plane map: the entries of the planes i = 0 and i = M1 in solver
-        // order, built on the device (no host loop, no copy)
-        const Geom& g = h->g;
-        const size_t np = (size_t)2 * g.n2 * g.n3;
-        if (!h->alloc(&h->pmap, np)) return bail(CSIPM_ERR_OOM, h->err);
-        plane_map_kernel<<<ew_blocks((long long)np), EW_THREADS, 0, h->stream>>>(g, h->pmap);
-        h->op64.pmap = h->pmap;
-        h->op32.pmap = h->pmap;
-        if (cudaGetLastError() != cudaSuccess || to_solver_order(h->g, h->b, h->bs, h->stream) != cudaSuccess)
+        if (to_solver_order(h->g, h->b, h->bs, h->stream) != cudaSuccess)
             return bail(CSIPM_ERR_CUDA, "solver-order set-up failed");
         h->sorder = true;
     }

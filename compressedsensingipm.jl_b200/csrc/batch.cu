@@ -9,7 +9,7 @@
 // PassArgs of its FFT passes (run-time plans: any length) — and launches
 // every element kernel and every FFT pass once with gridDim.y = instances.
 // Block (x, y) works on instance y; reductions complete per instance
-// (RedWorkspace::xonly); the persistent Stockham passes walk each instance's
+// (RedWorkspace::xonly); the run-time-plan passes walk each instance's
 // tiles with the same gridDim.x blocks.  An instance that has stopped
 // (converged, max_iter, non-finite) returns at once from every kernel (its
 // control block's status, or its CG scalars' done flag inside a CG loop).
@@ -17,7 +17,7 @@
 // The method is csipm_solve's FP64 path — the same kernel bodies, the same
 // device stop test and forcing term — in the reference packing, so each
 // instance takes csipm_solve's iterates up to the order of floating-point
-// sums (the FFT passes are the Stockham kernels, not the two-level ones).
+// sums (the FFT passes are the run-time-plan kernels (passes.cuh), not the two-level ones).
 // The reference has no counterpart: it solves one recovery per call
 // (src/CompressedSensingIPM.jl:31-36).
 #include <chrono>
@@ -54,7 +54,7 @@ struct BPass {
     const double* src;
     Epi epi;
     const double2* twN;
-    int P, Q, RB, TB;
+    int P, Q;
 };
 
 // ------------------------------------------------------------------ element kernels
@@ -206,34 +206,42 @@ __global__ void __launch_bounds__(EW_THREADS) bk_beta_step(const BInst* __restri
 }
 
 // ------------------------------------------------------------------ FFT pass kernels
-template <int TB, bool INV, int IN, int OUT, class Epi>
-__global__ void __launch_bounds__(256) bk_strided(const BPass<Epi>* __restrict__ B) {
-    const BPass<Epi>& e = B[blockIdx.y];
-    strided_pass_kernel_body<double, TB, INV, IN, OUT, double, Epi>(e.a, e.src, e.epi);
-}
+// One block size for all instances of a batch (each brings its own plan and
+// tile layout).
+constexpr int BATCH_THREADS = 256;
 
-template <int IN, int OUT, bool MASK, class Epi>
-__global__ void __launch_bounds__(256) bk_row(const BPass<Epi>* __restrict__ B) {
+template <bool INV, int IN, int OUT, class Epi>
+__global__ void __launch_bounds__(BATCH_THREADS) bk_strided(const BPass<Epi>* __restrict__ B) {
     const BPass<Epi>& e = B[blockIdx.y];
-    row_pass_kernel_body<double, IN, OUT, MASK, double, Epi>(e.a, e.src, e.epi);
-}
-
-template <class Epi>
-__global__ void __launch_bounds__(256) bk_l1d_first(const BPass<Epi>* __restrict__ B) {
-    const BPass<Epi>& e = B[blockIdx.y];
-    l1d_first_kernel_body<double, double>(e.a, e.src, e.twN, e.P, e.Q, e.TB);
+    const PassArgs<double>& a = e.a;
+    strided_pass_kernel_body<double, INV, IN, OUT, double, Epi>(a, e.src, e.epi);
 }
 
 template <bool MASK, class Epi>
-__global__ void __launch_bounds__(256) bk_l1d_row(const BPass<Epi>* __restrict__ B) {
-    const BPass<Epi>& e = B[blockIdx.y];
-    l1d_row_kernel_body<double, IN_SPEC, OUT_SPEC, MASK>(e.a, e.twN, e.P, e.Q, e.RB);
+__global__ void __launch_bounds__(BATCH_THREADS) bk_row(const BPass<Epi>* __restrict__ B) {
+    const PassArgs<double>& a = B[blockIdx.y].a;
+    row_pass_kernel_body<double, IN_SPEC, OUT_SPEC, MASK>(a);
 }
 
 template <class Epi>
-__global__ void __launch_bounds__(256) bk_l1d_post(const BPass<Epi>* __restrict__ B) {
+__global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_first(const BPass<Epi>* __restrict__ B) {
     const BPass<Epi>& e = B[blockIdx.y];
-    l1d_post_kernel_body<double, Epi>(e.a, e.twN, e.epi);
+    const PassArgs<double>& a = e.a;
+    l1d_first_kernel_body<double, double>(a, e.src, e.twN, e.P);
+}
+
+template <bool MASK, class Epi>
+__global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_row(const BPass<Epi>* __restrict__ B) {
+    const BPass<Epi>& e = B[blockIdx.y];
+    const PassArgs<double>& a = e.a;
+    l1d_row_kernel_body<double, IN_SPEC, OUT_SPEC, MASK>(a, e.twN, e.P, e.Q);
+}
+
+template <class Epi>
+__global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_last(const BPass<Epi>* __restrict__ B) {
+    const BPass<Epi>& e = B[blockIdx.y];
+    const PassArgs<double>& a = e.a;
+    l1d_last_kernel_body<double, Epi>(a, e.twN, e.P, e.Q, e.epi);
 }
 
 // ------------------------------------------------------------------ host side
@@ -249,7 +257,6 @@ struct BProduct {
     // device tables, one per pass (up to 5)
     BPass<Epi>* tab[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     // launch shapes
-    int tb[5] = {0, 0, 0, 0, 0};
     size_t smem[5] = {0, 0, 0, 0, 0};
     int gx[5] = {0, 0, 0, 0, 0};
     int npass = 0;
@@ -301,7 +308,7 @@ struct BatchState {
 int batch_kind(csipm_handle h) {
     if (h->g.dim == 3) return PK_3D;
     if (h->g.dim == 2) return PK_2D;
-    return h->op64.l1P ? PK_1DL : PK_1D;
+    return h->g.m1 > L1D_MIN_M ? PK_1DL : PK_1D;   // the split classes of a batch (internal.h)
 }
 
 // Persistent-pass grid: the batch shares one wave of the kernel's CTAs
@@ -330,105 +337,52 @@ int build_product(BatchState& B, BProduct<Epi>& P, const std::vector<csipm_handl
     P.kind = batch_kind(hs[0]);
     P.mask = hs[0]->op64.maskw != nullptr;
     std::vector<std::vector<BPass<Epi>>> t;
-    const double C = sizeof(double2);
-    auto add = [&](int pass, const PassArgs<double>& a, const double* src, const Epi& e, const double2* twN, int Pp,
-                   int Qq, int RB, int TB = 0) {
+    // an instance's pass: its tile at the handle's lines (or rows) per CTA,
+    // laid out for the batch's block size
+    auto add = [&](int pass, const FftOperator<double>& op, PassArgs<double> a, const PassCfg& cfg, PassKind kind,
+                   const double* src, const Epi& e, const int* sk) -> bool {
         if ((int)t.size() <= pass) t.resize(pass + 1);
+        PassCfg c;
+        const int n = cfg.tiles * cfg.tb;
+        for (int tb = cfg.tb; tb >= 1; tb /= 2) {
+            lay_pass(a.pl, a.Ltab, tb, n, kind, BATCH_THREADS, sizeof(double2), &c);
+            if (c.smem <= FftOperator<double>::smem_limit()) break;
+        }
+        FftOperator<double>::tile_args(c, &a);
+        a.skip = sk;
         BPass<Epi> bp{};
         bp.a = a;
         bp.src = src;
         bp.epi = e;
-        bp.twN = twN;
-        bp.P = Pp;
-        bp.Q = Qq;
-        bp.RB = RB;
-        bp.TB = TB;
+        bp.twN = op.tw1;
+        bp.P = op.l1P;
+        bp.Q = op.l1Q;
         t[pass].push_back(bp);
+        P.smem[pass] = std::max(P.smem[pass], c.smem);
+        P.gx[pass] = std::max(P.gx[pass], c.tiles);
+        return cfg.pp && c.smem <= FftOperator<double>::smem_limit();
     };
     for (int k = 0; k < K; ++k) {
         FftOperator<double>& op = hs[k]->op64;
-        const Geom& g = op.g;
-        const double sc = 1.0 / (2.0 * (double)g.N);
-        EpiStore<double> none{nullptr};
-        (void)none;
-        if (P.kind == PK_1D) {
-            PassArgs<double> ra = op.row_args(sc, nullptr, nullptr);
-            ra.skip = skip[k];
-            add(0, ra, x[k], epi[k], nullptr, 0, 0, 0);
-            P.smem[0] = std::max(P.smem[0], op.row_cfg.smem);
-            P.gx[0] = std::max(P.gx[0], op.row_cfg.tiles);
-        } else if (P.kind == PK_1DL) {
-            PassArgs<double> a0 = l1d_args(op, false, 1.0, skip[k]);
-            add(0, a0, x[k], epi[k], op.tw1, op.l1P, op.l1Q, op.l1RB, op.l1TB);
-            P.smem[0] = std::max(P.smem[0], (size_t)(2 * op.l1Q * op.l1TB * C));
-            P.gx[0] = std::max(P.gx[0], (op.l1P + op.l1TB - 1) / op.l1TB);
-            PassArgs<double> a1 = l1d_args(op, true, sc, skip[k]);
-            add(1, a1, nullptr, epi[k], op.tw1, op.l1P, op.l1Q, op.l1RB);
-            P.smem[1] = std::max(P.smem[1], (size_t)(2 * op.l1P * op.l1RB * C));
-            P.gx[1] = std::max(P.gx[1], (op.l1Q + op.l1RB - 1) / op.l1RB);
-            PassArgs<double> a2 = l1d_args(op, false, 1.0, skip[k]);
-            a2.tw_in_smem = op.q_cfg.tw_in_smem;
-            a2.n_lines = op.l1P;
-            a2.n_outer = 1;
-            a2.so = 0;
-            a2.sx = op.l1P;
-            a2.jk_mode = 2;
-            add(2, a2, nullptr, epi[k], op.tw1, op.l1P, op.l1Q, op.l1RB);
-            P.tb[2] = P.tb[2] ? std::min(P.tb[2], op.q_cfg.tb) : op.q_cfg.tb;
-            P.smem[2] = std::max(P.smem[2], op.q_cfg.smem);
-            P.gx[2] = std::max(P.gx[2], op.q_cfg.tiles);
-            PassArgs<double> a3 = l1d_args(op, false, 1.0, skip[k]);
-            add(3, a3, nullptr, epi[k], op.tw1, op.l1P, op.l1Q, op.l1RB);
-            P.gx[3] = std::max(P.gx[3], std::min(1024, (g.m1 / 2 + 1 + 255) / 256));
+        const double sc = 1.0 / (2.0 * (double)op.g.N);
+        const int* sk = skip[k];
+        bool ok = true;
+        if (op.g.dim == 1) {
+            ok = add(0, op, l1d_args(op, 0, 1.0, sk), op.f_cfg, PASS_LINES, x[k], epi[k], sk) &&
+                 add(1, op, l1d_args(op, 1, sc, sk), op.p_cfg, PASS_PAIRS, nullptr, epi[k], sk) &&
+                 add(2, op, l1d_args(op, 2, 1.0, sk), op.q_cfg, PASS_PAIRS, nullptr, epi[k], sk);
         } else {
-            PassArgs<double> a2 = op.strided_args(2);
-            a2.skip = skip[k];
-            PassArgs<double> ra = op.row_args(sc, nullptr, nullptr);
-            ra.skip = skip[k];
+            const PassArgs<double> a2 = op.strided_args(2), ra = op.row_args(sc, nullptr, nullptr);
             int pass = 0;
-            add(pass, a2, x[k], epi[k], nullptr, 0, 0, 0);   // gather + inverse dim 2
-            P.tb[pass] = P.tb[pass] ? std::min(P.tb[pass], op.s2_cfg.tb) : op.s2_cfg.tb;
-            P.gx[pass] = std::max(P.gx[pass], op.s2_cfg.tiles);
-            ++pass;
-            if (P.kind == PK_3D) {
-                PassArgs<double> a3 = op.strided_args(3);
-                a3.skip = skip[k];
-                add(pass, a3, nullptr, epi[k], nullptr, 0, 0, 0);   // inverse dim 3
-                P.tb[pass] = P.tb[pass] ? std::min(P.tb[pass], op.s3_cfg.tb) : op.s3_cfg.tb;
-                P.gx[pass] = std::max(P.gx[pass], op.s3_cfg.tiles);
-                ++pass;
-            }
-            add(pass, ra, nullptr, epi[k], nullptr, 0, 0, 0);   // rows
-            P.smem[pass] = std::max(P.smem[pass], op.row_cfg.smem);
-            P.gx[pass] = std::max(P.gx[pass], op.row_cfg.tiles);
-            ++pass;
-            if (P.kind == PK_3D) {
-                PassArgs<double> a3 = op.strided_args(3);
-                a3.skip = skip[k];
-                add(pass, a3, nullptr, epi[k], nullptr, 0, 0, 0);   // forward dim 3
-                P.tb[pass] = P.tb[pass] ? std::min(P.tb[pass], op.s3_cfg.tb) : op.s3_cfg.tb;
-                P.gx[pass] = std::max(P.gx[pass], op.s3_cfg.tiles);
-                ++pass;
-            }
-            add(pass, a2, nullptr, epi[k], nullptr, 0, 0, 0);   // forward dim 2 + scatter
-            P.tb[pass] = P.tb[pass] ? std::min(P.tb[pass], op.s2_cfg.tb) : op.s2_cfg.tb;
-            P.gx[pass] = std::max(P.gx[pass], op.s2_cfg.tiles);
+            ok = add(pass++, op, a2, op.s2_cfg, PASS_LINES, x[k], epi[k], sk);   // gather + inverse dim 2
+            if (P.kind == PK_3D) ok = add(pass++, op, op.strided_args(3), op.s3_cfg, PASS_LINES, nullptr, epi[k], sk) && ok;
+            ok = add(pass++, op, ra, op.row_cfg, PASS_ROWS, nullptr, epi[k], sk) && ok;   // rows
+            if (P.kind == PK_3D) ok = add(pass++, op, op.strided_args(3), op.s3_cfg, PASS_LINES, nullptr, epi[k], sk) && ok;
+            ok = add(pass++, op, a2, op.s2_cfg, PASS_LINES, nullptr, epi[k], sk) && ok;   // forward dim 2 + scatter
         }
+        if (!ok) return CSIPM_ERR_UNSUPPORTED;
     }
     P.npass = (int)t.size();
-    // strided passes at the batch's common lines per CTA: shared memory for
-    // the largest instance at that width (data buffers + its twiddles)
-    for (int pass = 0; pass < P.npass; ++pass) {
-        const bool strided = (P.kind == PK_2D || P.kind == PK_3D) ? (pass != (P.kind == PK_3D ? 2 : 1))
-                                                                   : (P.kind == PK_1DL && pass == 2);
-        if (!strided) continue;
-        size_t sm = 0;
-        for (auto& e : t[pass]) {
-            const size_t data = 3 * (size_t)e.a.pl.L * (size_t)C * P.tb[pass];
-            sm = std::max(sm, data + (e.a.tw_in_smem ? (size_t)e.a.Ltab * (size_t)C : 0));
-        }
-        P.smem[pass] = sm;
-    }
     for (int pass = 0; pass < P.npass; ++pass) {
         if (!B.alloc(&P.tab[pass], t[pass].size())) return CSIPM_ERR_OOM;
         if (B.upload(P.tab[pass], t[pass].data(), sizeof(BPass<Epi>) * t[pass].size()) != cudaSuccess)
@@ -437,36 +391,13 @@ int build_product(BatchState& B, BProduct<Epi>& P, const std::vector<csipm_handl
     return CSIPM_OK;
 }
 
-template <int TB, bool INV, int IN, int OUT, class Epi>
-cudaError_t launch_bstrided_tb(const BProduct<Epi>& P, int pass, cudaStream_t st) {
-    auto k = bk_strided<TB, INV, IN, OUT, Epi>;
-    cudaError_t e = smem_optin(k, P.smem[pass]);
+template <typename K, class Epi>
+cudaError_t launch_bpass(K kernel, const BProduct<Epi>& P, int pass, cudaStream_t st) {
+    const cudaError_t e = smem_optin(kernel, P.smem[pass]);
     if (e != cudaSuccess) return e;
-    const int gx = batch_grid(k, 256, P.smem[pass], P.count, P.gx[pass]);
-    k<<<dim3(gx, P.count), 256, P.smem[pass], st>>>(P.tab[pass]);
+    const int gx = batch_grid(kernel, BATCH_THREADS, P.smem[pass], P.count, P.gx[pass]);
+    kernel<<<dim3(gx, P.count), BATCH_THREADS, P.smem[pass], st>>>(P.tab[pass]);
     return cudaGetLastError();
-}
-
-template <bool INV, int IN, int OUT, class Epi>
-cudaError_t launch_bstrided(const BProduct<Epi>& P, int pass, cudaStream_t st) {
-    switch (P.tb[pass]) {
-        case 2: return launch_bstrided_tb<2, INV, IN, OUT, Epi>(P, pass, st);
-        case 4: return launch_bstrided_tb<4, INV, IN, OUT, Epi>(P, pass, st);
-        case 8: return launch_bstrided_tb<8, INV, IN, OUT, Epi>(P, pass, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <int IN, int OUT, class Epi>
-cudaError_t launch_brow(const BProduct<Epi>& P, int pass, cudaStream_t st) {
-    auto run = [&](auto k) -> cudaError_t {
-        cudaError_t e = smem_optin(k, P.smem[pass]);
-        if (e != cudaSuccess) return e;
-        const int gx = batch_grid(k, 256, P.smem[pass], P.count, P.gx[pass]);
-        k<<<dim3(gx, P.count), 256, P.smem[pass], st>>>(P.tab[pass]);
-        return cudaGetLastError();
-    };
-    return P.mask ? run(bk_row<IN, OUT, true, Epi>) : run(bk_row<IN, OUT, false, Epi>);
 }
 
 // One A'A product for every instance of the batch.
@@ -475,32 +406,22 @@ cudaError_t batch_product(BatchState& B, const BProduct<Epi>& P) {
     cudaStream_t st = B.st;
     cudaError_t e = cudaSuccess;
     B.launches += P.npass;
-    if (P.kind == PK_1D) return launch_brow<IN_GATHER, OUT_SCATTER, Epi>(P, 0, st);
-    if (P.kind == PK_1DL) {
-        {
-            auto k = bk_l1d_first<Epi>;
-            if ((e = smem_optin(k, P.smem[0])) != cudaSuccess) return e;
-            k<<<dim3(P.gx[0], P.count), 256, P.smem[0], st>>>(P.tab[0]);
-        }
-        {
-            auto run = [&](auto k) -> cudaError_t {
-                cudaError_t e2 = smem_optin(k, P.smem[1]);
-                if (e2 != cudaSuccess) return e2;
-                k<<<dim3(P.gx[1], P.count), 256, P.smem[1], st>>>(P.tab[1]);
-                return cudaGetLastError();
-            };
-            if ((e = P.mask ? run(bk_l1d_row<true, Epi>) : run(bk_l1d_row<false, Epi>)) != cudaSuccess) return e;
-        }
-        if ((e = launch_bstrided<false, IN_SPEC, OUT_SPEC, Epi>(P, 2, st)) != cudaSuccess) return e;
-        bk_l1d_post<Epi><<<dim3(P.gx[3], P.count), 256, 0, st>>>(P.tab[3]);
-        return cudaGetLastError();
+    if (P.kind == PK_1D || P.kind == PK_1DL) {
+        if ((e = launch_bpass(bk_l1d_first<Epi>, P, 0, st)) != cudaSuccess) return e;
+        e = P.mask ? launch_bpass(bk_l1d_row<true, Epi>, P, 1, st) : launch_bpass(bk_l1d_row<false, Epi>, P, 1, st);
+        if (e != cudaSuccess) return e;
+        return launch_bpass(bk_l1d_last<Epi>, P, 2, st);
     }
     int pass = 0;
-    if ((e = launch_bstrided<true, IN_GATHER, OUT_SPEC, Epi>(P, pass++, st)) != cudaSuccess) return e;
-    if (P.kind == PK_3D && (e = launch_bstrided<true, IN_SPEC, OUT_SPEC, Epi>(P, pass++, st)) != cudaSuccess) return e;
-    if ((e = launch_brow<IN_SPEC, OUT_SPEC, Epi>(P, pass++, st)) != cudaSuccess) return e;
-    if (P.kind == PK_3D && (e = launch_bstrided<false, IN_SPEC, OUT_SPEC, Epi>(P, pass++, st)) != cudaSuccess) return e;
-    return launch_bstrided<false, IN_SPEC, OUT_SCATTER, Epi>(P, pass, st);
+    if ((e = launch_bpass(bk_strided<true, IN_GATHER, OUT_SPEC, Epi>, P, pass++, st)) != cudaSuccess) return e;
+    if (P.kind == PK_3D && (e = launch_bpass(bk_strided<true, IN_SPEC, OUT_SPEC, Epi>, P, pass++, st)) != cudaSuccess)
+        return e;
+    e = P.mask ? launch_bpass(bk_row<true, Epi>, P, pass, st) : launch_bpass(bk_row<false, Epi>, P, pass, st);
+    if (e != cudaSuccess) return e;
+    ++pass;
+    if (P.kind == PK_3D && (e = launch_bpass(bk_strided<false, IN_SPEC, OUT_SPEC, Epi>, P, pass++, st)) != cudaSuccess)
+        return e;
+    return launch_bpass(bk_strided<false, IN_SPEC, OUT_SCATTER, Epi>, P, pass, st);
 }
 
 int read_flag(BatchState& B) {

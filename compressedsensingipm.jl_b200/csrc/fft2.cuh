@@ -5,7 +5,7 @@
 // flight per thread), runs DFT_A, multiplies by W_L^{t*ka} and writes the A
 // results to shared memory.  Step 2: thread s < A reads its B values, runs
 // DFT_B and owns the outputs X[s + A*kb].  One shared-memory round trip per
-// transform (the Stockham engine needs one per radix stage).
+// transform (the run-time-plan passes need one per stage but the first).
 //
 // In the row pass the inverse transform (A, B) leaves thread s with
 // z[s + A*kb]; the forward transform is run with the factors swapped (B, A),
@@ -15,7 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "bulk.cuh"
-#include "fft_device.cuh"
+#include "dft.cuh"
 #include "operator.cuh"
 
 namespace csipm {
@@ -41,6 +41,11 @@ __device__ __forceinline__ C tw_apply(C v, const C* __restrict__ tw, int e) {
 }
 
 // ------------------------------------------------------------ strided pass
+// The planes i = 0, M1 of a solver-order gather or scatter go through the
+// line's affine map (make_line): with a table look-up and a branch per element
+// the lanes of those planes held up their warps, and at 1024^2 (FP64) the
+// gather took 17.3 us where it now takes 7.0, the scatter with the CG
+// epilogue 20.1 -> 14.7 us.
 // CTAs per SM the register allocation of a strided pass must allow, by
 // precision, CTA size (NT threads) and pass kind, as measured on B200 at
 // 256^3 and 320^3: more CTAs hide the gather/scatter load latency (the
@@ -49,10 +54,10 @@ __device__ __forceinline__ C tw_apply(C v, const C* __restrict__ tw, int e) {
 // fastest unconstrained.  (An explicit 1 lets the compiler use up to 255
 // registers, more than it picks with no bound at all.)
 template <typename T, int IN, int OUT, int NT> constexpr int fft2_min_ctas() {
-    constexpr bool scatter = OUT == OUT_SSCATTER || OUT == OUT_SCATTER;
+    constexpr bool scatter = OUT == OUT_SSCATTER;
     if (sizeof(T) == 4) return scatter ? 3 : (NT <= 256 ? 4 : 3);
     if (NT <= 128) return 4;
-    return scatter ? 3 : ((IN == IN_SGATHER || IN == IN_GATHER) ? 4 : 1);
+    return scatter ? 3 : (IN == IN_SGATHER ? 4 : 1);
 }
 
 template <typename T, int A, int B, bool INV, int IN, int OUT, typename TS, class Epi>
@@ -70,9 +75,7 @@ strided2_kernel(PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
     const bool live = b < nb;
     const long long base = i0 + b + (long long)o * a.so;
     const C* __restrict__ tw = a.tw;    // L-th roots (Ltab == L)
-    const C zero = mk((T)0, (T)0);
-    // each thread keeps one dim-1 position for the whole tile: interior
-    // positions (all but i = 0 and i = M1) take the short decode
+    // each thread keeps one dim-1 position for the whole tile
     const int ii = i0 + b;
     const bool interior = ii >= 1 && ii <= a.g.m1 - 1;
 
@@ -103,61 +106,11 @@ strided2_kernel(PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
     if (t < B) {
         C v[A];
         if constexpr (IN == IN_SGATHER) {
-            // interior lines: one base pair index plus q times a fixed stride
-            // (the branch is per thread and outside the element loop, so the
-            // A loads issue back to back)
-            if (live && interior) {
-                const cplx_t<TS>* __restrict__ s2 = reinterpret_cast<const cplx_t<TS>*>(src);
-                int j0, k0;
-                jk_of(a.jk_mode, o, t, j0, k0);
-                const int64_t p0 = sol_pair(a.g, ii, j0, k0);
-                const int64_t ps = (a.jk_mode == 0 ? (int64_t)a.g.n2 : (int64_t)1) * (a.g.m1 - 1) * B;
-                const T r = (T)0.7071067811865476;
-#pragma unroll
-                for (int q = 0; q < A; ++q) {
-                    const cplx_t<TS> w = s2[p0 + q * ps];
-                    v[q] = mk((T)w.x * r, (T)w.y * r);
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < A; ++q) {
-                    const int x = t + B * q;
-                    int j, k;
-                    jk_of(a.jk_mode, o, x, j, k);
-                    if (live) {
-                        const int4 t4 = a.pmap[((ii == 0 ? 0 : 1) * a.g.n3 + k) * a.g.n2 + j];
-                        v[q] = gather_val<T>(MapEntry{t4.x, t4.y, t4.z, t4.w}, src);
-                    } else {
-                        v[q] = zero;
-                    }
-                }
-            }
+            GatherLine<T, TS, true> gl;
+            gl.set(a.g, src, ii, a.jk_mode == 1 ? o : 0, live);
+            gl.template load<A>(v, t, B, b);
         } else {
-#pragma unroll
-        for (int q = 0; q < A; ++q) {
-            const int x = t + B * q;
-            if (!live) {
-                v[q] = zero;
-            } else if constexpr (IN == IN_SPEC) {
-                v[q] = a.spec[base + (long long)x * a.sx];
-            } else if constexpr (IN == IN_SGATHER) {
-                int j, k;
-                jk_of(a.jk_mode, o, x, j, k);
-                if (interior) {
-                    const cplx_t<TS> w = reinterpret_cast<const cplx_t<TS>*>(src)[sol_pair(a.g, ii, j, k)];
-                    const T r = (T)0.7071067811865476;
-                    v[q] = mk((T)w.x * r, (T)w.y * r);
-                } else {   // planes i = 0, M1: tabulated entries (no per-element decode)
-                    const int4 t4 = a.pmap[((ii == 0 ? 0 : 1) * a.g.n3 + k) * a.g.n2 + j];
-                    v[q] = gather_val<T>(MapEntry{t4.x, t4.y, t4.z, t4.w}, src);
-                }
-            } else {
-                int j, k;
-                jk_of(a.jk_mode, o, x, j, k);
-                const MapEntry en = interior ? decode_interior(a.g, ii, j, k) : decode(a.g, ii, j, k);
-                v[q] = gather_val<T>(en, src);
-            }
-        }
+            SpecLine<T>{a.spec + base, a.sx, live}.template load<A>(v, t, B, b);
         }
         Dft<A, INV, T>::run(v);
 #pragma unroll
@@ -210,45 +163,13 @@ strided2_kernel(PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
                                     sc_pre[q]);
                 }
             }
-        } else {
-            constexpr int U = 2;
-#pragma unroll
-            for (int k0 = 0; k0 < B; k0 += U) {
-                MapEntry en[U];
-                typename Epi::Pre pr[U], pi[U];
-#pragma unroll
-                for (int q = 0; q < U; ++q) {
-                    if (k0 + q < B) {
-                        int j, k;
-                        jk_of(a.jk_mode, o, s + A * (k0 + q), j, k);
-                        if (OUT == OUT_SSCATTER) {   // planes i = 0, M1 in solver order: tabulated
-                            const int4 t4 = a.pmap[((ii == 0 ? 0 : 1) * a.g.n3 + k) * a.g.n2 + j];
-                            en[q] = MapEntry{t4.x, t4.y, t4.z, t4.w};
-                        } else {
-                            en[q] = interior ? decode_interior(a.g, ii, j, k) : decode(a.g, ii, j, k);
-                        }
-                        if (en[q].src) {
-                            pr[q] = ep.pre(en[q].re);
-                            if (en[q].kind != KIND_VERT) pi[q] = ep.pre(en[q].im);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < U; ++q) {
-                    if (k0 + q < B && en[q].src) {
-                        const C v = u[k0 + q];
-                        if (en[q].kind == KIND_VERT) {
-                            ep.put(en[q].re, (double)v.x, pr[q]);
-                        } else {
-                            ep.put(en[q].re, SQRT2_D * (double)v.x, pr[q]);
-                            ep.put(en[q].im, (en[q].kind == KIND_PLUS ? SQRT2_D : -SQRT2_D) * (double)v.y, pi[q]);
-                        }
-                    }
-                }
-            }
+        } else {   // planes i = 0, M1
+            ScatterLine<T, Epi, true> sl;
+            sl.set(a.g, &ep, ii, a.jk_mode == 1 ? o : 0, true);
+            sl.template store<B>(u, s, A, b);
         }
     }
-    if (OUT == OUT_SCATTER || OUT == OUT_SSCATTER) ep.finish();
+    if (OUT == OUT_SSCATTER) ep.finish();
 }
 
 // ---------------------------------------------------------------- row pass
@@ -634,7 +555,7 @@ inline bool fft2_factor(int L, int* A, int* B) {
 // stream's recoveries (3D sides of 32-128, 2D sides of 128-1024, factors
 // 2, 3, 5), picked from its length histogram weighted by work (pairs whose
 // kernels spill registers heavily, or that the autotuner found slower than
-// Stockham, are left to Stockham).
+// the run-time-plan passes, are left to those).
 #define CSIPM_FFT2_SPAIRS(X) \
     X(16, 20) X(16, 16) X(10, 16) X(8, 16) X(8, 8) X(10, 12) X(9, 12) X(8, 10) X(8, 9) X(9, 10) X(10, 10) \
     X(8, 12) X(5, 8) X(6, 8) X(6, 9) X(6, 6) X(6, 10) X(5, 10) X(4, 8) X(32, 32) X(20, 20) X(25, 32) \
@@ -664,20 +585,15 @@ cudaError_t launch_row2(int A, int B, const PassArgs<T>& a, cudaStream_t st);
 // The instantiations of the two-level passes (fft2.cu): (T, INV, IN, OUT, TS,
 // Epi) and (T, IN, OUT, MASK).  Fft2S / Fft2R tell the dispatch which exist.
 #define CSIPM_FFT2_STRIDED_LIST64(X)                                 \
-    X(double, true, IN_GATHER, OUT_SPEC, double, EpiStore<double>)   \
     X(double, true, IN_SPEC, OUT_SPEC, double, EpiStore<double>)     \
     X(double, false, IN_SPEC, OUT_SPEC, double, EpiStore<double>)    \
-    X(double, false, IN_SPEC, OUT_SCATTER, double, EpiStore<double>) \
-    X(double, false, IN_SPEC, OUT_SCATTER, double, EpiCG<double>)    \
     X(double, true, IN_SGATHER, OUT_SPEC, double, EpiStore<double>)  \
     X(double, false, IN_SPEC, OUT_SSCATTER, double, EpiStore<double>) \
     X(double, false, IN_SPEC, OUT_SSCATTER, double, EpiCG<double>)
 #define CSIPM_FFT2_STRIDED_LIST32(X)                                 \
-    X(float, true, IN_GATHER, OUT_SPEC, float, EpiStore<double>)     \
     X(float, true, IN_SGATHER, OUT_SPEC, float, EpiStore<double>)    \
     X(float, true, IN_SPEC, OUT_SPEC, double, EpiStore<double>)      \
     X(float, false, IN_SPEC, OUT_SPEC, double, EpiStore<double>)     \
-    X(float, false, IN_SPEC, OUT_SCATTER, double, EpiCG<float>)      \
     X(float, false, IN_SPEC, OUT_SSCATTER, double, EpiCG<float>)
 #define CSIPM_FFT2_STRIDED_LIST(X) CSIPM_FFT2_STRIDED_LIST64(X) CSIPM_FFT2_STRIDED_LIST32(X)
 
@@ -704,19 +620,5 @@ CSIPM_FFT2_STRIDED_LIST(CSIPM_FFT2_HAS_S)
 CSIPM_FFT2_ROW_LIST(CSIPM_FFT2_HAS_R)
 #undef CSIPM_FFT2_HAS_S
 #undef CSIPM_FFT2_HAS_R
-
-}  // namespace csipm
-
-namespace csipm {
-
-template <typename T>
-inline void FftOperator<T>::choose_two_level() {
-    s2_A = s2_B = s3_A = s3_B = r_A = r_B = 0;
-    if (g.dim < 2) return;
-    int A = 0, B = 0;
-    if (fft2_factor(g.n2, &A, &B) && fft2_strided_pair(A, B)) { s2_A = A; s2_B = B; }
-    if (g.dim == 3 && fft2_factor(g.n3, &A, &B) && fft2_strided_pair(A, B)) { s3_A = A; s3_B = B; }
-    if (fft2_factor(g.m1, &A, &B) && fft2_row_pair(A, B)) { r_A = A; r_B = B; }
-}
 
 }  // namespace csipm

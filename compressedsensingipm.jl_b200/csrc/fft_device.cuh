@@ -1,251 +1,352 @@
-// Mixed-radix Stockham FFT over lines held in shared memory.
+// Mixed-radix Stockham FFT over a tile of TB interleaved lines of length L,
+// with the radices of a run-time plan.
 //
-// A CTA holds TB interleaved lines of length L in shared memory, element
-// (x, b) at buf[x*TBP + b] (b fastest, TBP >= TB).  Two stage engines:
-//   ping-pong (default): each stage reads one buffer and writes the other, one
-//     butterfly per loop trip, so only R complex values are live per thread;
-//   in place (lines too long to double-buffer): each thread loads all its
-//     butterflies into registers, the block synchronises, then it stores;
-//     this path may spill registers and is only used for very long rows.
-// Stage s with radix
-// R and Ns = product of the radices before it maps butterfly u of line b to
+// Stage s with radix R and Ns = product of the radices before it maps
+// butterfly u of line b to
 //   inputs  x = u + r*(L/R)                       (r = 0..R-1)
 //   outputs x = (u - u%Ns)*R + u%Ns + r*Ns
 // with twiddle W_{Ns*R}^{(u%Ns)*r} on input r, giving natural order after the
 // last stage.  Twiddles come from a table of Ltab-th roots of unity
 // W^e = exp(-2*pi*i*e/Ltab) (Ltab a multiple of L); the inverse transform uses
-// their conjugates.  Radices 2, 3, 4, 5, 7, 8 have register butterflies; any
-// other prime is done as a direct DFT.
+// their conjugates.
+//
+// Radices up to 10 are register butterflies: the first stage's inputs come
+// straight from the pass's source and the last stage's outputs go straight to
+// its destination, so a line of two stages (up to 100 points) crosses shared
+// memory once.  Primes above 7 are one stage each, computed from the sums
+// and differences of mirrored inputs (prime_stage).  The former engine
+// (radices up to 8, every stage through shared memory, primes as direct
+// sums with a table look-up per product) spent its time on shared-memory
+// traffic and run-time index division.
+//
+// Rows too long for two tile buffers use the in-place engine at the end of
+// this file (radices up to 8, register-staged).
 #pragma once
 #include "cplx.cuh"
-#include "roots.h"
+#include "dft.cuh"
+#include "plan_dev.h"
 
 namespace csipm {
 
-constexpr int FFT_MAX_STAGES = 24;
+// ------------------------------------------------------------------- stages
+// x/d for 0 <= x < 2^16, d < 2^16 from mag = floor((2^32 - 1)/d) + 1 (exact in
+// that range); d == 1 is the one divisor whose reciprocal does not fit
+__device__ __forceinline__ int quot(int x, int d, unsigned mag) { return d == 1 ? x : (int)__umulhi((unsigned)x, mag); }
 
-struct FftPlanDev {
-    int L;                       // transform length
-    int nst;                     // number of stages
-    int rad[FFT_MAX_STAGES];     // radices, in order
+// One butterfly of a stage: inputs v, twiddled and transformed.
+template <int R, bool INV, typename T>
+__device__ __forceinline__ void twiddle_dft(cplx_t<T>* v, int k, const FftStage& s, const cplx_t<T>* __restrict__ tw) {
+    if (R > 1 && s.Ns > 1) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = twmul<INV>(v[r], tw[k * r * s.step]);
+    }
+    Dft<R, INV, T>::run(v);
+}
+
+#define CSIPM_RADICES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10)
+
+// Butterfly w of a smem -> smem stage: load<R> and transform, then put<R>.
+template <typename T, int R, bool INV>
+__device__ __forceinline__ void bfly_load(cplx_t<T>* v, const cplx_t<T>* in, const TileLay& lay, const FftStage& s,
+                                          const cplx_t<T>* __restrict__ tw, int u, int k, int b) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = in[lay.at(u + r * s.m, b)];
+    twiddle_dft<R, INV, T>(v, k, s, tw);
+}
+template <typename T, int R>
+__device__ __forceinline__ void bfly_put(const cplx_t<T>* v, cplx_t<T>* out, const TileLay& lay, int o, int Ns, int b) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) out[lay.at(o + r * Ns, b)] = v[r];
+}
+
+// ---- prime stages
+// A radix p without a register butterfly: with t_j = x_j + x_{p-j} and
+// d_j = x_j - x_{p-j} (j = 1..h, h = (p-1)/2) of the twiddled inputs,
+//   X_k, X_{p-k} = (x_0 + sum_j cos(2 pi j k/p) t_j) -+ i sum_j sin(2 pi j k/p) d_j,
+// (p-1)^2 real multiply-adds a butterfly instead of 4 p^2, and each
+// thread takes PRIME_K pairs (k, p-k), so a value read from shared memory
+// serves 2*PRIME_K of them.  Up to PRIME_MAT the cosines and sines of all
+// (j, k) lie in shared memory, PRIME_K neighbours at a time (a broadcast read
+// at a fixed offset each; one table of p roots with the index j k mod p kept
+// by additions spent more instructions on indices than on arithmetic); larger
+// primes use the table of roots.
+constexpr int PRIME_K = 5;
+constexpr int PRIME_MAT = 64;
+
+__host__ __device__ constexpr int prime_groups(int p) { return ((p - 1) / 2 + PRIME_K - 1) / PRIME_K; }
+__host__ __device__ constexpr int prime_table(int p) {
+    return p <= PRIME_MAT ? (p - 1) / 2 * prime_groups(p) * PRIME_K : p;
+}
+
+// the tables (cos, -sin) of every prime stage, each at its cs
+template <typename C>
+__device__ __forceinline__ void prime_tables(const FftStage* st, int nst, const C* __restrict__ tw, int Ltab, C* cs) {
+    for (int s = 0; s < nst; ++s) {
+        const int p = st[s].R;
+        if (reg_radix(p)) continue;
+        C* t = cs + st[s].cs;
+        const int unit = Ltab / p;
+        if (p > PRIME_MAT) {
+            for (int e = threadIdx.x; e < p; e += blockDim.x) t[e] = tw[e * unit];
+        } else {
+            const int nk = prime_groups(p) * PRIME_K;
+            for (int e = threadIdx.x; e < (p - 1) / 2 * nk; e += blockDim.x)
+                t[e] = tw[((e / nk + 1) * (e % nk + 1)) % p * unit];
+        }
+    }
+}
+
+// t_j at position j, d_j at position p - j of buf, from ld(x, b) (the source
+// of a first stage, or buf itself: one thread owns both positions).
+template <typename T, bool INV, class Ld>
+__device__ __forceinline__ void prime_combine(cplx_t<T>* buf, const TileLay& lay, const FftStage& s, bool first,
+                                              const cplx_t<T>* __restrict__ tw, Ld&& ld) {
+    using C = cplx_t<T>;
+    const int p = s.R, h = (p - 1) / 2, mask = (1 << lay.lg) - 1;
+    const int n = (s.m * (h + 1)) << lay.lg;
+    for (int w = threadIdx.x; w < n; w += blockDim.x) {
+        const int b = w & mask, rest = w >> lay.lg;
+        const int j = quot(rest, s.m, s.mag_m), u = rest - j * s.m;
+        if (j == 0) {
+            if (first) buf[lay.at(u, b)] = ld(u, b);
+            continue;
+        }
+        const int x1 = u + j * s.m, x2 = u + (p - j) * s.m;
+        C a = ld(x1, b), c = ld(x2, b);
+        if (s.Ns > 1) {
+            const int k = u - s.Ns * quot(u, s.Ns, s.mag_ns);
+            a = twmul<INV>(a, tw[k * j * s.step]);
+            c = twmul<INV>(c, tw[k * (p - j) * s.step]);
+        }
+        buf[lay.at(x1, b)] = cadd(a, c);
+        buf[lay.at(x2, b)] = csub(a, c);
+    }
+}
+
+// The sums of one thread's PRIME_K pairs; put(x, b, value) receives the
+// outputs (never into buf).
+template <typename T, bool INV, class Put>
+__device__ __forceinline__ void prime_sums(const cplx_t<T>* buf, const TileLay& lay, const FftStage& s,
+                                           const cplx_t<T>* cs, Put&& put) {
+    using C = cplx_t<T>;
+    const int p = s.R, h = (p - 1) / 2, mask = (1 << lay.lg) - 1;
+    const int ng = prime_groups(p);
+    const int n = (s.m * ng) << lay.lg;
+    for (int w = threadIdx.x; w < n; w += blockDim.x) {
+        const int b = w & mask, rest = w >> lay.lg;
+        const int g = quot(rest, s.m, s.mag_m), u = rest - g * s.m;
+        const C x0 = buf[lay.at(u, b)];
+        C e[PRIME_K], f[PRIME_K], sum = x0;
+#pragma unroll
+        for (int q = 0; q < PRIME_K; ++q) {
+            e[q] = x0;
+            f[q] = mk((T)0, (T)0);
+        }
+        auto add = [&](int q, C r, C t, C d) {   // r = (cos, -sin)
+            e[q].x += r.x * t.x;
+            e[q].y += r.x * t.y;
+            f[q].x -= r.y * d.x;
+            f[q].y -= r.y * d.y;
+        };
+        if (p <= PRIME_MAT) {
+            const C* row = cs + g * PRIME_K;
+#pragma unroll 1
+            for (int j = 1; j <= h; ++j, row += ng * PRIME_K) {
+                const C t = buf[lay.at(u + j * s.m, b)], d = buf[lay.at(u + (p - j) * s.m, b)];
+                sum = cadd(sum, t);
+#pragma unroll
+                for (int q = 0; q < PRIME_K; ++q) add(q, row[q], t, d);
+            }
+        } else {
+            int idx[PRIME_K];
+#pragma unroll
+            for (int q = 0; q < PRIME_K; ++q) idx[q] = 0;
+#pragma unroll 1
+            for (int j = 1; j <= h; ++j) {
+                const C t = buf[lay.at(u + j * s.m, b)], d = buf[lay.at(u + (p - j) * s.m, b)];
+                sum = cadd(sum, t);
+#pragma unroll
+                for (int q = 0; q < PRIME_K; ++q) {
+                    idx[q] += min(g * PRIME_K + q + 1, h);
+                    if (idx[q] >= p) idx[q] -= p;
+                    add(q, cs[idx[q]], t, d);
+                }
+            }
+        }
+        const int k0 = u - s.Ns * quot(u, s.Ns, s.mag_ns);
+        const int o = (u - k0) * p + k0;
+        if (g == 0) put(o, b, sum);
+#pragma unroll
+        for (int q = 0; q < PRIME_K; ++q) {
+            const int k = g * PRIME_K + q + 1;
+            if (k <= h) {
+                const C jf = cmul_i(f[q]);
+                put(o + k * s.Ns, b, INV ? cadd(e[q], jf) : csub(e[q], jf));
+                put(o + (p - k) * s.Ns, b, INV ? csub(e[q], jf) : cadd(e[q], jf));
+            }
+        }
+    }
+}
+
+// Items of a stage: what one thread takes at a time.
+__host__ __device__ __forceinline__ int stage_items(int R, int L, int lg) {
+    return reg_radix(R) ? (L / R) << lg : ((L / R) * prime_groups(R)) << lg;
+}
+
+// A tile's buffers and tables.
+template <typename C>
+struct FftTile {
+    TileLay lay;
+    const FftStage* st;
+    int nst, L;
+    const C* tw;
+    const C* cs;      // prime roots of st
+    C* cur;           // holds the tile between stages
+    C* oth;           // second buffer (only touched by stages from shared memory to shared memory)
+    __device__ __forceinline__ void swap() { C* t = cur; cur = oth; oth = t; }
 };
 
+// Stages s0..s1-1, smem -> smem from one buffer to the other (the tile in
+// t.cur before and after); ends with a barrier.  There is no barrier inside a
+// radix's branch: the compiler cannot prove the branch uniform and spills what
+// lives across one.
+template <typename T, bool INV>
+__device__ __forceinline__ void mid_stages(FftTile<cplx_t<T>>& t, int s0, int s1) {
+    using C = cplx_t<T>;
+    const TileLay lay = t.lay;
+    const int mask = (1 << lay.lg) - 1;
+#pragma unroll 1
+    for (int q = s0; q < s1; ++q) {
+        const FftStage s = t.st[q];
+        const int n = s.m << lay.lg;
+        if (reg_radix(s.R)) {
+            for (int w = threadIdx.x; w < n; w += blockDim.x) {
+                const int b = w & mask, u = w >> lay.lg;
+                const int k = u - s.Ns * quot(u, s.Ns, s.mag_ns);
+                const int o = (u - k) * s.R + k;
+                switch (s.R) {
+#define CSIPM_MID(RR)                                                       \
+                    case RR: {                                              \
+                        C v[RR];                                            \
+                        bfly_load<T, RR, INV>(v, t.cur, lay, s, t.tw, u, k, b); \
+                        bfly_put<T, RR>(v, t.oth, lay, o, s.Ns, b);         \
+                    } break;
+                    CSIPM_RADICES(CSIPM_MID)
+#undef CSIPM_MID
+                }
+            }
+        } else {
+            C* buf = t.cur;
+            prime_combine<T, INV>(buf, lay, s, false, t.tw, [&](int x, int c) { return buf[lay.at(x, c)]; });
+            __syncthreads();
+            C* out = t.oth;
+            prime_sums<T, INV>(buf, lay, s, t.cs + s.cs, [&](int x, int c, C w) { out[lay.at(x, c)] = w; });
+        }
+        t.swap();
+        __syncthreads();
+    }
+}
+
+// First stage: ld.load<R>(v, u, m, b) brings the inputs u + r*m of line b
+// (ld.one(x, b) a single one), the results go to t.cur; ends with a barrier.
+template <typename T, bool INV, class Ld>
+__device__ __forceinline__ void first_stage(FftTile<cplx_t<T>>& t, Ld& ld) {
+    using C = cplx_t<T>;
+    const FftStage s = t.st[0];
+    const int mask = (1 << t.lay.lg) - 1;
+    switch (s.R) {
+#define CSIPM_FIRST(RR)                                                                   \
+        case RR:                                                                          \
+            for (int w = threadIdx.x; w < s.m << t.lay.lg; w += blockDim.x) {             \
+                const int b = w & mask, u = w >> t.lay.lg;                                \
+                C v[RR];                                                                  \
+                ld.template load<RR>(v, u, s.m, b);                                       \
+                Dft<RR, INV, T>::run(v);                                                  \
+                _Pragma("unroll") for (int r = 0; r < RR; ++r) t.cur[t.lay.at(u * RR + r, b)] = v[r]; \
+            }                                                                             \
+            break;
+        CSIPM_RADICES(CSIPM_FIRST)
+#undef CSIPM_FIRST
+        default: {
+            C* out = t.oth;
+            const TileLay lay = t.lay;
+            prime_combine<T, INV>(t.cur, lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
+            __syncthreads();
+            prime_sums<T, INV>(t.cur, lay, s, t.cs + s.cs, [&](int x, int b, C v) { out[lay.at(x, b)] = v; });
+            t.swap();
+        } break;
+    }
+    __syncthreads();
+}
+
+// Last stage: outputs x = u + r*Ns of line b go to out.store<R>(v, u, Ns, b)
+// (out.one(x, b, v) a single one).
+template <typename T, bool INV, class St>
+__device__ __forceinline__ void last_stage(FftTile<cplx_t<T>>& t, St& out) {
+    using C = cplx_t<T>;
+    const FftStage s = t.st[t.nst - 1];
+    const int mask = (1 << t.lay.lg) - 1;
+    const TileLay lay = t.lay;
+    switch (s.R) {
+#define CSIPM_LAST(RR)                                                                    \
+        case RR:                                                                          \
+            for (int w = threadIdx.x; w < s.m << lay.lg; w += blockDim.x) {               \
+                const int b = w & mask, u = w >> lay.lg;                                  \
+                C v[RR];                                                                  \
+                _Pragma("unroll") for (int r = 0; r < RR; ++r) v[r] = t.cur[lay.at(u + r * s.m, b)]; \
+                twiddle_dft<RR, INV, T>(v, u, s, t.tw);                                   \
+                out.template store<RR>(v, u, s.Ns, b);                                    \
+            }                                                                             \
+            break;
+        CSIPM_RADICES(CSIPM_LAST)
+#undef CSIPM_LAST
+        default: {
+            C* buf = t.cur;
+            prime_combine<T, INV>(buf, lay, s, false, t.tw, [&](int x, int b) { return buf[lay.at(x, b)]; });
+            __syncthreads();
+            prime_sums<T, INV>(buf, lay, s, t.cs + s.cs,
+                               [&](int x, int b, C v) { out.one(x, b, v); });
+        } break;
+    }
+}
+
+// A whole transform from ld to out.  Every thread of the block calls it (it
+// contains barriers); the caller synchronises before the buffers are reused.
+template <typename T, bool INV, class Ld, class St>
+__device__ __forceinline__ void fft_through(FftTile<cplx_t<T>>& t, Ld& ld, St& out) {
+    using C = cplx_t<T>;
+    if (t.nst == 1) {   // one radix: no exchange (a prime goes through shared memory)
+        const FftStage s = t.st[0];
+        const int mask = (1 << t.lay.lg) - 1;
+        switch (s.R) {
+#define CSIPM_ONE(RR)                                                     \
+            case RR:                                                      \
+                for (int w = threadIdx.x; w < 1 << t.lay.lg; w += blockDim.x) { \
+                    C v[RR];                                              \
+                    ld.template load<RR>(v, 0, 1, w & mask);              \
+                    Dft<RR, INV, T>::run(v);                              \
+                    out.template store<RR>(v, 0, 1, w & mask);            \
+                }                                                         \
+                break;
+            CSIPM_RADICES(CSIPM_ONE)
+#undef CSIPM_ONE
+            default:
+                prime_combine<T, INV>(t.cur, t.lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
+                __syncthreads();
+                prime_sums<T, INV>(t.cur, t.lay, s, t.cs + s.cs, [&](int x, int b, C v) { out.one(x, b, v); });
+                break;
+        }
+        return;
+    }
+    first_stage<T, INV>(t, ld);
+    mid_stages<T, INV>(t, 1, t.nst - 1);
+    last_stage<T, INV>(t, out);
+}
+
+// ------------------------------------------------- in-place engine (very long rows)
 // per-thread register budget: about 8 complex values per stage
 template <int R> struct MaxItems { static constexpr int v = (8 + R - 1) / R; };
 constexpr int GENERIC_MAX_ITEMS = 8;
-
-// ---------------------------------------------------------------- butterflies
-template <bool INV, typename C> __device__ __forceinline__ C rot_mi(C a) {   // a * (-i) forward, a * (+i) inverse
-    return INV ? cmul_i(a) : cmul_mi(a);
-}
-
-template <int R, bool INV, typename T> struct Dft;
-
-template <bool INV, typename T> struct Dft<2, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        C t = a[0];
-        a[0] = cadd(t, a[1]);
-        a[1] = csub(t, a[1]);
-    }
-};
-
-template <bool INV, typename T> struct Dft<4, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        C t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
-        C t2 = cadd(a[1], a[3]), t3 = rot_mi<INV>(csub(a[1], a[3]));
-        a[0] = cadd(t0, t2);
-        a[2] = csub(t0, t2);
-        a[1] = cadd(t1, t3);
-        a[3] = csub(t1, t3);
-    }
-};
-
-template <bool INV, typename T> struct Dft<8, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        const T h = (T)0.7071067811865476;   // sqrt(2)/2
-        C e[4] = {a[0], a[2], a[4], a[6]};
-        C o[4] = {a[1], a[3], a[5], a[7]};
-        Dft<4, INV, T>::run(e);
-        Dft<4, INV, T>::run(o);
-        // o[k] *= W8^k  (W8 = exp(-i*pi/4) forward)
-        C o1, o2, o3;
-        if (!INV) {
-            o1 = mk((o[1].x + o[1].y) * h, (o[1].y - o[1].x) * h);
-            o2 = cmul_mi(o[2]);
-            o3 = mk((o[3].y - o[3].x) * h, -(o[3].x + o[3].y) * h);
-        } else {
-            o1 = mk((o[1].x - o[1].y) * h, (o[1].x + o[1].y) * h);
-            o2 = cmul_i(o[2]);
-            o3 = mk(-(o[3].x + o[3].y) * h, (o[3].x - o[3].y) * h);
-        }
-        a[0] = cadd(e[0], o[0]); a[4] = csub(e[0], o[0]);
-        a[1] = cadd(e[1], o1);   a[5] = csub(e[1], o1);
-        a[2] = cadd(e[2], o2);   a[6] = csub(e[2], o2);
-        a[3] = cadd(e[3], o3);   a[7] = csub(e[3], o3);
-    }
-};
-
-template <bool INV, typename T> struct Dft<3, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        const T s = (T)0.8660254037844386;   // sin(2*pi/3)
-        C t1 = cadd(a[1], a[2]), t2 = csub(a[1], a[2]);
-        C m = mk(a[0].x - (T)0.5 * t1.x, a[0].y - (T)0.5 * t1.y);
-        a[0] = cadd(a[0], t1);
-        // forward: y1 = m - i*s*t2, y2 = m + i*s*t2
-        C st = mk(s * t2.x, s * t2.y);
-        C ist = cmul_i(st);
-        if (!INV) { a[1] = csub(m, ist); a[2] = cadd(m, ist); }
-        else      { a[1] = cadd(m, ist); a[2] = csub(m, ist); }
-    }
-};
-
-template <bool INV, typename T> struct Dft<5, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        const T c1 = (T)0.30901699437494745, c2 = (T)-0.8090169943749475;
-        const T s1 = (T)0.9510565162951535, s2 = (T)0.5877852522924731;
-        C t1 = cadd(a[1], a[4]), t2 = cadd(a[2], a[3]);
-        C t3 = csub(a[1], a[4]), t4 = csub(a[2], a[3]);
-        C b1 = mk(a[0].x + c1 * t1.x + c2 * t2.x, a[0].y + c1 * t1.y + c2 * t2.y);
-        C b2 = mk(a[0].x + c2 * t1.x + c1 * t2.x, a[0].y + c2 * t1.y + c1 * t2.y);
-        C e1 = mk(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
-        C e2 = mk(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
-        a[0] = cadd(a[0], cadd(t1, t2));
-        C ie1 = cmul_i(e1), ie2 = cmul_i(e2);
-        if (!INV) { a[1] = csub(b1, ie1); a[4] = cadd(b1, ie1); a[2] = csub(b2, ie2); a[3] = cadd(b2, ie2); }
-        else      { a[1] = cadd(b1, ie1); a[4] = csub(b1, ie1); a[2] = cadd(b2, ie2); a[3] = csub(b2, ie2); }
-    }
-};
-
-template <bool INV, typename T> struct Dft<7, INV, T> {
-    using C = cplx_t<T>;
-    __device__ __forceinline__ static void run(C* a) {
-        const T c1 = (T)0.6234898018587335, c2 = (T)-0.2225209339563144, c3 = (T)-0.9009688679024191;
-        const T s1 = (T)0.7818314824680298, s2 = (T)0.9749279121818236, s3 = (T)0.4338837391175581;
-        C t1 = cadd(a[1], a[6]), t2 = cadd(a[2], a[5]), t3 = cadd(a[3], a[4]);
-        C d1 = csub(a[1], a[6]), d2 = csub(a[2], a[5]), d3 = csub(a[3], a[4]);
-        C x0 = a[0];
-        C b1 = mk(x0.x + c1 * t1.x + c2 * t2.x + c3 * t3.x, x0.y + c1 * t1.y + c2 * t2.y + c3 * t3.y);
-        C b2 = mk(x0.x + c2 * t1.x + c3 * t2.x + c1 * t3.x, x0.y + c2 * t1.y + c3 * t2.y + c1 * t3.y);
-        C b3 = mk(x0.x + c3 * t1.x + c1 * t2.x + c2 * t3.x, x0.y + c3 * t1.y + c1 * t2.y + c2 * t3.y);
-        C e1 = mk(s1 * d1.x + s2 * d2.x + s3 * d3.x, s1 * d1.y + s2 * d2.y + s3 * d3.y);
-        C e2 = mk(s2 * d1.x - s3 * d2.x - s1 * d3.x, s2 * d1.y - s3 * d2.y - s1 * d3.y);
-        C e3 = mk(s3 * d1.x - s1 * d2.x + s2 * d3.x, s3 * d1.y - s1 * d2.y + s2 * d3.y);
-        a[0] = cadd(x0, cadd(t1, cadd(t2, t3)));
-        C i1 = cmul_i(e1), i2 = cmul_i(e2), i3 = cmul_i(e3);
-        if (!INV) {
-            a[1] = csub(b1, i1); a[6] = cadd(b1, i1);
-            a[2] = csub(b2, i2); a[5] = cadd(b2, i2);
-            a[3] = csub(b3, i3); a[4] = cadd(b3, i3);
-        } else {
-            a[1] = cadd(b1, i1); a[6] = csub(b1, i1);
-            a[2] = cadd(b2, i2); a[5] = csub(b2, i2);
-            a[3] = cadd(b3, i3); a[4] = csub(b3, i3);
-        }
-    }
-};
-
-// Composite radix R = R1*R2 in registers: R2 DFTs of size R1 over
-// a[n2 + R2*n1], twiddles W_R^{n2*k1} (compile-time constants), then R1 DFTs
-// of size R2; output X[k1 + R1*k2].
-template <int R1, int R2, bool INV, typename T> struct DftComp {
-    using C = cplx_t<T>;
-    static constexpr int R = R1 * R2;
-    __device__ __forceinline__ static void run(C* a) {
-        C y[R];
-#pragma unroll
-        for (int n2 = 0; n2 < R2; ++n2) {
-            C t[R1];
-#pragma unroll
-            for (int n1 = 0; n1 < R1; ++n1) t[n1] = a[n2 + R2 * n1];
-            Dft<R1, INV, T>::run(t);
-#pragma unroll
-            for (int k1 = 0; k1 < R1; ++k1) {
-                const int m = (n2 * k1) % R;
-                C v = t[k1];
-                if (m != 0) {
-                    const C w = mk((T)RootTab<R>::re(m), (T)RootTab<R>::im(m));
-                    v = INV ? cmulc(v, w) : cmul(v, w);
-                }
-                y[k1 * R2 + n2] = v;
-            }
-        }
-#pragma unroll
-        for (int k1 = 0; k1 < R1; ++k1) {
-            C t[R2];
-#pragma unroll
-            for (int n2 = 0; n2 < R2; ++n2) t[n2] = y[k1 * R2 + n2];
-            Dft<R2, INV, T>::run(t);
-#pragma unroll
-            for (int k2 = 0; k2 < R2; ++k2) a[k1 + R1 * k2] = t[k2];
-        }
-    }
-};
-
-template <bool INV, typename T> struct Dft<6, INV, T> : DftComp<2, 3, INV, T> {};
-template <bool INV, typename T> struct Dft<9, INV, T> : DftComp<3, 3, INV, T> {};
-template <bool INV, typename T> struct Dft<10, INV, T> : DftComp<2, 5, INV, T> {};
-template <bool INV, typename T> struct Dft<12, INV, T> : DftComp<4, 3, INV, T> {};
-template <bool INV, typename T> struct Dft<15, INV, T> : DftComp<3, 5, INV, T> {};
-template <bool INV, typename T> struct Dft<16, INV, T> : DftComp<4, 4, INV, T> {};
-template <bool INV, typename T> struct Dft<20, INV, T> : DftComp<4, 5, INV, T> {};
-template <bool INV, typename T> struct Dft<25, INV, T> : DftComp<5, 5, INV, T> {};
-template <bool INV, typename T> struct Dft<32, INV, T> : DftComp<8, 4, INV, T> {};
-template <bool INV, typename T> struct Dft<18, INV, T> : DftComp<2, 9, INV, T> {};
-template <bool INV, typename T> struct Dft<24, INV, T> : DftComp<8, 3, INV, T> {};
-template <bool INV, typename T> struct Dft<27, INV, T> : DftComp<3, 9, INV, T> {};
-template <bool INV, typename T> struct Dft<30, INV, T> : DftComp<5, 6, INV, T> {};
-
-// ------------------------------------------------------------------- stages
-template <typename T, int R, bool INV>
-__device__ __forceinline__ void stage_pp(const cplx_t<T>* __restrict__ in, cplx_t<T>* __restrict__ out, int L, int TB,
-                                         int TBP, int Ns, const cplx_t<T>* __restrict__ tw, int step) {
-    using C = cplx_t<T>;
-    const int m = L / R;
-    const int nitems = TB * m;
-    for (int w = threadIdx.x; w < nitems; w += blockDim.x) {
-        const int b = w % TB, u = w / TB, k = u % Ns;
-        C v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[(u + r * m) * TBP + b];
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = twmul<INV>(v[r], tw[k * r * step]);
-        }
-        Dft<R, INV, T>::run(v);
-        const int o = ((u - k) * R + k) * TBP + b;
-#pragma unroll
-        for (int r = 0; r < R; ++r) out[o + r * Ns * TBP] = v[r];
-    }
-}
-
-// direct DFT of an arbitrary (prime) radix p: one output per loop trip
-template <typename T, bool INV>
-__device__ __forceinline__ void stage_generic_pp(const cplx_t<T>* __restrict__ in, cplx_t<T>* __restrict__ out, int L,
-                                                 int TB, int TBP, int Ns, int p, const cplx_t<T>* __restrict__ tw,
-                                                 int step, int Ltab) {
-    using C = cplx_t<T>;
-    const int m = L / p;
-    const int nitems = TB * L;   // (b, u, r_out)
-    for (int w = threadIdx.x; w < nitems; w += blockDim.x) {
-        const int b = w % TB, rest = w / TB;
-        const int u = rest % m, ro = rest / m, k = u % Ns;
-        // exponent of input t: t*step*(k + ro*Ns)  (mod Ltab)
-        const int e0 = (int)(((long long)step * (k + ro * Ns)) % Ltab);
-        C acc = mk((T)0, (T)0);
-        int e = 0;
-        for (int t = 0; t < p; ++t) {
-            acc = cadd(acc, twmul<INV>(in[(u + t * m) * TBP + b], tw[e]));
-            e += e0;
-            if (e >= Ltab) e -= Ltab;
-        }
-        out[((u - k) * p + k + ro * Ns) * TBP + b] = acc;
-    }
-}
 
 template <typename T, int R, bool INV>
 __device__ __forceinline__ void stage_ip(cplx_t<T>* __restrict__ buf, int L, int TB, int TBP, int Ns,
@@ -329,55 +430,27 @@ __device__ __forceinline__ void load_radices(const FftPlanDev& pl, int* s_rad) {
         if (threadIdx.x == s) s_rad[s] = pl.rad[s];
 }
 
-// Full transform of TB interleaved lines of length L.  PP: data starts in
-// `buf`, `alt` is the second buffer; returns the buffer holding the result.
-// In place (PP == false): `alt` is unused and `buf` is returned.
-// Every thread of the block must call this (it contains barriers).
-template <typename T, bool INV, bool PP>
-__device__ cplx_t<T>* fft_lines(cplx_t<T>* buf, cplx_t<T>* alt, const int* s_rad, int nst, int L, int TB, int TBP,
-                                const cplx_t<T>* __restrict__ tw, int Ltab) {
+// Full transform of TB interleaved lines of length L in place.  Every thread
+// of the block must call this (it contains barriers).
+template <typename T, bool INV>
+__device__ void fft_lines_ip(cplx_t<T>* buf, const int* s_rad, int nst, int L, int TB, int TBP,
+                             const cplx_t<T>* __restrict__ tw, int Ltab) {
     int Ns = 1;
-    cplx_t<T>* in = buf;
-    cplx_t<T>* out = alt;
 #pragma unroll 1
     for (int s = 0; s < nst; ++s) {
         const int R = s_rad[s];
         const int step = Ltab / (Ns * R);
-        if (PP) {
-            switch (R) {
-                case 2: stage_pp<T, 2, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 3: stage_pp<T, 3, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 4: stage_pp<T, 4, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 5: stage_pp<T, 5, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 6: stage_pp<T, 6, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 7: stage_pp<T, 7, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 8: stage_pp<T, 8, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 9: stage_pp<T, 9, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 10: stage_pp<T, 10, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 12: stage_pp<T, 12, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 15: stage_pp<T, 15, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 16: stage_pp<T, 16, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 20: stage_pp<T, 20, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 25: stage_pp<T, 25, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                case 32: stage_pp<T, 32, INV>(in, out, L, TB, TBP, Ns, tw, step); break;
-                default: stage_generic_pp<T, INV>(in, out, L, TB, TBP, Ns, R, tw, step, Ltab); break;
-            }
-            __syncthreads();
-            cplx_t<T>* t = in; in = out; out = t;
-        } else {
-            switch (R) {
-                case 2: stage_ip<T, 2, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                case 3: stage_ip<T, 3, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                case 4: stage_ip<T, 4, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                case 5: stage_ip<T, 5, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                case 7: stage_ip<T, 7, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                case 8: stage_ip<T, 8, INV>(buf, L, TB, TBP, Ns, tw, step); break;
-                default: stage_generic_ip<T, INV>(buf, L, TB, TBP, Ns, R, tw, step, Ltab); break;
-            }
+        switch (R) {
+            case 2: stage_ip<T, 2, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            case 3: stage_ip<T, 3, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            case 4: stage_ip<T, 4, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            case 5: stage_ip<T, 5, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            case 7: stage_ip<T, 7, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            case 8: stage_ip<T, 8, INV>(buf, L, TB, TBP, Ns, tw, step); break;
+            default: stage_generic_ip<T, INV>(buf, L, TB, TBP, Ns, R, tw, step, Ltab); break;
         }
         Ns *= R;
     }
-    return PP ? in : buf;
 }
 
 }  // namespace csipm

@@ -231,6 +231,128 @@ CSIPM_HD MapEntry decode(const Geom& g, int i, int j, int k) {
     return g.dim == 3 ? decode3(g, i, j, k) : (g.dim == 2 ? decode2(g, i, j) : decode1(g, i));
 }
 
+// ---------------------------------------------------------------- lines along dim 2
+// The beta indices of a whole line j = 0..N2-1 at fixed (i, k): below and above
+// N2/2 they are affine in j, so a pass that walks lines along dim 2 decodes once
+// per line and then takes a multiply-add per element instead of the class tests
+// of decode() (which made the reference-order gather and scatter integer-bound).
+//   re(j) = re0 (j = 0), reH (j = N2/2), bL + j*sL (below), bU + j*sU (above)
+//   im(j) = re(j) + imoE (j = 0, N2/2), + imo (otherwise)
+struct LineMap {
+    int m2;
+    int bL, sL, bU, sU, imo;
+    int re0, reH, imoE;
+    unsigned fl;
+};
+enum : unsigned { LM_MINUS_L = 1, LM_MINUS_U = 2, LM_MINUS_E = 4, LM_VERT_E = 8, LM_SRC_L = 16, LM_SRC_U = 32,
+                  LM_SRC_E = 64 };
+
+// sol: solver order (geometry below); its interior lines are pairs, so only
+// the planes i = 0 and i = M1 are meant there.
+CSIPM_HD LineMap make_line(const Geom& g, int i, int k, bool sol) {
+    LineMap l;
+    l.m2 = g.m2;
+    l.fl = LM_SRC_L | LM_SRC_U | LM_SRC_E;
+    if (i >= 1 && i <= g.m1 - 1) {
+        const int ti = i - 1, tm = g.m1 - i - 1, p1 = g.p1;
+        l.sL = l.sU = p1;
+        if (g.dim == 2) {
+            l.bL = g.o2C - p1 + ti;
+            l.bU = g.o2C + 2 * g.PP - (g.m2 + 1) * p1 + ti;
+            l.imo = g.PP;
+            l.re0 = g.o2E1 + ti;
+            l.reH = l.re0 + 2 * p1;
+            l.imoE = p1;
+        } else {
+            const int ck = coord_class(k, g.m3);
+            if (ck <= 1) {
+                const int o = g.oFk + 4 * ck * g.P12;
+                l.bL = o - p1 + ti;
+                l.bU = o + 2 * g.P12 + (g.n2 - 1) * p1 + tm;
+                l.sU = -p1;
+                l.imo = g.P12;
+                l.re0 = g.oE1 + 2 * ck * p1 + ti;
+                l.reH = l.re0 + 4 * p1;
+                l.imoE = p1;
+                l.fl |= LM_MINUS_U;
+            } else if (ck == 2) {
+                l.bL = g.oC + (k - 1) * g.P12 - p1 + ti;
+                l.bU = g.oC + 4 * g.P123 + (k - 1) * g.P12 - (g.m2 + 1) * p1 + ti;
+                l.imo = g.P123;
+                l.re0 = g.oFj + (k - 1) * p1 + ti;
+                l.reH = l.re0 + 4 * g.P13;
+                l.imoE = g.P13;
+            } else {
+                const int kk = g.n3 - k - 1;
+                l.sL = l.sU = -p1;
+                l.bL = g.oC + 6 * g.P123 + kk * g.P12 + (g.m2 - 1) * p1 + tm;
+                l.bU = g.oC + 2 * g.P123 + kk * g.P12 + (g.n2 - 1) * p1 + tm;
+                l.imo = g.P123;
+                l.re0 = g.oFj + 2 * g.P13 + kk * p1 + tm;
+                l.reH = l.re0 + 4 * g.P13;
+                l.imoE = g.P13;
+                l.fl |= LM_MINUS_L | LM_MINUS_U | LM_MINUS_E;
+            }
+        }
+        return l;
+    }
+    const int ci = i == 0 ? 0 : 1;
+    int shE = 0, shLU = 0;   // solver order: the tail's place of the block
+    if (sol) shE = shLU = (int)(2 * g.NI);
+    l.sL = 1;
+    l.sU = -1;
+    const int ck = g.dim == 2 ? 0 : coord_class(k, g.m3);
+    if (ck <= 1) {
+        l.re0 = g.dim == 2 ? 2 * ci : 4 * ci + ck;
+        l.reH = g.dim == 2 ? 2 * ci + 1 : 4 * ci + 2 + ck;
+        l.imoE = 0;
+        const int base = g.dim == 2 ? 4 + 2 * ci * g.p2 : g.oE2 + 2 * (2 * ci + ck) * g.p2;
+        l.bL = base - 1;
+        l.bU = base + g.n2 - 1;
+        l.imo = g.p2;
+        l.fl = LM_VERT_E | LM_MINUS_U | LM_SRC_E | LM_SRC_L;
+    } else {
+        const int kk = ck == 2 ? k - 1 : g.n3 - k - 1;
+        l.re0 = 8 + 4 * ci * g.p3 + kk;
+        l.reH = l.re0 + 2 * g.p3;
+        l.imoE = g.p3;
+        const int o = g.oFi + 4 * ci * g.P23 + kk * g.p2;
+        l.imo = g.P23;
+        if (ck == 2) {
+            l.bL = o - 1;
+            l.bU = o + 2 * g.P23 - (g.m2 + 1);
+            l.sU = 1;
+        } else {
+            l.bL = o + 2 * g.P23 + g.m2 - 1;
+            l.bU = o + g.n2 - 1;
+            l.sL = -1;
+            l.fl = LM_MINUS_L | LM_MINUS_U | LM_MINUS_E;
+        }
+        if (sol) shLU += g.oE1 - g.oFi;
+    }
+    l.re0 += shE;
+    l.reH += shE;
+    l.bL += shLU;
+    l.bU += shLU;
+    return l;
+}
+
+CSIPM_HD MapEntry line_at(const LineMap& l, int j) {
+    const bool lo = j < l.m2, e = j == 0 || j == l.m2;
+    MapEntry o;
+    o.re = lo ? l.bL + j * l.sL : l.bU + j * l.sU;
+    if (e) o.re = j == 0 ? l.re0 : l.reH;
+    o.im = o.re + (e ? l.imoE : l.imo);
+    const unsigned f = e ? l.fl >> 2 : (lo ? l.fl : l.fl >> 1);   // bit 0: minus, bit 4: source
+    o.kind = (f & 1u) ? KIND_MINUS : KIND_PLUS;
+    o.src = (f >> 4) & 1u;
+    if (e && (l.fl & LM_VERT_E)) {
+        o.kind = KIND_VERT;
+        o.im = -1;
+    }
+    return o;
+}
+
 // ---------------------------------------------------------------- solver order
 // The interior-point solve keeps its beta-space vectors in a "solver order"
 // that follows the half spectrum instead of the reference packing:

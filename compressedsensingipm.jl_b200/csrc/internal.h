@@ -14,12 +14,22 @@
 #include "../../include/csipm.h"
 #include "geometry.h"
 #include "fft2.cuh"
-#include "operator.cuh"
+#include "passes.cuh"
 #include "solver_kernels.cuh"
 #include "long1d.cuh"
 #include <type_traits>
 
 namespace csipm {
+template <typename T>
+inline void FftOperator<T>::choose_two_level() {
+    s2_A = s2_B = s3_A = s3_B = r_A = r_B = 0;
+    if (g.dim < 2) return;
+    int A = 0, B = 0;
+    if (fft2_factor(g.n2, &A, &B) && fft2_strided_pair(A, B)) { s2_A = A; s2_B = B; }
+    if (g.dim == 3 && fft2_factor(g.n3, &A, &B) && fft2_strided_pair(A, B)) { s3_A = A; s3_B = B; }
+    if (fft2_factor(g.m1, &A, &B) && fft2_row_pair(A, B)) { r_A = A; r_B = B; }
+}
+
 void set_last_error(const std::string& msg);
 const char* get_last_error();
 
@@ -112,7 +122,6 @@ struct csipm_handle_s {
     double* b = nullptr;            // A^T z0
     bool sorder = false;            // solve runs in solver order (geometry.h)
     double* bs = nullptr;           // A^T z0 in solver order (when sorder)
-    int4* pmap = nullptr;           // solver-order plane map (when sorder)
     double *beta = nullptr, *c = nullptr, *z1 = nullptr, *z2 = nullptr, *Qb = nullptr, *rd = nullptr;
     double *s1 = nullptr, *s2 = nullptr;    // slacks c + beta, c - beta (stored; c is output scratch)
     double *Db = nullptr, *Minv = nullptr, *rhs = nullptr, *dba = nullptr, *db = nullptr;
@@ -225,7 +234,7 @@ enum { SL_RED = 0, SL_MAXB = 16, SL_SS = 24, SL_DUMMY = 32, SL_DOT = 40, SL_SIGM
 // ------------------------------------------------------------------ pass dispatch
 // Strided pass along `axis`: the two-level register kernel when the axis has
 // an instantiated factor pair and the epilogue is a hot-path one, else the
-// persistent Stockham kernel.
+// run-time-plan kernel.
 template <typename T, bool INV, int IN, int OUT, typename TS, class Epi>
 cudaError_t run_strided(FftOperator<T>& op, int axis, const PassArgs<T>& a, const TS* src, const Epi& epi,
                         cudaStream_t st) {
@@ -233,29 +242,24 @@ cudaError_t run_strided(FftOperator<T>& op, int axis, const PassArgs<T>& a, cons
         const int A = axis == 3 ? op.s3_A : op.s2_A, B = axis == 3 ? op.s3_B : op.s2_B;
         if (A) return launch_strided2<T, INV, IN, OUT, TS, Epi>(A, B, a, src, epi, st);
     }
-    if constexpr (IN == IN_SGATHER || OUT == OUT_SSCATTER) {
-        return cudaErrorInvalidValue;   // solver order runs on the two-level kernels only
-    } else {
-        return launch_strided<T, INV, IN, OUT>(axis == 3 ? op.s3_cfg : op.s2_cfg, a, src, epi, st);
-    }
+    return launch_strided<T, INV, IN, OUT>(axis == 3 ? op.s3_cfg : op.s2_cfg, a, src, epi, st);
 }
 
-// Row pass: the two-level kernel for 2D/3D spectrum/real passes with an
-// instantiated factor pair, else the Stockham kernel (also all 1D passes).
-template <typename T, int IN, int OUT, bool MASK, typename TS, class Epi>
-cudaError_t run_row(FftOperator<T>& op, const PassArgs<T>& a, const TS* src, const Epi& epi, cudaStream_t st) {
+// Row pass (2D/3D): the two-level kernel for an instantiated factor pair,
+// else the run-time-plan kernel.
+template <typename T, int IN, int OUT, bool MASK>
+cudaError_t run_row(FftOperator<T>& op, const PassArgs<T>& a, cudaStream_t st) {
     if constexpr (Fft2R<T, IN, OUT, MASK>::value) {
-        if (op.r_A && op.g.dim >= 2) return launch_row2<T, IN, OUT, MASK>(op.r_A, op.r_B, a, st);
+        if (op.r_A) return launch_row2<T, IN, OUT, MASK>(op.r_A, op.r_B, a, st);
     }
-    return launch_row<T, IN, OUT, MASK>(op.row_cfg, a, src, epi, st);
+    return launch_row<T, IN, OUT, MASK>(op.row_cfg, a, st);
 }
 
 // True when beta-space vectors of the solve can be kept in solver order
-// (geometry.h): the gather and scatter passes along dim 2 then run on the
-// two-level kernels.
+// (geometry.h).
 template <typename T>
 inline bool solver_order_ok(const FftOperator<T>& op) {
-    return op.g.dim >= 2 && op.s2_A != 0;
+    return op.g.dim >= 2;
 }
 
 // ------------------------------------------------------------------ operator
@@ -274,26 +278,21 @@ cudaError_t op_AtA(FftOperator<T>& op, const TS* x, const Epi& epi, const int* s
     constexpr int SOUT = SOL ? OUT_SSCATTER : OUT_SCATTER;
     if constexpr (SOL) {
         if (!solver_order_ok(op)) return cudaErrorInvalidValue;
-    } else if (g.dim == 1 && op.l1P) {
+    } else if (g.dim == 1) {
         e = l1d_first(op, x, skip, st);
         if (e != cudaSuccess) return e;
         e = mask ? l1d_row<T, IN_SPEC, OUT_SPEC, true>(op, sc, nullptr, nullptr, skip, st)
                  : l1d_row<T, IN_SPEC, OUT_SPEC, false>(op, sc, nullptr, nullptr, skip, st);
         if (e != cudaSuccess) return e;
-        e = l1d_lines_forward(op, skip, st);
-        if (e != cudaSuccess) return e;
-        return l1d_post(op, epi, skip, st);
-    } else if (g.dim == 1) {
-        return mask ? run_row<T, IN_GATHER, OUT_SCATTER, true>(op, ra, x, epi, st)
-                    : run_row<T, IN_GATHER, OUT_SCATTER, false>(op, ra, x, epi, st);
+        return l1d_last(op, epi, skip, st);
     }
     if (g.dim == 2) {
         PassArgs<T> a2 = op.strided_args(2);
         a2.skip = skip;
         e = run_strided<T, true, GIN, OUT_SPEC>(op, 2, a2, x, none, st);
         if (e != cudaSuccess) return e;
-        e = mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, (const double*)nullptr, none, st)
-                 : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, (const double*)nullptr, none, st);
+        e = mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, st)
+                 : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, st);
         if (e != cudaSuccess) return e;
         return run_strided<T, false, IN_SPEC, SOUT>(op, 2, a2, (const double*)nullptr, epi, st);
     }
@@ -306,8 +305,8 @@ cudaError_t op_AtA(FftOperator<T>& op, const TS* x, const Epi& epi, const int* s
     if (e != cudaSuccess) return e;
     e = run_strided<T, true, IN_SPEC, OUT_SPEC>(op, 3, a3, (const double*)nullptr, none, st);
     if (e != cudaSuccess) return e;
-    e = mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, (const double*)nullptr, none, st)
-             : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, (const double*)nullptr, none, st);
+    e = mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, st)
+             : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, st);
     if (e != cudaSuccess) return e;
     e = run_strided<T, false, IN_SPEC, OUT_SPEC>(op, 3, a3, (const double*)nullptr, none, st);
     if (e != cudaSuccess) return e;
@@ -322,15 +321,12 @@ cudaError_t op_A(FftOperator<T>& op, const TS* beta, T* x, cudaStream_t st) {
     EpiStore<double> none{nullptr};
     PassArgs<T> ra = op.row_args(1.0 / std::sqrt((double)g.N), nullptr, x);
     cudaError_t e;
-    if (g.dim == 1 && op.l1P) {
+    if (g.dim == 1) {
         e = l1d_first(op, beta, nullptr, st);
         if (e != cudaSuccess) return e;
         return mask ? l1d_row<T, IN_SPEC, OUT_REAL, true>(op, ra.scale, nullptr, x, nullptr, st)
                     : l1d_row<T, IN_SPEC, OUT_REAL, false>(op, ra.scale, nullptr, x, nullptr, st);
     }
-    if (g.dim == 1)
-        return mask ? run_row<T, IN_GATHER, OUT_REAL, true>(op, ra, beta, none, st)
-                    : run_row<T, IN_GATHER, OUT_REAL, false>(op, ra, beta, none, st);
     if (g.dim == 3) {
         e = run_strided<T, true, IN_GATHER, OUT_SPEC>(op, 2, op.strided_args(2), beta, none, st);
         if (e != cudaSuccess) return e;
@@ -339,8 +335,8 @@ cudaError_t op_A(FftOperator<T>& op, const TS* beta, T* x, cudaStream_t st) {
         e = run_strided<T, true, IN_GATHER, OUT_SPEC>(op, 2, op.strided_args(2), beta, none, st);
     }
     if (e != cudaSuccess) return e;
-    return mask ? run_row<T, IN_SPEC, OUT_REAL, true>(op, ra, (const double*)nullptr, none, st)
-                : run_row<T, IN_SPEC, OUT_REAL, false>(op, ra, (const double*)nullptr, none, st);
+    return mask ? run_row<T, IN_SPEC, OUT_REAL, true>(op, ra, st)
+                : run_row<T, IN_SPEC, OUT_REAL, false>(op, ra, st);
 }
 
 // beta = B^T(fft(z)/sqrt(N)) through the epilogue
@@ -350,15 +346,12 @@ cudaError_t op_At(FftOperator<T>& op, const T* z, const Epi& epi, cudaStream_t s
     EpiStore<double> none{nullptr};
     PassArgs<T> ra = op.row_args(1.0 / (2.0 * std::sqrt((double)g.N)), z, nullptr);
     cudaError_t e;
-    if (g.dim == 1 && op.l1P) {
+    if (g.dim == 1) {
         e = l1d_row<T, IN_REAL, OUT_SPEC, false>(op, ra.scale, z, nullptr, nullptr, st);
         if (e != cudaSuccess) return e;
-        e = l1d_lines_forward(op, nullptr, st);
-        if (e != cudaSuccess) return e;
-        return l1d_post(op, epi, nullptr, st);
+        return l1d_last(op, epi, nullptr, st);
     }
-    if (g.dim == 1) return run_row<T, IN_REAL, OUT_SCATTER, false>(op, ra, (const double*)nullptr, epi, st);
-    e = run_row<T, IN_REAL, OUT_SPEC, false>(op, ra, (const double*)nullptr, none, st);
+    e = run_row<T, IN_REAL, OUT_SPEC, false>(op, ra, st);
     if (e != cudaSuccess) return e;
     if (g.dim == 2) return run_strided<T, false, IN_SPEC, OUT_SCATTER>(op, 2, op.strided_args(2), (const double*)nullptr, epi, st);
     e = run_strided<T, false, IN_SPEC, OUT_SPEC>(op, 3, op.strided_args(3), (const double*)nullptr, none, st);
@@ -369,7 +362,7 @@ cudaError_t op_At(FftOperator<T>& op, const T* z, const Epi& epi, cudaStream_t s
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 inline int passes_per_product(const Geom& g) {
-    return g.dim == 3 ? 5 : (g.dim == 2 ? 3 : (g.m1 > L1D_MIN_M ? 4 : 1));
+    return g.dim == 3 ? 5 : 3;
 }
 
 inline int read_slots(csipm_handle h, int first, int count) {

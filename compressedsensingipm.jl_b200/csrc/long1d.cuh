@@ -1,5 +1,5 @@
-// Long 1D rows: the real FFT of length N1 = 2M runs its length-M complex FFT
-// as M = P*Q (four-step) over many CTAs instead of one row per CTA.
+// 1D: the real FFT of length N1 = 2M runs its length-M complex FFT as
+// M = P*Q (four-step) over many CTAs.
 //
 // Spectrum index k = k1 + P*k2 (k1 < P, k2 < Q), spatial index n = n2 + Q*n1.
 // With W = exp(+2 pi i / M) for the inverse transform:
@@ -14,175 +14,259 @@
 //           scaled and masked -> (A: store the real samples) or forward
 //           DFT_P -> twiddle w_M^{n2 k1} -> spec[k1 + P n2]
 //           (A^T: the row starts from the real samples instead)
-//   lines:  forward DFT_Q along k2 (the ordinary strided pass)
-//   post:   R2C post-processing of Z[k], Z[M-k] -> scatter to beta
+//   last:   lines k1 and their mirrors P - k1 together: forward DFT_Q along
+//           k2, then Z[k] and Z[M-k] are both in the tile: R2C
+//           post-processing -> scatter to beta with the epilogue
 //
 // w_M^e = exp(-2 pi i e / M) is read from the N1-th root table (index 2e).
+//
+// The passes are bound by latency, not bandwidth (1D vectors of the serving
+// range sit in L2), so what counts is launches and the chain inside one:
+// three launches where four kernels ran (a plain lines pass, then the post-
+// processing over all k), and register-radix stages (fft_device.cuh) with
+// loads and stores attached to the first and last stage.
 #pragma once
-#include "operator.cuh"
+#include "passes.cuh"
 
 namespace csipm {
 
-// ---------------------------------------------------------------- first pass
-// TB lines k1 per CTA (l1d_tiles), interleaved in shared memory as buf[x*TB + b].
+// beta of spectrum position k (0 <= k <= M), 1D packing
 template <typename T, typename TS>
-__device__ __forceinline__ void l1d_first_kernel_body(PassArgs<T> a, const TS* __restrict__ src,
-                                                        const cplx_t<T>* __restrict__ twN, int P, int Q, int TB) {
+__device__ __forceinline__ cplx_t<T> gather1(const TS* __restrict__ src, int M, int k) {
+    const bool vert = k == 0 || k == M;
+    const T a = (T)src[k == 0 ? 0 : (k == M ? 1 : k + 1)], b = (T)src[vert ? 0 : M + k];
+    const T r = (T)0.7071067811865476;
+    return vert ? mk(a, (T)0) : mk(a * r, b * r);
+}
+
+// ---------------------------------------------------------------- first pass
+template <typename T, typename TS>
+struct L1dFirst {
     using C = cplx_t<T>;
+    const TS* src;
+    C* spec;
+    const C* twN;
+    int M, P, k1;
+    __device__ __forceinline__ C one(int x, int) const {
+        if (k1 >= P) return mk((T)0, (T)0);
+        const int k = k1 + P * x;
+        return c2r_pre(gather1<T>(src, M, k), gather1<T>(src, M, M - k), twN[k]);
+    }
+    __device__ __forceinline__ void one(int x, int, C v) const {
+        if (k1 >= P) return;
+        const int ex = x * k1;   // < M
+        spec[k1 + (size_t)P * x] = ex ? cmulc(v, twN[2 * ex]) : v;
+    }
+    template <int R> __device__ __forceinline__ void load(C* v, int u, int m, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = one(u + r * m, b);
+    }
+    template <int R> __device__ __forceinline__ void store(const C* v, int u, int Ns, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) one(u + r * Ns, b, v[r]);
+    }
+};
+
+template <typename T, typename TS>
+__device__ __forceinline__ void l1d_first_kernel_body(const PassArgs<T>& a, const TS* __restrict__ src,
+                                                      const cplx_t<T>* __restrict__ twN, int P) {
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* buf = reinterpret_cast<C*>(smem_raw);
-    C* work = buf + Q * TB;
-    __shared__ int s_rad[FFT_MAX_STAGES];
-    load_radices(a.pl, s_rad);
-    const int M = a.g.m1;
-    const int i0 = blockIdx.x * TB;
-    for (int e = threadIdx.x; e < Q * TB; e += blockDim.x) {
-        const int x = e / TB, b = e % TB;
-        const int k1 = i0 + b;
-        C v = mk((T)0, (T)0);
-        if (k1 < P) {
-            const int k = k1 + P * x;
-            const C xa = gather_val<T>(decode1(a.g, k), src);
-            const C xb = gather_val<T>(decode1(a.g, M - k), src);
-            v = c2r_pre(xa, xb, twN[k]);
-        }
-        buf[e] = v;
-    }
-    __syncthreads();
-    C* res = fft_lines<T, true, true>(buf, work, s_rad, a.pl.nst, Q, TB, TB, a.tw, a.Ltab);
-    for (int e = threadIdx.x; e < Q * TB; e += blockDim.x) {
-        const int x = e / TB, b = e % TB;
-        const int k1 = i0 + b;
-        if (k1 < P) {
-            C v = res[e];
-            const int ex = x * k1;   // < M
-            if (ex) v = cmulc(v, twN[2 * ex]);
-            a.spec[k1 + (size_t)P * x] = v;
-        }
+    FftTile<cplx_t<T>> t = make_tile(a, smem_raw);
+    const int b = threadIdx.x & ((1 << a.lay.lg) - 1);
+    for (int i0 = blockIdx.x << a.lay.lg; i0 < P; i0 += gridDim.x << a.lay.lg) {
+        L1dFirst<T, TS> io{src, a.spec, twN, a.g.m1, P, i0 + b};
+        fft_through<T, true>(t, io, io);
+        __syncthreads();
     }
 }
 template <typename T, typename TS>
-__global__ void __launch_bounds__(256) l1d_first_kernel(PassArgs<T> a, const TS* __restrict__ src,
-                                                        const cplx_t<T>* __restrict__ twN, int P, int Q, int TB) {
-    l1d_first_kernel_body<T, TS>(a, src, twN, P, Q, TB);
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
+l1d_first_kernel(const __grid_constant__ PassArgs<T> a, const TS* __restrict__ src, const cplx_t<T>* __restrict__ twN, int P) {
+    l1d_first_kernel_body<T, TS>(a, src, twN, P);
 }
 
 // ------------------------------------------------------------------ row pass
-// RB rows n2 per CTA, interleaved in shared memory as buf[n1*RB + b].
+// one row n2: P contiguous spectrum values, or the real samples n2 + Q n1
+template <typename T, bool MASK>
+struct L1dRow {
+    using C = cplx_t<T>;
+    C* spec;             // of this row
+    const T* in;
+    T* out;
+    const uint32_t* mask;
+    const C* twN;
+    int n2, Q;
+    T sc;
+    bool live;
+    __device__ __forceinline__ C keep(int n1, C y) const {
+        y.x *= sc;
+        y.y *= sc;
+        if (MASK && live) {
+            const int n = n2 + Q * n1;
+            const uint32_t w = mask[n >> 4];
+            const int sh = (2 * n) & 31;
+            if (!((w >> sh) & 1u)) y.x = (T)0;
+            if (!((w >> (sh + 1)) & 1u)) y.y = (T)0;
+        }
+        return y;
+    }
+};
+template <typename T, bool MASK>
+struct L1dRowSpec : L1dRow<T, MASK> {   // spectrum in, twiddled spectrum out
+    using C = cplx_t<T>;
+    __device__ __forceinline__ C one(int k1, int) const { return this->live ? this->spec[k1] : mk((T)0, (T)0); }
+    __device__ __forceinline__ void one(int k1, int, C v) const {
+        if (!this->live) return;
+        const int ex = this->n2 * k1;   // < M
+        this->spec[k1] = ex ? cmul(v, this->twN[2 * ex]) : v;
+    }
+    template <int R> __device__ __forceinline__ void load(C* v, int u, int m, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = one(u + r * m, b);
+    }
+    template <int R> __device__ __forceinline__ void store(const C* v, int u, int Ns, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) one(u + r * Ns, b, v[r]);
+    }
+};
+template <typename T, bool MASK>
+struct L1dRowReal : L1dRow<T, MASK> {   // real samples
+    using C = cplx_t<T>;
+    __device__ __forceinline__ C one(int n1, int) const {
+        if (!this->live) return mk((T)0, (T)0);
+        return this->keep(n1, *reinterpret_cast<const C*>(this->in + 2 * ((size_t)this->n2 + (size_t)this->Q * n1)));
+    }
+    __device__ __forceinline__ void one(int n1, int, C v) const {
+        if (this->live) *reinterpret_cast<C*>(this->out + 2 * ((size_t)this->n2 + (size_t)this->Q * n1)) = this->keep(n1, v);
+    }
+    template <int R> __device__ __forceinline__ void load(C* v, int u, int m, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = one(u + r * m, b);
+    }
+    template <int R> __device__ __forceinline__ void store(const C* v, int u, int Ns, int b) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) one(u + r * Ns, b, v[r]);
+    }
+};
+
 template <typename T, int IN, int OUT, bool MASK>
-__device__ __forceinline__ void l1d_row_kernel_body(PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P,
-                                                      int Q, int RB) {
+__device__ __forceinline__ void l1d_row_kernel_body(const PassArgs<T>& a, const cplx_t<T>* __restrict__ twN, int P,
+                                                    int Q) {
     using C = cplx_t<T>;
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* buf = reinterpret_cast<C*>(smem_raw);
-    C* work = buf + P * RB;
-    __shared__ int s_rad[FFT_MAX_STAGES];
-    load_radices(a.pl, s_rad);
-    const int r0 = blockIdx.x * RB;
-    const int nr = min(RB, Q - r0);
-    if (IN == IN_REAL) {
-        // z[n] = (x[2n], x[2n+1]) with n = n2 + Q n1: consecutive rows are consecutive n
-        for (int e = threadIdx.x; e < P * RB; e += blockDim.x) {
-            const int b = e % RB, n1 = e / RB;
-            buf[n1 * RB + b] = b < nr ? *reinterpret_cast<const C*>(a.real_in + 2 * ((size_t)(r0 + b) + (size_t)Q * n1))
-                                      : mk((T)0, (T)0);
-        }
-    } else {
-        for (int e = threadIdx.x; e < P * RB; e += blockDim.x) {
-            const int b = e / P, n1 = e % P;
-            buf[n1 * RB + b] = b < nr ? a.spec[(size_t)P * (r0 + b) + n1] : mk((T)0, (T)0);
-        }
-    }
-    __syncthreads();
-    C* c1 = buf;
-    C* other = work;
-    if (IN != IN_REAL) {
-        c1 = fft_lines<T, true, true>(buf, work, s_rad, a.pl.nst, P, RB, RB, a.tw, a.Ltab);
-        other = (c1 == buf) ? work : buf;
-    }
-    const T sc = (T)a.scale;
-    for (int e = threadIdx.x; e < P * RB; e += blockDim.x) {
-        const int b = e % RB, n1 = e / RB;
-        if (b < nr) {
-            const size_t n = (size_t)(r0 + b) + (size_t)Q * n1;
-            C y = c1[n1 * RB + b];
-            y.x *= sc;
-            y.y *= sc;
-            if (MASK) {
-                const uint32_t w = a.maskw[n >> 4];
-                const int sh = (int)((2 * n) & 31);
-                if (!((w >> sh) & 1u)) y.x = (T)0;
-                if (!((w >> (sh + 1)) & 1u)) y.y = (T)0;
+    FftTile<C> t = make_tile(a, smem_raw);
+    const int b = threadIdx.x & ((1 << a.lay.lg) - 1);
+    for (int r0 = blockIdx.x << a.lay.lg; r0 < Q; r0 += gridDim.x << a.lay.lg) {
+        const int n2 = r0 + b;
+        const L1dRow<T, MASK> base{a.spec + (size_t)P * n2, a.real_in, a.real_out, a.maskw, twN, n2, Q, (T)a.scale,
+                                   n2 < Q};
+        L1dRowSpec<T, MASK> sp{base};
+        L1dRowReal<T, MASK> re{base};
+        if (IN == IN_REAL) {
+            first_stage<T, false>(t, re);
+        } else {
+            t.st = a.inv;
+            first_stage<T, true>(t, sp);
+            mid_stages<T, true>(t, 1, t.nst - 1);
+            if (OUT == OUT_REAL) {
+                last_stage<T, true>(t, re);
+                __syncthreads();
+                continue;
             }
-            if (OUT == OUT_REAL) *reinterpret_cast<C*>(a.real_out + 2 * n) = y;
-            else c1[n1 * RB + b] = y;
+            chain_stage<T>(t, [&](int n1, int, C z) { return base.keep(n1, z); });
+            t.st = a.fwd;
         }
-    }
-    if (OUT == OUT_REAL) return;
-    __syncthreads();
-    C* c2 = fft_lines<T, false, true>(c1, other, s_rad, a.pl.nst, P, RB, RB, a.tw, a.Ltab);
-    for (int e = threadIdx.x; e < P * RB; e += blockDim.x) {
-        const int b = e / P, k1 = e % P;
-        if (b < nr) {
-            const int n2 = r0 + b;
-            C v = c2[k1 * RB + b];
-            const int ex = n2 * k1;   // < M
-            if (ex) v = cmul(v, twN[2 * ex]);
-            a.spec[(size_t)P * n2 + k1] = v;
-        }
+        mid_stages<T, false>(t, 1, t.nst - 1);
+        last_stage<T, false>(t, sp);
+        __syncthreads();
     }
 }
 template <typename T, int IN, int OUT, bool MASK>
-__global__ void __launch_bounds__(256) l1d_row_kernel(PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P,
-                                                      int Q, int RB) {
-    l1d_row_kernel_body<T, IN, OUT, MASK>(a, twN, P, Q, RB);
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
+l1d_row_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P, int Q) {
+    l1d_row_kernel_body<T, IN, OUT, MASK>(a, twN, P, Q);
 }
 
-// ------------------------------------------------------------------ post pass
-// X[k] from Z[k], Z[M-k] (k = 0 also gives X[M]) and the scatter to beta.
+// ----------------------------------------------------------------- last pass
+// Lanes b < TB/2 hold line i0 + b, the others the mirror P - (i0 + b - TB/2);
+// the lines 0 and P/2 are their own mirrors (their second lane idles).
+template <typename T>
+struct L1dLast {
+    using C = cplx_t<T>;
+    const C* spec;
+    int P, k1;           // k1 < 0: idle lane
+    __device__ __forceinline__ C one(int x, int) const {
+        return k1 >= 0 ? spec[k1 + (size_t)P * x] : mk((T)0, (T)0);
+    }
+    template <int R> __device__ __forceinline__ void load(C* v, int u, int m, int) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = one(u + r * m, 0);
+    }
+};
+
 template <typename T, class Epi>
-__device__ __forceinline__ void l1d_post_kernel_body(PassArgs<T> a, const cplx_t<T>* __restrict__ twN, Epi epi) {
+__device__ __forceinline__ void scatter1(int M, int k, cplx_t<T> v, Epi& ep) {
+    scatter_one<T>(MapEntry{k == 0 ? 0 : (k == M ? 1 : k + 1), M + k, (k == 0 || k == M) ? KIND_VERT : KIND_PLUS, 1}, v, ep);
+}
+
+template <typename T, class Epi>
+__device__ __forceinline__ void l1d_last_kernel_body(const PassArgs<T>& a, const cplx_t<T>* __restrict__ twN, int P,
+                                                     int Q, const Epi& epi) {
     using C = cplx_t<T>;
     if (a.skip && *a.skip) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FftTile<C> t = make_tile(a, smem_raw);
     const int M = a.g.m1;
-    const int half = M / 2;
+    const int lh = a.lay.lg - 1, TH = 1 << lh;   // pairs per tile
+    const int npair = P / 2 + 1;
+    const int b = threadIdx.x & (2 * TH - 1);
     Epi ep = epi;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= half; k += gridDim.x * blockDim.x) {
-        if (k == 0) {
-            const C z0 = a.spec[0];
-            scatter_one<T>(decode1(a.g, 0), r2c_post(z0, z0, twN[0]), ep);
-            scatter_one<T>(decode1(a.g, M), mk((T)2 * (z0.x - z0.y), (T)0), ep);
-        } else if (2 * k == M) {
-            const C zk = a.spec[k];
-            scatter_one<T>(decode1(a.g, k), r2c_post(zk, zk, twN[k]), ep);
-        } else {
-            const C zk = a.spec[k], zm = a.spec[M - k];
-            scatter_one<T>(decode1(a.g, k), r2c_post(zk, zm, twN[k]), ep);
-            scatter_one<T>(decode1(a.g, M - k), r2c_post(zm, zk, twN[M - k]), ep);
+    for (int i0 = blockIdx.x << lh; i0 < npair; i0 += gridDim.x << lh) {
+        const int ib = i0 + (b & (TH - 1));
+        const bool self = ib == 0 || 2 * ib == P;
+        L1dLast<T> ld{a.spec, P, ib >= npair ? -1 : (b < TH ? ib : (self ? -1 : P - ib))};
+        first_stage<T, false>(t, ld);
+        mid_stages<T, false>(t, 1, t.nst);
+        for (int w = threadIdx.x; w < Q << lh; w += blockDim.x) {
+            const int c = w & (TH - 1), k2 = w >> lh, i = i0 + c;
+            if (i >= npair) continue;
+            const int k = i + P * k2;
+            const C zk = t.cur[t.lay.at(k2, c)];
+            if (k == 0) {
+                scatter1<T>(M, 0, r2c_post(zk, zk, twN[0]), ep);
+                scatter1<T>(M, M, mk((T)2 * (zk.x - zk.y), (T)0), ep);
+            } else if (i == 0 || 2 * i == P) {
+                const C zm = t.cur[t.lay.at(i == 0 ? Q - k2 : Q - 1 - k2, c)];
+                scatter1<T>(M, k, r2c_post(zk, zm, twN[k]), ep);
+            } else {
+                const C zm = t.cur[t.lay.at(Q - 1 - k2, TH + c)];
+                scatter1<T>(M, k, r2c_post(zk, zm, twN[k]), ep);
+                scatter1<T>(M, M - k, r2c_post(zm, zk, twN[M - k]), ep);
+            }
         }
+        __syncthreads();
     }
     ep.finish();
 }
 template <typename T, class Epi>
-__global__ void __launch_bounds__(256) l1d_post_kernel(PassArgs<T> a, const cplx_t<T>* __restrict__ twN, Epi epi) {
-    l1d_post_kernel_body<T, Epi>(a, twN, epi);
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
+l1d_last_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P, int Q, Epi epi) {
+    l1d_last_kernel_body<T, Epi>(a, twN, P, Q, epi);
 }
 
-}  // namespace csipm
-
-namespace csipm {
-
 // ---------------------------------------------------------------- launchers
+// pass: 0 first, 1 row, 2 last
 template <typename T>
-PassArgs<T> l1d_args(const FftOperator<T>& op, bool row, double scale, const int* skip) {
+PassArgs<T> l1d_args(const FftOperator<T>& op, int pass, double scale, const int* skip) {
     PassArgs<T> a{};
     a.g = op.g;
     a.spec = op.spec;
-    a.pl = row ? op.planP : op.planQ;
-    a.tw = row ? op.twP : op.twQ;
-    a.Ltab = row ? op.l1P : op.l1Q;
+    a.pl = pass == 1 ? op.planP : op.planQ;
+    a.tw = pass == 1 ? op.twP : op.twQ;
+    a.Ltab = pass == 1 ? op.l1P : op.l1Q;
+    FftOperator<T>::tile_args(pass == 0 ? op.f_cfg : (pass == 1 ? op.p_cfg : op.q_cfg), &a);
     a.maskw = op.maskw;
     a.wpr = op.wpr;
     a.scale = scale;
@@ -193,11 +277,10 @@ PassArgs<T> l1d_args(const FftOperator<T>& op, bool row, double scale, const int
 template <typename T, typename TS>
 cudaError_t l1d_first(const FftOperator<T>& op, const TS* src, const int* skip, cudaStream_t st) {
     auto k = l1d_first_kernel<T, TS>;
-    const size_t smem = 2 * (size_t)op.l1Q * op.l1TB * sizeof(cplx_t<T>);
-    cudaError_t e = smem_optin(k, smem);
+    const PassCfg& c = op.f_cfg;
+    const cudaError_t e = smem_optin(k, c.smem);
     if (e != cudaSuccess) return e;
-    k<<<(op.l1P + op.l1TB - 1) / op.l1TB, 256, smem, st>>>(l1d_args(op, false, 1.0, skip), src, op.tw1, op.l1P,
-                                                            op.l1Q, op.l1TB);
+    k<<<c.tiles, c.threads, c.smem, st>>>(l1d_args(op, 0, 1.0, skip), src, op.tw1, op.l1P);
     return cudaGetLastError();
 }
 
@@ -205,36 +288,47 @@ template <typename T, int IN, int OUT, bool MASK>
 cudaError_t l1d_row(const FftOperator<T>& op, double scale, const T* real_in, T* real_out, const int* skip,
                     cudaStream_t st) {
     auto k = l1d_row_kernel<T, IN, OUT, MASK>;
-    const size_t smem = 2 * (size_t)op.l1P * op.l1RB * sizeof(cplx_t<T>);
-    cudaError_t e = smem_optin(k, smem);
+    const PassCfg& c = op.p_cfg;
+    const cudaError_t e = smem_optin(k, c.smem);
     if (e != cudaSuccess) return e;
-    PassArgs<T> a = l1d_args(op, true, scale, skip);
+    PassArgs<T> a = l1d_args(op, 1, scale, skip);
     a.real_in = real_in;
     a.real_out = real_out;
-    k<<<(op.l1Q + op.l1RB - 1) / op.l1RB, 256, smem, st>>>(a, op.tw1, op.l1P, op.l1Q, op.l1RB);
+    k<<<c.tiles, c.threads, c.smem, st>>>(a, op.tw1, op.l1P, op.l1Q);
     return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t l1d_lines_forward(const FftOperator<T>& op, const int* skip, cudaStream_t st) {
-    PassArgs<T> a = l1d_args(op, false, 1.0, skip);
-    a.tw_in_smem = op.q_cfg.tw_in_smem;
-    a.n_lines = op.l1P;
-    a.n_outer = 1;
-    a.so = 0;
-    a.sx = op.l1P;
-    a.jk_mode = 2;
-    EpiStore<double> none{nullptr};
-    return launch_strided<T, false, IN_SPEC, OUT_SPEC>(op.q_cfg, a, (const double*)nullptr, none, st);
 }
 
 template <typename T, class Epi>
-cudaError_t l1d_post(const FftOperator<T>& op, const Epi& epi, const int* skip, cudaStream_t st) {
-    const int half = op.g.m1 / 2 + 1;
-    int blocks = (half + 255) / 256;
-    if (blocks > 1024) blocks = 1024;
-    l1d_post_kernel<T, Epi><<<blocks, 256, 0, st>>>(l1d_args(op, false, 1.0, skip), op.tw1, epi);
+cudaError_t l1d_last(const FftOperator<T>& op, const Epi& epi, const int* skip, cudaStream_t st) {
+    auto k = l1d_last_kernel<T, Epi>;
+    const PassCfg& c = op.q_cfg;
+    const cudaError_t e = smem_optin(k, c.smem);
+    if (e != cudaSuccess) return e;
+    k<<<c.tiles, c.threads, c.smem, st>>>(l1d_args(op, 2, 1.0, skip), op.tw1, op.l1P, op.l1Q, epi);
     return cudaGetLastError();
 }
+
+// compiled once (passes_r*.cu): the kernels of one precision, and the last
+// pass's epilogues
+#define CSIPM_1D_LIST64(X) X(double, EpiStore<double>, EpiCG<double>)
+#define CSIPM_1D_LIST32(X) X(float, EpiCG<float>, EpiStore<float>)
+#define CSIPM_PASS_1D_ROW(EXT, T, IN, OUT, MASK)                                                                      \
+    EXT template cudaError_t l1d_row<T, IN, OUT, MASK>(const FftOperator<T>&, double, const T*, T*, const int*,        \
+                                                       cudaStream_t);
+#define CSIPM_PASS_1D(EXT, T, EPI1, EPI2)                                                                              \
+    EXT template cudaError_t l1d_first<T, T>(const FftOperator<T>&, const T*, const int*, cudaStream_t);               \
+    CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_SPEC, true)                                                                 \
+    CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_SPEC, false)                                                                \
+    CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_REAL, true)                                                                 \
+    CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_REAL, false)                                                                \
+    CSIPM_PASS_1D_ROW(EXT, T, IN_REAL, OUT_SPEC, false)                                                                \
+    EXT template cudaError_t l1d_last<T, EPI1>(const FftOperator<T>&, const EPI1&, const int*, cudaStream_t);          \
+    EXT template cudaError_t l1d_last<T, EPI2>(const FftOperator<T>&, const EPI2&, const int*, cudaStream_t);
+#ifndef CSIPM_PASSES_HERE
+#define CSIPM_X(...) CSIPM_PASS_1D(extern, __VA_ARGS__)
+CSIPM_1D_LIST64(CSIPM_X)
+CSIPM_1D_LIST32(CSIPM_X)
+#undef CSIPM_X
+#endif
 
 }  // namespace csipm

@@ -21,7 +21,6 @@
 #include "../../include/csipm.h"
 #include "geometry.h"
 #include "long1d.cuh"
-#include "operator.cuh"
 
 using namespace csipm;
 
@@ -90,24 +89,8 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
     op.g = g;
     op.stream = (cudaStream_t)stream;
     std::string err;
-    const bool long1d = dim == 1 && g.m1 > L1D_MIN_M;   // the handle path's four-step rows
-    if (long1d) {
-        if (!l1d_split(g.m1, &op.l1P, &op.l1Q))
-            return static_fail(CSIPM_ERR_UNSUPPORTED, "1D length has no split M = P*Q with P <= 4096, Q <= 768");
-        if (!make_fft_plan(op.l1P, &op.planP, &err, op.max_radix()) ||
-            !make_fft_plan(op.l1Q, &op.planQ, &err, op.max_radix()))
-            return static_fail(CSIPM_ERR_UNSUPPORTED, err);
-        if (!op.choose_strided(op.planQ, op.l1Q, op.l1P, 1, &op.q_cfg, &err)) return static_fail(CSIPM_ERR_UNSUPPORTED, err);
-        l1d_tiles(op.l1P, op.l1Q, sizeof(C), &op.l1TB, &op.l1RB);
-        op.plan1 = op.planP;
-    } else {
-        if (!op.make_plans(&err)) return static_fail(CSIPM_ERR_UNSUPPORTED, err);
-        if (!op.choose_row(g.n2 * g.n3, &op.row_cfg, &err)) return static_fail(CSIPM_ERR_UNSUPPORTED, err);
-    }
-    if (dim >= 2 && !op.choose_strided(op.plan2, g.n2, g.m1 + 1, dim == 3 ? g.n3 : 1, &op.s2_cfg, &err))
-        return static_fail(CSIPM_ERR_UNSUPPORTED, err);
-    if (dim >= 3 && !op.choose_strided(op.plan3, g.n3, g.m1 + 1, g.n2, &op.s3_cfg, &err))
-        return static_fail(CSIPM_ERR_UNSUPPORTED, err);
+    const bool long1d = dim == 1;   // the handle path's four-step rows
+    if (!op.make_plans(&err)) return static_fail(CSIPM_ERR_UNSUPPORTED, err);
 
     const size_t spec_b = align256(sizeof(C) * (size_t)g.ld1 * g.n2 * g.n3);
     const size_t tw1_b = align256(sizeof(C) * (size_t)g.n1);
@@ -144,8 +127,7 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
     if (e == cudaSuccess && long1d) e = put_twiddles(op.l1Q, op.twQ, s);
     if (e != cudaSuccess) return static_fail(CSIPM_ERR_CUDA, std::string("twiddle kernel: ") + cudaGetErrorString(e));
 
-    // the fused passes of A^T A: five (3D), three (2D), one row pass (1D) or
-    // the four passes of a long 1D row
+    // the fused passes of A^T A: five (3D) or three (2D, 1D)
     const double sc = 1.0 / (2.0 * (double)g.N);
     const bool mask = keep_bits != nullptr;
     EpiStore<double> none{nullptr};
@@ -156,11 +138,7 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
         if (e == cudaSuccess)
             e = mask ? l1d_row<double, IN_SPEC, OUT_SPEC, true>(op, sc, nullptr, nullptr, nullptr, s)
                      : l1d_row<double, IN_SPEC, OUT_SPEC, false>(op, sc, nullptr, nullptr, nullptr, s);
-        if (e == cudaSuccess) e = l1d_lines_forward(op, nullptr, s);
-        if (e == cudaSuccess) e = l1d_post(op, out, nullptr, s);
-    } else if (dim == 1) {
-        e = mask ? launch_row<double, IN_GATHER, OUT_SCATTER, true>(op.row_cfg, ra, x, out, s)
-                 : launch_row<double, IN_GATHER, OUT_SCATTER, false>(op.row_cfg, ra, x, out, s);
+        if (e == cudaSuccess) e = l1d_last(op, out, nullptr, s);
     } else {
         // beta-side passes along dim 2, plain spectrum passes along dim 3
         PassArgs<double> a2 = op.strided_args(2);
@@ -169,8 +147,8 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
         if (e == cudaSuccess && dim == 3)
             e = launch_strided<double, true, IN_SPEC, OUT_SPEC>(op.s3_cfg, a3, (const double*)nullptr, none, s);
         if (e == cudaSuccess)
-            e = mask ? launch_row<double, IN_SPEC, OUT_SPEC, true>(op.row_cfg, ra, (const double*)nullptr, none, s)
-                     : launch_row<double, IN_SPEC, OUT_SPEC, false>(op.row_cfg, ra, (const double*)nullptr, none, s);
+            e = mask ? launch_row<double, IN_SPEC, OUT_SPEC, true>(op.row_cfg, ra, s)
+                     : launch_row<double, IN_SPEC, OUT_SPEC, false>(op.row_cfg, ra, s);
         if (e == cudaSuccess && dim == 3)
             e = launch_strided<double, false, IN_SPEC, OUT_SPEC>(op.s3_cfg, a3, (const double*)nullptr, none, s);
         if (e == cudaSuccess)

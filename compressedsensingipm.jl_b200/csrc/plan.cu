@@ -1,38 +1,111 @@
 #include "plan.h"
 
+#include "fft_device.cuh"
+
+#include <algorithm>
 #include <cmath>
 
 namespace csipm {
 
-bool make_fft_plan(int L, FftPlanDev* out, std::string* err, int max_radix) {
+namespace {
+
+// n register radices of product r, descending and none above cap: the first
+// as small as possible, then the second, ...
+bool split_regs(int r, int n, int cap, int* out) {
+    if (n == 0) return r == 1;
+    for (int f = 2; f <= cap && f <= r; ++f) {
+        if (!reg_radix(f) || r % f || !split_regs(r / f, n - 1, f, out + 1)) continue;
+        out[0] = f;
+        return true;
+    }
+    return false;
+}
+
+}  // namespace
+
+bool make_fft_plan(int L, FftPlanDev* out, std::string* err) {
+    FftPlanDev p{};
+    p.L = L;
+    if (L < 1) {
+        if (err) *err = "FFT length must be positive";
+        return false;
+    }
+    std::vector<int> primes;
+    int r = L;
+    for (int f = 2; r > 1; ++f) {
+        if ((long long)f * f > r) f = r;   // what is left is prime
+        for (; r % f == 0; r /= f)
+            if (f > 7) primes.push_back(f);
+    }
+    int regs = L;
+    for (int q : primes) regs /= q;
+    int rad[FFT_MAX_STAGES];
+    int n = 0;
+    if (regs > 1) {
+        for (n = 1; n <= FFT_MAX_STAGES && !split_regs(regs, n, 10, rad);) ++n;
+    }
+    if (n + (int)primes.size() > FFT_MAX_STAGES) {
+        if (err) *err = "FFT length has too many prime factors";
+        return false;
+    }
+    for (int s = 0; s < n; ++s) p.rad[p.nst++] = rad[s];
+    for (int q : primes) p.rad[p.nst++] = q;
+    if (p.nst == 0) p.rad[p.nst++] = 1;
+    *out = p;
+    return true;
+}
+
+void fill_stages(const FftPlanDev& pl, int Ltab, bool rev, FftStage* out) {
+    int cs[FFT_MAX_STAGES], at = 0;
+    for (int s = 0; s < pl.nst; ++s) {
+        cs[s] = at;
+        if (!reg_radix(pl.rad[s])) at += prime_table(pl.rad[s]);
+    }
+    int Ns = 1;
+    for (int s = 0; s < pl.nst; ++s) {
+        const int q = rev ? pl.nst - 1 - s : s;
+        FftStage& o = out[s];
+        o.R = pl.rad[q];
+        o.Ns = Ns;
+        o.m = pl.L / o.R;
+        o.step = Ltab / (Ns * o.R);
+        o.mag_ns = 0xffffffffu / (unsigned)Ns + 1u;
+        o.mag_m = 0xffffffffu / (unsigned)o.m + 1u;
+        o.cs = cs[q];
+        Ns *= o.R;
+    }
+}
+
+int prime_table_size(const FftPlanDev& pl) {
+    int n = 0;
+    for (int s = 0; s < pl.nst; ++s)
+        if (!reg_radix(pl.rad[s])) n += prime_table(pl.rad[s]);
+    return n;
+}
+
+bool make_row_plan(int L, FftPlanDev* out, std::string* err) {
+    FftPlanDev p;
+    if (!make_fft_plan(L, &p, err)) return false;
+    if (p.nst == 1 || !reg_radix(p.rad[0])) {
+        if (p.nst >= FFT_MAX_STAGES) {
+            if (err) *err = "FFT length has too many prime factors";
+            return false;
+        }
+        for (int s = p.nst; s > 0; --s) p.rad[s] = p.rad[s - 1];
+        p.rad[0] = 1;
+        ++p.nst;
+    }
+    *out = p;
+    return true;
+}
+
+bool make_fft_plan_ip(int L, FftPlanDev* out, std::string* err) {
     FftPlanDev p{};
     p.L = L;
     p.nst = 0;
     if (L < 1) {
         if (err) *err = "FFT length must be positive";
         return false;
-    }
-    if (max_radix > 8) {
-        static const int cand[] = {32, 25, 20, 16, 15, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-        int r = L;
-        while (r > 1) {
-            int pick = 0;
-            for (int c : cand)
-                if (c <= max_radix && r % c == 0) { pick = c; break; }
-            if (!pick) {   // a prime > 7 (or a composite of them): smallest factor as a direct DFT
-                pick = r;
-                for (int f = 11; (long long)f * f <= r; f += 2)
-                    if (r % f == 0) { pick = f; break; }
-            }
-            if (p.nst >= FFT_MAX_STAGES) {
-                if (err) *err = "FFT length has too many prime factors";
-                return false;
-            }
-            p.rad[p.nst++] = pick;
-            r /= pick;
-        }
-        *out = p;
-        return true;
     }
     int r = L;
     int twos = 0;

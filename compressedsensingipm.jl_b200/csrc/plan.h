@@ -4,20 +4,33 @@
 #include <string>
 #include <vector>
 
-#include "fft_device.cuh"
+#include "plan_dev.h"
 
 namespace csipm {
 
-// Factor L into stages.  max_radix <= 8: radix 8 first, then 4/2 for the rest
-// of the power of two, then 5, 3, 7 (the register-staged in-place engine).
-// Larger max_radix: greedy largest-first over the composite register radices
-// {32, 25, 20, 16, 15, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2} up to max_radix, which
-// cuts the number of shared-memory round trips (320 = 20*16, 160 = 20*8).
-// Any remaining prime becomes a direct-DFT stage.
-bool make_fft_plan(int L, FftPlanDev* out, std::string* err, int max_radix = 8);
+// Factor L into stages: the fewest register radices (up to 10; plan_dev.h)
+// that give its factors 2, 3, 5 and 7, balanced and in descending order, then
+// every larger prime as a stage of its own.  Fewer stages mean fewer trips
+// through shared memory: 90 = 10*9 takes one, 256 = 8*8*4 and 720 = 10*9*8 two.
+bool make_fft_plan(int L, FftPlanDev* out, std::string* err);
 
-// True when every stage of `pl` respects the per-thread register budget for
-// `lines` interleaved lines processed by `nthreads` threads.
+// The same for a row pass, which runs the plan reversed and then in order and
+// joins the two at the first radix: at least two stages, a register radix first.
+bool make_row_plan(int L, FftPlanDev* out, std::string* err);
+
+// The plan's stages in plan order (rev: reversed, as the inverse half of a row
+// pass runs it) with twiddles from a table of Ltab-th roots.
+void fill_stages(const FftPlanDev& pl, int Ltab, bool rev, FftStage* out);
+
+// Complex values of the plan's prime tables (prime_tables, fft_device.cuh).
+int prime_table_size(const FftPlanDev& pl);
+
+// Radices up to 8 for the in-place engine: radix 8 first, then 4/2 for the
+// rest of the power of two, then 5, 3, 7; any other prime a direct DFT.
+bool make_fft_plan_ip(int L, FftPlanDev* out, std::string* err);
+
+// True when every stage of an in-place plan respects the per-thread register
+// budget for `lines` interleaved lines processed by `nthreads` threads.
 bool plan_fits(const FftPlanDev& pl, int lines, int nthreads);
 
 }  // namespace csipm

@@ -1,0 +1,45 @@
+// What a run-time-plan FFT pass is told about its transform and its tile.
+#pragma once
+
+#ifndef CSIPM_HD
+#ifdef __CUDACC__
+#define CSIPM_HD __host__ __device__ __forceinline__
+#else
+#define CSIPM_HD inline
+#endif
+#endif
+
+namespace csipm {
+
+constexpr int FFT_MAX_STAGES = 12;
+
+struct FftPlanDev {
+    int L;                       // transform length
+    int nst;                     // number of stages
+    int rad[FFT_MAX_STAGES];     // radices, in order
+};
+
+// The radices with a register butterfly in the stage dispatch.  Up to 10: a
+// radix-16 FP64 butterfly with its twiddles and addresses does not fit 128
+// registers (it spilled kilobytes), and the longer straight-line code cost
+// more in instruction fetches than the third stage of a 256-point line.
+CSIPM_HD constexpr bool reg_radix(int r) { return r <= 10; }
+
+// One stage of a plan as the kernels read it (fill_stages, plan.cu).
+struct FftStage {
+    int R, Ns, m;           // radix, product of the earlier radices, L/R
+    int step;               // Ltab/(Ns*R): table stride of the stage's twiddles
+    unsigned mag_ns, mag_m; // reciprocals of Ns and m (quot)
+    int cs;                 // prime stages: where its cosines and sines start (prime_tables)
+};
+
+// Shared-memory place of element (x, b) of a tile.  b is fastest, so a stage
+// access of 8 FP64 (16 FP32) lines covers whole 128-byte rows; narrower
+// tiles leave one slot free after every 8 positions (sh = 3, else 31), or
+// the stride R of a stage's writes would fall on the same banks.
+struct TileLay {
+    int lg, tbp, sh;   // log2(lines), pitch, padding shift
+    CSIPM_HD int at(int x, int b) const { return (x + (x >> sh)) * tbp + b; }
+};
+
+}  // namespace csipm

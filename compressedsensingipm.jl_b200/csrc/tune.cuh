@@ -5,11 +5,9 @@
 // handle's stream, one warm launch, best of TUNE_REPS) and keeps the fastest:
 //
 //   dim-3 lines:  two-level register kernel (when the length has a pair)
-//                 or the Stockham kernel with 2/4/8(/16 in FP32) lines per CTA
-//   dim-2 lines:  Stockham lines per CTA when the length has no pair (with a
-//                 pair the two-level kernel stays: the solver-order gather and
-//                 scatter need it)
-//   dim-1 rows:   two-level row kernel (pair) or Stockham with 1..16 rows per CTA
+//                 or the run-time-plan kernel with 2/4/8(/16 in FP32) lines per CTA
+//   dim-2 lines:  the same
+//   dim-1 rows:   two-level row kernel (pair) or run-time plan with 1..16 rows per CTA
 //
 // Results are cached per process, so every later handle of the same size
 // starts with the tuned configuration at no cost.  When the environment
@@ -17,7 +15,7 @@
 // processes: the file's choices are read at the first tuning, and every new
 // choice is appended to it as one JSON object per line,
 //   {"elem": 4, "dim": 3, "n": [320, 320, 320], "masked": 1,
-//    "s3_two": 1, "s3_tb": 0, "s2_tb": 0, "row_two": 1, "row_rb": 0}
+//    "s3_two": 1, "s3_tb": 0, "s2_tb": 0, "row_two": 1, "row_rb": 0, "s2_two": 1}
 #pragma once
 #include <cstdio>
 #include <cstdlib>
@@ -31,8 +29,8 @@
 namespace csipm_internal {
 
 struct TuneChoice {
-    int s3_two = 1, s3_tb = 0;     // 1: two-level; else Stockham tb (0: the heuristic's)
-    int s2_tb = 0;
+    int s3_two = 1, s3_tb = 0;     // 1: two-level; else run-time-plan tb (0: the heuristic's)
+    int s2_two = 1, s2_tb = 0;     // likewise
     int row_two = 1, row_rb = 0;
 };
 
@@ -74,11 +72,12 @@ inline void tune_cache_load() {
     while (std::fgets(line, sizeof(line), f)) {
         int elem, dim, n1, n2, n3, masked;
         TuneChoice c;
+        // lines without s2_two (written before it was tuned) keep the two-level kernel
         if (std::sscanf(line,
                         " {\"elem\": %d, \"dim\": %d, \"n\": [%d, %d, %d], \"masked\": %d, \"s3_two\": %d, "
-                        "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d}",
+                        "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d",
                         &elem, &dim, &n1, &n2, &n3, &masked, &c.s3_two, &c.s3_tb, &c.s2_tb, &c.row_two,
-                        &c.row_rb) == 11)
+                        &c.row_rb, &c.s2_two) >= 11)
             tune_cache()[TuneKey{elem, dim, n1, n2, n3, masked}] = c;
     }
     std::fclose(f);
@@ -92,50 +91,25 @@ inline void tune_cache_append(const TuneKey& k, const TuneChoice& c) {
     if (!f) return;
     std::fprintf(f,
                  "{\"elem\": %d, \"dim\": %d, \"n\": [%d, %d, %d], \"masked\": %d, \"s3_two\": %d, "
-                 "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d}\n",
+                 "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d}\n",
                  std::get<0>(k), std::get<1>(k), std::get<2>(k), std::get<3>(k), std::get<4>(k), std::get<5>(k),
-                 c.s3_two, c.s3_tb, c.s2_tb, c.row_two, c.row_rb);
+                 c.s3_two, c.s3_tb, c.s2_tb, c.row_two, c.row_rb, c.s2_two);
     std::fclose(f);
 }
 
-// Stockham strided configuration with a forced number of lines per CTA
+// a tuned tile takes 96 KB of shared memory at most (two CTAs per SM)
+constexpr size_t TUNE_SMEM = 96 * 1024;
+
+// run-time-plan strided configuration with a forced number of lines per CTA
 template <typename T>
-bool strided_cfg_tb(const FftOperator<T>& op, const FftPlanDev& pl, int Ltab, int n_lines, int n_outer, int tb,
-                    PassCfg* cfg) {
-    using C = cplx_t<T>;
-    const size_t data = 3 * (size_t)pl.L * sizeof(C) * tb;
-    if (data > FftOperator<T>::smem_limit() || data > 96 * 1024) return false;
-    cfg->tb = tb;
-    cfg->tbp = tb;
-    cfg->threads = 256;
-    cfg->pp = 1;
-    const size_t tws = (size_t)Ltab * sizeof(C);
-    cfg->tw_in_smem = (data + tws <= FftOperator<T>::smem_limit() && tws <= 32 * 1024) ? 1 : 0;
-    cfg->smem = data + (cfg->tw_in_smem ? tws : 0);
-    cfg->tiles = ((n_lines + tb - 1) / tb) * n_outer;
-    cfg->grid = dim3(cfg->tiles, 1, 1);
-    return true;
+bool strided_cfg_tb(const FftPlanDev& pl, int n_lines, int n_outer, int tb, PassCfg* cfg) {
+    return FftOperator<T>::strided_cfg(pl, n_lines, n_outer, tb, TUNE_SMEM, cfg);
 }
 
-// Stockham persistent row configuration with a forced number of rows per CTA
+// run-time-plan row configuration with a forced number of rows per CTA
 template <typename T>
 bool row_cfg_rb(const FftOperator<T>& op, int nrows, int rb, PassCfg* cfg) {
-    using C = cplx_t<T>;
-    const int M = op.g.m1;
-    if (rb > nrows) return false;
-    const int tbp = rb > 1 ? rb + 1 : 1;
-    const size_t one = (size_t)(M + 1) * tbp * sizeof(C);
-    if (3 * one > FftOperator<T>::smem_limit() || 3 * one > 96 * 1024) return false;
-    const size_t tws = (size_t)op.g.n1 * sizeof(C);
-    cfg->pp = 1;
-    cfg->tb = rb;
-    cfg->tbp = tbp;
-    cfg->threads = 256;
-    cfg->tw_in_smem = (3 * one + tws <= FftOperator<T>::smem_limit() && tws <= 32 * 1024) ? 1 : 0;
-    cfg->smem = 3 * one + (cfg->tw_in_smem ? tws : 0);
-    cfg->tiles = (nrows + rb - 1) / rb;
-    cfg->grid = dim3(cfg->tiles, 1, 1);
-    return true;
+    return FftOperator<T>::rows_cfg(op.plan1, nrows, rb, TUNE_SMEM, cfg);
 }
 
 template <typename T, class F>
@@ -165,9 +139,10 @@ void apply_choice(FftOperator<T>& op, const TuneChoice& c) {
     const Geom& g = op.g;
     if (g.dim == 3) {
         if (!c.s3_two) op.s3_A = op.s3_B = 0;
-        if (c.s3_tb) strided_cfg_tb(op, op.plan3, g.n3, g.m1 + 1, g.n2, c.s3_tb, &op.s3_cfg);
+        if (c.s3_tb) strided_cfg_tb<T>(op.plan3, g.m1 + 1, g.n2, c.s3_tb, &op.s3_cfg);
     }
-    if (g.dim >= 2 && c.s2_tb) strided_cfg_tb(op, op.plan2, g.n2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, c.s2_tb, &op.s2_cfg);
+    if (!c.s2_two) op.s2_A = op.s2_B = 0;
+    if (g.dim >= 2 && c.s2_tb) strided_cfg_tb<T>(op.plan2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, c.s2_tb, &op.s2_cfg);
     if (g.dim >= 2) {
         if (!c.row_two) op.r_A = op.r_B = 0;
         if (c.row_rb) row_cfg_rb(op, g.n2 * g.n3, c.row_rb, &op.row_cfg);
@@ -212,7 +187,7 @@ void autotune(FftOperator<T>& op, cudaStream_t st) {
         for (int tb : tbs) {
             if (tb > max_tb) continue;
             PassCfg c;
-            if (!strided_cfg_tb(op, op.plan3, g.n3, g.m1 + 1, g.n2, tb, &c)) continue;
+            if (!strided_cfg_tb<T>(op.plan3, g.m1 + 1, g.n2, tb, &c)) continue;
             op.s3_cfg = c;
             const float t = tune_time<T>(st, e0, e1, [&] {
                 return run_strided<T, true, IN_SPEC, OUT_SPEC>(op, 3, op.strided_args(3), (const double*)nullptr, none, st);
@@ -222,35 +197,54 @@ void autotune(FftOperator<T>& op, cudaStream_t st) {
         op.s3_A = A;
         op.s3_B = B;
         op.s3_cfg = keep;
+        if (A && best.s3_tb) {   // the incumbent once more: its first timing may have met an idle GPU's clocks
+            const float t = tune_time<T>(st, e0, e1, [&] {
+                return run_strided<T, true, IN_SPEC, OUT_SPEC>(op, 3, op.strided_args(3), (const double*)nullptr, none, st);
+            });
+            if (t_best >= TUNE_MARGIN * t) { best.s3_two = 1; best.s3_tb = 0; }
+        }
     }
-    // dim-2 lines without a two-level pair
-    if (!op.s2_A) {
+    // dim-2 lines, by the two passes a solve runs along them: the solver-order
+    // gather (the spectrum buffer stands in for the vector) and a forward pass
+    {
+        auto both = [&] {
+            const cudaError_t e = run_strided<T, true, IN_SGATHER, OUT_SPEC>(
+                op, 2, op.strided_args(2), reinterpret_cast<const T*>(op.spec), none, st);
+            return e != cudaSuccess ? e
+                                    : run_strided<T, false, IN_SPEC, OUT_SPEC>(op, 2, op.strided_args(2),
+                                                                               (const double*)nullptr, none, st);
+        };
+        const int A = op.s2_A, B = op.s2_B;
         const PassCfg keep = op.s2_cfg;
-        float t_best = tune_time<T>(st, e0, e1, [&] {
-            return run_strided<T, true, IN_SPEC, OUT_SPEC>(op, 2, op.strided_args(2), (const double*)nullptr, none, st);
-        });
+        float t_best = tune_time<T>(st, e0, e1, both);
+        best.s2_two = A ? 1 : 0;
+        op.s2_A = op.s2_B = 0;
         for (int tb : tbs) {
             if (tb > max_tb) continue;
             PassCfg c;
-            if (!strided_cfg_tb(op, op.plan2, g.n2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, tb, &c)) continue;
+            if (!strided_cfg_tb<T>(op.plan2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, tb, &c)) continue;
             op.s2_cfg = c;
-            const float t = tune_time<T>(st, e0, e1, [&] {
-                return run_strided<T, true, IN_SPEC, OUT_SPEC>(op, 2, op.strided_args(2), (const double*)nullptr, none, st);
-            });
-            if (t < TUNE_MARGIN * t_best) { t_best = t; best.s2_tb = tb; }
+            const float t = tune_time<T>(st, e0, e1, both);
+            if (t < TUNE_MARGIN * t_best) { t_best = t; best.s2_two = 0; best.s2_tb = tb; }
         }
+        op.s2_A = A;
+        op.s2_B = B;
         op.s2_cfg = keep;
+        if (A && best.s2_tb && t_best >= TUNE_MARGIN * tune_time<T>(st, e0, e1, both)) {   // as above
+            best.s2_two = 1;
+            best.s2_tb = 0;
+        }
     }
-    // dim-1 rows (persistent Stockham candidates only when the heuristic's row
-    // configuration is the persistent one)
+    // dim-1 rows (run-time-plan candidates only when the heuristic's row
+    // configuration is not the in-place one)
     {
         const int A = op.r_A, B = op.r_B;
         const PassCfg keep = op.row_cfg;
         const bool mask = op.maskw != nullptr;
         PassArgs<T> ra = op.row_args(1.0, nullptr, nullptr);
         auto row = [&] {
-            return mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, (const double*)nullptr, none, st)
-                        : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, (const double*)nullptr, none, st);
+            return mask ? run_row<T, IN_SPEC, OUT_SPEC, true>(op, ra, st)
+                        : run_row<T, IN_SPEC, OUT_SPEC, false>(op, ra, st);
         };
         float t_best = tune_time<T>(st, e0, e1, row);
         best.row_two = A ? 1 : 0;
@@ -268,6 +262,10 @@ void autotune(FftOperator<T>& op, cudaStream_t st) {
         op.r_A = A;
         op.r_B = B;
         op.row_cfg = keep;
+        if (A && best.row_rb) {   // as above
+            ra = op.row_args(1.0, nullptr, nullptr);
+            if (t_best >= TUNE_MARGIN * tune_time<T>(st, e0, e1, row)) { best.row_two = 1; best.row_rb = 0; }
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

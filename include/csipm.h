@@ -97,7 +97,7 @@ typedef struct {
                                   csipm_admm as one graph launch; graphs are captured once per
                                   handle; 0: plain launches (same kernels, same results) */
     int autotune;              /* 1 (default): csipm_create times the candidate launch configurations
-                                  of the FFT passes for this size (two-level vs Stockham kernels,
+                                  of the FFT passes for this size (two-level vs run-time-plan kernels,
                                   lines / rows per CTA) once per process and keeps the fastest;
                                   with the environment variable CSIPM_TUNE_CACHE naming a file, the
                                   choices persist there (one JSON object per line) and later
@@ -254,7 +254,7 @@ CSIPM_API int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm
 
 /* Batched solves: advances `count` handles' interior-point solves together,
  * every step one kernel launch for all of them — the FFT passes are
- * persistent Stockham kernels over an instance table (per instance its
+ * run-time-plan kernels over an instance table (per instance its
  * sizes, run-time plans, vector offsets, reduction workspace and control
  * block) and every element kernel runs all instances at once (gridDim.y =
  * instance).  Any sizes mix; the handles must share the dimension count,
