@@ -164,7 +164,7 @@ struct csipm_handle_s {
 
     cudaMemPool_t pool = nullptr;   // device_pool(device): every device buffer of the handle
     static constexpr size_t HSLOT_BYTES = sizeof(double) * 64;   // SL_COUNT slots
-    static constexpr size_t HCGS_BYTES = 64;                     // >= sizeof(CgScalars)
+    static constexpr size_t HCGS_BYTES = 128;                    // >= sizeof(CgScalars)
     static constexpr size_t HCTL_BYTES = 256;                    // >= sizeof(IpmCtl)
     void* hmiss = nullptr;          // pinned bounce buffer of the missing indices (csipm_create)
     size_t hmiss_bytes = 0;

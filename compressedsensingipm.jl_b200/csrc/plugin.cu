@@ -110,22 +110,63 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
     if (!h->L1) return fail(h, CSIPM_ERR_INVALID, "csipm_kkt_build must be called first");
     const long long n = h->N;
     cudaStream_t st = h->stream;
-    const bool pc = h->opt.preconditioner != 0;
-    const double *P11 = pc ? h->P11 : nullptr, *P12 = pc ? h->P12 : nullptr, *P22 = pc ? h->P22 : nullptr;
+    const int maxit = h->opt.cg_maxit;
+    auto finish = [&]() -> int {
+        cudaEventRecord(h->ev1, st);
+        CK(cudaEventSynchronize(h->ev1));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, h->ev0, h->ev1);
+        h->krylov_ms += ms;
+        if (cg_iters) *cg_iters = h->hcgs->iters;
+        if (h->hcgs->breakdown) return fail(h, CSIPM_ERR_NONFINITE, "CG breakdown in solve_kkt");
+        return CSIPM_OK;
+    };
     cudaEventRecord(h->ev0, st);
+    if (h->opt.preconditioner) {
+        // on N unknowns (kkt_schur_init_kernel says why the iterates are the 2N
+        // method's); the second halves of the 2N buffers hold the diagonals
+        double *x = h->k_x, *r = h->k_r, *p = h->k_p, *q = h->k_q, *D = h->k_x + n, *M = h->k_r + n;
+        const int so = h->sorder ? 1 : 0;
+        ew_launch(kkt_schur_init_kernel, so ? n / 2 : n, st, h->g, so, w, pr_diag, x, r, p, D, M,
+                  h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
+        CK(cudaGetLastError());
+        int chunk = 2, since = 0;
+        for (int it = 0; it < maxit; ++it) {
+            EpiCG<double> ep{p, D, q, h->ws(&h->cgs->pq), 0.0};
+            CK(solve_AtA(h, p, ep, &h->cgs->done, st));
+            ew_launch(cg_update_kernel<double, double>, n, st, n, it, x, r, p, q, (const double*)M,
+                      h->ws(h->slots + SL_DUMMY), h->cgs);
+            ew_launch(cg_pupdate_kernel<double>, n, st, n, it, r, (const double*)M, p, h->cgs);
+            CK(cudaGetLastError());
+            if (++since >= chunk || it + 1 == maxit) {
+                since = 0;
+                if (chunk < 8) chunk *= 2;
+                CK(cudaMemcpyAsync(h->hcgs, h->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
+                CK(cudaStreamSynchronize(st));
+                if (h->hcgs->done) break;
+            }
+        }
+        CK(cudaMemcpyAsync(h->hcgs, h->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
+        ew_launch(kkt_schur_back_kernel, so ? n / 2 : n, st, h->g, so, w, (const double*)x, pr_diag,
+                  (const CgScalars*)h->cgs);
+        CK(cudaGetLastError());
+        const int f = finish();
+        h->matvecs += h->hcgs->iters;
+        return f;
+    }
+    const double* none = nullptr;   // no preconditioner: 2N vectors, reference packing
     ew_launch(kkt_rhs_kernel, n, st, n, w, pr_diag, h->k_b);
     CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
-    ew_launch(kcg_init_kernel, n, st, n, h->k_b, h->k_x, h->k_r, h->k_p, P11, P12, P22,
+    ew_launch(kcg_init_kernel, n, st, n, h->k_b, h->k_x, h->k_r, h->k_p, none, none, none,
                                               h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
     CK(cudaGetLastError());
     int chunk = 2, since = 0;
-    const int maxit = h->opt.cg_maxit;
     for (int it = 0; it < maxit; ++it) {
         EpiKcg ep{h->k_p, h->k_q, h->L1, h->L2, n, h->ws(&h->cgs->pq), 0.0};
         CK(op_AtA(h->op64, h->k_p, ep, &h->cgs->done, st));
-        ew_launch(kcg_update_kernel, n, st, n, it, h->k_x, h->k_r, h->k_p, h->k_q, P11, P12, P22,
+        ew_launch(kcg_update_kernel, n, st, n, it, h->k_x, h->k_r, h->k_p, h->k_q, none, none, none,
                                                      h->ws(h->slots + SL_DUMMY), h->cgs);
-        ew_launch(kcg_pupdate_kernel, n, st, n, it, h->k_r, h->k_p, P11, P12, P22, h->cgs);
+        ew_launch(kcg_pupdate_kernel, n, st, n, it, h->k_r, h->k_p, none, none, none, h->cgs);
         CK(cudaGetLastError());
         if (++since >= chunk || it + 1 == maxit) {
             since = 0;
@@ -140,14 +181,7 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
     h->matvecs += h->hcgs->iters;
     ew_launch(kkt_back_kernel, n, st, n, w, h->k_x, pr_diag);
     CK(cudaGetLastError());
-    cudaEventRecord(h->ev1, st);
-    CK(cudaEventSynchronize(h->ev1));
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-    h->krylov_ms += ms;
-    if (cg_iters) *cg_iters = h->hcgs->iters;
-    if (h->hcgs->breakdown) return fail(h, CSIPM_ERR_NONFINITE, "CG breakdown in solve_kkt");
-    return CSIPM_OK;
+    return finish();
 }
 
 }  // extern "C"

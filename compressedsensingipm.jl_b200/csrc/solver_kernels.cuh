@@ -44,6 +44,11 @@ struct CgScalars {
     int iters;          // iterations completed
     int breakdown;      // 1: p'q <= 0 or non-finite
     int pad;
+    // Newton solves of the KKT plugin (kkt_schur_init_kernel): the eliminated
+    // half's share of the scalars, zero elsewhere
+    double S, rho, sig;
+    // p.q and the next r.z with that share
+    __device__ __forceinline__ double full_pq() const { return pq + sig * sig * S; }
 };
 
 // CG scalars of a start whose r.(Minv r) = rz was reduced by the kernel that
@@ -57,6 +62,7 @@ __device__ __forceinline__ void cg_start(CgScalars* sc, double rz, double atol, 
     sc->thresh = atol + rtol * sqrt(rz);
     sc->iters = 0;
     sc->breakdown = 0;
+    sc->S = sc->rho = sc->sig = 0.0;
     sc->done = (sqrt(rz) <= sc->thresh) ? 1 : 0;
     if (!isfinite(rz)) { sc->done = 1; sc->breakdown = 1; }
 }
@@ -83,6 +89,7 @@ __device__ __forceinline__ void cg_init_kernel_body(long long n, const double* _
         sc->thresh = atol + rtol_s.get() * sqrt(rz);
         sc->iters = 0;
         sc->breakdown = 0;
+        sc->S = sc->rho = sc->sig = 0.0;
         sc->done = (sqrt(rz) <= sc->thresh) ? 1 : 0;
         if (!isfinite(rz)) { sc->done = 1; sc->breakdown = 1; }
     }
@@ -99,7 +106,7 @@ template <typename TV, typename TX>
 __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* __restrict__ x, TV* __restrict__ r, const TV* __restrict__ p,
                                  const TV* __restrict__ q, const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
     if (sc->done) return;
-    const double pq = sc->pq;
+    const double pq = sc->full_pq();
     const double rz = sc->rz[it & 1];
     // breakdown: every block sees the same p.q and returns before touching
     // x or r, so the iterate stays the last good one
@@ -128,7 +135,11 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
     }
     if (i < n) elem(i, (double)x[i], (double)r[i], (double)p[i], (double)q[i], Minv ? (double)Minv[i] : 1.0);
     if (grid_reduce<1>(acc, ws, 0u, 0u) && threadIdx.x == 0) {
-        const double rzn = ws.out[0];
+        // the last block: every other one has read sig and pq
+        const double rho = sc->rho - alpha * sc->sig;
+        const double rzn = ws.out[0] + rho * rho * sc->S;
+        sc->rho = rho;
+        sc->sig = rho + rzn / rz * sc->sig;
         sc->rz[(it + 1) & 1] = rzn;
         sc->iters += 1;     // counted on the device: graph replays reuse the same `it` values
         if (!isfinite(rzn)) { sc->breakdown = 1; sc->done = 1; }
@@ -902,7 +913,105 @@ static __global__ void kkt_back_kernel(long long n, double* __restrict__ w, cons
     }
 }
 
-// ---- 2N PCG of the KKT plugin (Krylov.jl cg semantics, M = block preconditioner)
+// ---- the same PCG on N unknowns
+// With the block preconditioner P = [I + L1, L2; L2, L1]^-1 the 2N PCG on
+// K = [Q + L1, L2; L2, L1] (Q = A'A) from zero never leaves N unknowns: since
+// K P r = r + [(Q - I) z_b; 0], the second halves of the residuals stay
+// rho b_z and those of the products sig b_z, with
+//     rho <- rho - alpha sig,   sig <- rho + beta sig,   rho_0 = sig_0 = 1.
+// Then x_z = ((1 - rho) b_z - L2 x_b)/L1 and p_z = (sig b_z - L2 p_b)/L1 follow
+// from the first halves, which are the iterates of a PCG on (Q + D),
+// D = L1 - L2^2/L1 = 4 S1 S2/(S1 + S2), with preconditioner 1/(1 + D) and
+// residual r~ = r_b - rho L2/L1 b_z, whose scalars are
+//     p.q = p_b.q~ + sig^2 S,   r.z = r~.z_b + rho^2 S,   S = sum b_z^2/L1.
+// The iterates, step lengths and stop test are those of the 2N method; an
+// iteration moves 14 instead of 31 vectors of N besides the spectrum, and runs
+// in solver order.
+
+// One thread per solver-order pair and tail entry (or per index when the
+// solve keeps the reference packing): body(ref index, solver index, sign).
+template <class F>
+__device__ __forceinline__ void for_solver_entries(const Geom& g, int sorder, F&& body) {
+    if (!sorder) {
+        CSIPM_GRID_LOOP(i, g.N) body(i, i, 1.0);
+        return;
+    }
+    const long long tail = g.N - 2 * g.NI;
+    const int pl = g.m1 - 1;
+    CSIPM_GRID_LOOP(idx, g.NI + tail) {
+        if (idx < g.NI) {
+            const int i = (int)(idx % pl) + 1;
+            const long long r = idx / pl;
+            const MapEntry e = decode_interior(g, i, (int)(r % g.n2), (int)(r / g.n2));
+            body((long long)e.re, 2 * idx, 1.0);
+            body((long long)e.im, 2 * idx + 1, e.kind == KIND_MINUS ? -1.0 : 1.0);
+        } else {
+            const long long t = idx - g.NI;
+            body((long long)sol_tail_ref(g, t), 2 * g.NI + t, 1.0);
+        }
+    }
+}
+
+// the reduced right-hand side's halves (src/fft_kkt.jl:334-335)
+__device__ __forceinline__ void kkt_rhs(const double* __restrict__ w, long long n, long long i, double S1, double S2,
+                                        double& bb, double& bz) {
+    const double w3 = w[2 * n + i], w4 = w[3 * n + i], a = S1 * w[4 * n + i], c = S2 * w[5 * n + i];
+    bb = w[i] - w3 + w4 - a + c;
+    bz = w[n + i] - w3 - w4 - a - c;
+}
+
+// start: x = 0, r = r~, p = M r, the diagonals D and M, and the scalars
+static __global__ void __launch_bounds__(EW_THREADS)
+kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const double* __restrict__ pr_diag,
+                      double* __restrict__ x, double* __restrict__ r, double* __restrict__ p, double* __restrict__ D,
+                      double* __restrict__ M, RedWorkspace ws, CgScalars* sc, double atol, double rtol) {
+    const long long n = g.N;
+    double acc[2] = {0.0, 0.0};
+    for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
+        const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i], l1 = S1 + S2;
+        double bb, bz;
+        kkt_rhs(w, n, i, S1, S2, bb, bz);
+        const double u = bz / l1, d = 4.0 * (S1 / l1) * S2, m = 1.0 / (1.0 + d);
+        const double rv = sg * (bb - (S1 - S2) * u), z = m * rv;
+        x[s] = 0.0;
+        r[s] = rv;
+        p[s] = z;
+        D[s] = d;
+        M[s] = m;
+        acc[0] += rv * z;
+        acc[1] += bz * u;
+    });
+    if (grid_reduce<2>(acc, ws, 0u, 0u) && threadIdx.x == 0) {
+        const double S = ws.out[1];
+        cg_start(sc, ws.out[0] + S, atol, DevScalar(rtol));
+        sc->S = S;
+        sc->rho = sc->sig = 1.0;
+    }
+}
+
+// x_z and the back-substitution (src/fft_kkt.jl:345-350), in place on w
+static __global__ void __launch_bounds__(EW_THREADS)
+kkt_schur_back_kernel(Geom g, int sorder, double* __restrict__ w, const double* __restrict__ x,
+                      const double* __restrict__ pr_diag, const CgScalars* __restrict__ sc) {
+    const long long n = g.N;
+    const double left = 1.0 - sc->rho;
+    for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
+        const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i];
+        double bb, bz;
+        kkt_rhs(w, n, i, S1, S2, bb, bz);
+        const double w1 = sg * x[s], w2 = (left * bz - (S1 - S2) * w1) / (S1 + S2);
+        const double w5 = -(w[2 * n + i] + S1 * (w1 + w2 + w[4 * n + i]));
+        const double w6 = -(w[3 * n + i] + S2 * (-w1 + w2 + w[5 * n + i]));
+        w[i] = w1;
+        w[n + i] = w2;
+        w[2 * n + i] = (w[2 * n + i] + w5) / S1;
+        w[3 * n + i] = (w[3 * n + i] + w6) / S2;
+        w[4 * n + i] = w5;
+        w[5 * n + i] = w6;
+    });
+}
+
+// ---- 2N PCG of the KKT plugins (Krylov.jl cg semantics, M = block preconditioner)
 // z = P r (2x2 blocks), written into z; returns r.z
 __device__ __forceinline__ void pblock(const double* P11, const double* P12, const double* P22, long long i,
                                        double rb, double rz, double& zb, double& zz) {
