@@ -37,8 +37,9 @@ __device__ __forceinline__ int quot(int x, int d, unsigned mag) { return d == 1 
 template <int R, bool INV, typename T>
 __device__ __forceinline__ void twiddle_dft(cplx_t<T>* v, int k, const FftStage& s, const cplx_t<T>* __restrict__ tw) {
     if (R > 1 && s.Ns > 1) {
+        const int e = k * s.step;
 #pragma unroll
-        for (int r = 1; r < R; ++r) v[r] = twmul<INV>(v[r], tw[k * r * s.step]);
+        for (int r = 1; r < R; ++r) v[r] = twmul<INV>(v[r], tw[r * e]);
     }
     Dft<R, INV, T>::run(v);
 }
@@ -49,14 +50,18 @@ __device__ __forceinline__ void twiddle_dft(cplx_t<T>* v, int k, const FftStage&
 template <typename T, int R, bool INV>
 __device__ __forceinline__ void bfly_load(cplx_t<T>* v, const cplx_t<T>* in, const TileLay& lay, const FftStage& s,
                                           const cplx_t<T>* __restrict__ tw, int u, int k, int b) {
+    const cplx_t<T>* p = in + lay.at(u, b);
+    const int d = s.m * lay.tbp;
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = in[lay.at(u + r * s.m, b)];
+    for (int r = 0; r < R; ++r) v[r] = p[r * d];
     twiddle_dft<R, INV, T>(v, k, s, tw);
 }
 template <typename T, int R>
 __device__ __forceinline__ void bfly_put(const cplx_t<T>* v, cplx_t<T>* out, const TileLay& lay, int o, int Ns, int b) {
+    cplx_t<T>* p = out + lay.at(o, b);
+    const int d = Ns * lay.tbp;
 #pragma unroll
-    for (int r = 0; r < R; ++r) out[lay.at(o + r * Ns, b)] = v[r];
+    for (int r = 0; r < R; ++r) p[r * d] = v[r];
 }
 
 // ---- prime stages
@@ -148,11 +153,13 @@ __device__ __forceinline__ void prime_sums(const cplx_t<T>* buf, const TileLay& 
             f[q].x -= r.y * d.x;
             f[q].y -= r.y * d.y;
         };
+        const int step = s.m * lay.tbp;
+        const C *pt = buf + lay.at(u, b), *pd = pt + p * step;   // t_j, d_j
         if (p <= PRIME_MAT) {
             const C* row = cs + g * PRIME_K;
 #pragma unroll 1
             for (int j = 1; j <= h; ++j, row += ng * PRIME_K) {
-                const C t = buf[lay.at(u + j * s.m, b)], d = buf[lay.at(u + (p - j) * s.m, b)];
+                const C t = *(pt += step), d = *(pd -= step);
                 sum = cadd(sum, t);
 #pragma unroll
                 for (int q = 0; q < PRIME_K; ++q) add(q, row[q], t, d);
@@ -163,7 +170,7 @@ __device__ __forceinline__ void prime_sums(const cplx_t<T>* buf, const TileLay& 
             for (int q = 0; q < PRIME_K; ++q) idx[q] = 0;
 #pragma unroll 1
             for (int j = 1; j <= h; ++j) {
-                const C t = buf[lay.at(u + j * s.m, b)], d = buf[lay.at(u + (p - j) * s.m, b)];
+                const C t = *(pt += step), d = *(pd -= step);
                 sum = cadd(sum, t);
 #pragma unroll
                 for (int q = 0; q < PRIME_K; ++q) {
@@ -201,9 +208,9 @@ struct FftTile {
     int nst, L;
     const C* tw;
     const C* cs;      // prime roots of st
-    C* cur;           // holds the tile between stages
-    C* oth;           // second buffer (only touched by stages from shared memory to shared memory)
-    __device__ __forceinline__ void swap() { C* t = cur; cur = oth; oth = t; }
+    C* buf;           // shared memory; the tile between stages is at buf + cur,
+    int cur, oth;     // the second buffer (only touched by stages from shared to shared memory) at buf + oth
+    __device__ __forceinline__ void swap() { const int t = cur; cur = oth; oth = t; }
 };
 
 // Stages s0..s1-1, smem -> smem from one buffer to the other (the tile in
@@ -228,18 +235,18 @@ __device__ __forceinline__ void mid_stages(FftTile<cplx_t<T>>& t, int s0, int s1
 #define CSIPM_MID(RR)                                                       \
                     case RR: {                                              \
                         C v[RR];                                            \
-                        bfly_load<T, RR, INV>(v, t.cur, lay, s, t.tw, u, k, b); \
-                        bfly_put<T, RR>(v, t.oth, lay, o, s.Ns, b);         \
+                        bfly_load<T, RR, INV>(v, t.buf + t.cur, lay, s, t.tw, u, k, b); \
+                        bfly_put<T, RR>(v, t.buf + t.oth, lay, o, s.Ns, b); \
                     } break;
                     CSIPM_RADICES(CSIPM_MID)
 #undef CSIPM_MID
                 }
             }
         } else {
-            C* buf = t.cur;
+            C* buf = t.buf + t.cur;
             prime_combine<T, INV>(buf, lay, s, false, t.tw, [&](int x, int c) { return buf[lay.at(x, c)]; });
             __syncthreads();
-            C* out = t.oth;
+            C* out = t.buf + t.oth;
             prime_sums<T, INV>(buf, lay, s, t.cs + s.cs, [&](int x, int c, C w) { out[lay.at(x, c)] = w; });
         }
         t.swap();
@@ -262,17 +269,17 @@ __device__ __forceinline__ void first_stage(FftTile<cplx_t<T>>& t, Ld& ld) {
                 C v[RR];                                                                  \
                 ld.template load<RR>(v, u, s.m, b);                                       \
                 Dft<RR, INV, T>::run(v);                                                  \
-                _Pragma("unroll") for (int r = 0; r < RR; ++r) t.cur[t.lay.at(u * RR + r, b)] = v[r]; \
+                bfly_put<T, RR>(v, t.buf + t.cur, t.lay, u * RR, 1, b);                  \
             }                                                                             \
             break;
         CSIPM_RADICES(CSIPM_FIRST)
 #undef CSIPM_FIRST
         default: {
-            C* out = t.oth;
+            C* out = t.buf + t.oth;
             const TileLay lay = t.lay;
-            prime_combine<T, INV>(t.cur, lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
+            prime_combine<T, INV>(t.buf + t.cur, lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
             __syncthreads();
-            prime_sums<T, INV>(t.cur, lay, s, t.cs + s.cs, [&](int x, int b, C v) { out[lay.at(x, b)] = v; });
+            prime_sums<T, INV>(t.buf + t.cur, lay, s, t.cs + s.cs, [&](int x, int b, C v) { out[lay.at(x, b)] = v; });
             t.swap();
         } break;
     }
@@ -293,15 +300,14 @@ __device__ __forceinline__ void last_stage(FftTile<cplx_t<T>>& t, St& out) {
             for (int w = threadIdx.x; w < s.m << lay.lg; w += blockDim.x) {               \
                 const int b = w & mask, u = w >> lay.lg;                                  \
                 C v[RR];                                                                  \
-                _Pragma("unroll") for (int r = 0; r < RR; ++r) v[r] = t.cur[lay.at(u + r * s.m, b)]; \
-                twiddle_dft<RR, INV, T>(v, u, s, t.tw);                                   \
+                bfly_load<T, RR, INV>(v, t.buf + t.cur, lay, s, t.tw, u, u, b);           \
                 out.template store<RR>(v, u, s.Ns, b);                                    \
             }                                                                             \
             break;
         CSIPM_RADICES(CSIPM_LAST)
 #undef CSIPM_LAST
         default: {
-            C* buf = t.cur;
+            C* buf = t.buf + t.cur;
             prime_combine<T, INV>(buf, lay, s, false, t.tw, [&](int x, int b) { return buf[lay.at(x, b)]; });
             __syncthreads();
             prime_sums<T, INV>(buf, lay, s, t.cs + s.cs,
@@ -331,9 +337,9 @@ __device__ __forceinline__ void fft_through(FftTile<cplx_t<T>>& t, Ld& ld, St& o
             CSIPM_RADICES(CSIPM_ONE)
 #undef CSIPM_ONE
             default:
-                prime_combine<T, INV>(t.cur, t.lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
+                prime_combine<T, INV>(t.buf + t.cur, t.lay, s, true, t.tw, [&](int x, int b) { return ld.one(x, b); });
                 __syncthreads();
-                prime_sums<T, INV>(t.cur, t.lay, s, t.cs + s.cs, [&](int x, int b, C v) { out.one(x, b, v); });
+                prime_sums<T, INV>(t.buf + t.cur, t.lay, s, t.cs + s.cs, [&](int x, int b, C v) { out.one(x, b, v); });
                 break;
         }
         return;

@@ -65,11 +65,11 @@ struct EpiGzMul {
     const double* Dq;
     long long n;
     double alpha, beta;
-    using Pre = NoPre;
-    __device__ __forceinline__ NoPre pre(int) const { return {}; }
-    __device__ __forceinline__ void put(int l, double v, const NoPre&) {
-        y[l] = alpha * (Dp[l] * x[l] + v) + beta * y[l];
-        y[n + l] = alpha * (Dq[l] * x[n + l] - v) + beta * y[n + l];
+    struct Pre { double xp, xq, dp, dq, yp, yq; };
+    __device__ __forceinline__ Pre pre(int l) const { return Pre{x[l], x[n + l], Dp[l], Dq[l], y[l], y[n + l]}; }
+    __device__ __forceinline__ void put(int l, double v, const Pre& r) {
+        y[l] = alpha * (r.dp * r.xp + v) + beta * r.yp;
+        y[n + l] = alpha * (r.dq * r.xq - v) + beta * r.yq;
     }
     __device__ __forceinline__ void finish() {}
 };

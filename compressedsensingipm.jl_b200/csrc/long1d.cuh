@@ -233,15 +233,15 @@ __device__ __forceinline__ void l1d_last_kernel_body(const PassArgs<T>& a, const
             const int c = w & (TH - 1), k2 = w >> lh, i = i0 + c;
             if (i >= npair) continue;
             const int k = i + P * k2;
-            const C zk = t.cur[t.lay.at(k2, c)];
+            const C zk = t.buf[t.cur + t.lay.at(k2, c)];
             if (k == 0) {
                 scatter1<T>(M, 0, r2c_post(zk, zk, twN[0]), ep);
                 scatter1<T>(M, M, mk((T)2 * (zk.x - zk.y), (T)0), ep);
             } else if (i == 0 || 2 * i == P) {
-                const C zm = t.cur[t.lay.at(i == 0 ? Q - k2 : Q - 1 - k2, c)];
+                const C zm = t.buf[t.cur + t.lay.at(i == 0 ? Q - k2 : Q - 1 - k2, c)];
                 scatter1<T>(M, k, r2c_post(zk, zm, twN[k]), ep);
             } else {
-                const C zm = t.cur[t.lay.at(Q - 1 - k2, TH + c)];
+                const C zm = t.buf[t.cur + t.lay.at(Q - 1 - k2, TH + c)];
                 scatter1<T>(M, k, r2c_post(zk, zm, twN[k]), ep);
                 scatter1<T>(M, M - k, r2c_post(zm, zk, twN[M - k]), ep);
             }

@@ -167,8 +167,10 @@ struct SpecLine {
     }
     template <int R> __device__ __forceinline__ void load(C* v, int u, int m, int) const {
         if (live) {
+            const C* q = p + u * sx;
+            const long long d = m * sx;
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = p[(u + r * m) * sx];
+            for (int r = 0; r < R; ++r, q += d) v[r] = *q;
         } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) v[r] = mk((T)0, (T)0);
@@ -176,8 +178,10 @@ struct SpecLine {
     }
     template <int R> __device__ __forceinline__ void store(const C* v, int u, int Ns, int) const {
         if (!live) return;
+        C* q = p + u * sx;
+        const long long d = Ns * sx;
 #pragma unroll
-        for (int r = 0; r < R; ++r) p[(u + r * Ns) * sx] = v[r];
+        for (int r = 0; r < R; ++r, q += d) *q = v[r];
     }
 };
 
@@ -287,7 +291,7 @@ struct ScatterLine {
                 return;
             }
         }
-        constexpr int U = 2;
+        constexpr int U = sizeof(typename Epi::Pre) > 48 ? 1 : 2;
 #pragma unroll
         for (int r0 = 0; r0 < R; r0 += U) {
             MapEntry en[U];

@@ -8,9 +8,11 @@
 // then HBM.  Measured on B200 against the former passes (radices up to 8,
 // every stage and load through shared memory, run-time index division, primes
 // as direct sums), A'A product in FP64: 310 x 410 x 410 (primes 31 and 41)
-// 10.64 -> 2.02 ms, the synthesis and analysis of a 1024^2 image 84 -> 51 us,
-// 1D 777600 137 -> 69 us, 1D 4096 26.8 -> 23.2 us; condensed KKT product at
-// 256^3 1.38 -> 0.81 ms; a batch of 16 images of sides 128-256 11.7 -> 8.6 ms.
+// 10.64 -> 1.95 ms, the synthesis and analysis of a 1024^2 image 84 -> 51 us,
+// 1D 777600 137 -> 61 us, 1D 4096 26.7 -> 21.8 us; condensed KKT product at
+// 256^3 1.38 -> 0.64 ms; a batch of 16 images of sides 128-256 11.7 -> 8.5 ms.
+// 80 registers (768 threads per SM) measured 8-21% slower on the 1D and 2D
+// passes than 128 (512 threads).
 #pragma once
 #include "fft_device.cuh"
 #include "operator.cuh"
@@ -29,9 +31,10 @@ __device__ __forceinline__ FftTile<cplx_t<T>> make_tile(const PassArgs<T>& a, un
     t.nst = a.pl.nst;
     t.L = a.pl.L;
     t.tw = a.tw;
-    t.cur = reinterpret_cast<C*>(smem);
-    t.oth = a.two ? t.cur + a.span : t.cur;
-    C* cs = t.oth + a.span;
+    t.buf = reinterpret_cast<C*>(smem);
+    t.cur = 0;
+    t.oth = a.two ? a.span : 0;
+    C* cs = t.buf + t.oth + a.span;
     t.cs = cs;
     if (a.primes) {
         prime_tables(a.fwd, a.pl.nst, a.tw, a.Ltab, cs);
@@ -162,10 +165,10 @@ __device__ __forceinline__ void chain_stage(FftTile<cplx_t<T>>& t, Keep&& keep) 
 #define CSIPM_CHAIN(RR)                                                                   \
             case RR: {                                                                    \
                 C v[RR];                                                                  \
-                bfly_load<T, RR, true>(v, t.cur, lay, s, t.tw, u, u, b);                  \
+                bfly_load<T, RR, true>(v, t.buf + t.cur, lay, s, t.tw, u, u, b);          \
                 _Pragma("unroll") for (int r = 0; r < RR; ++r) v[r] = keep(u + r * s.m, b, v[r]); \
                 Dft<RR, false, T>::run(v);                                                \
-                bfly_put<T, RR>(v, t.oth, lay, u * RR, 1, b);                             \
+                bfly_put<T, RR>(v, t.buf + t.oth, lay, u * RR, 1, b);                     \
             } break;
             CSIPM_RADICES(CSIPM_CHAIN)
 #undef CSIPM_CHAIN
@@ -201,7 +204,7 @@ __device__ __forceinline__ void row_pass_kernel_body(const PassArgs<T>& a) {
             // whole rows, coalesced, into the second buffer; C2R and the first
             // inverse stage read them there (read in place from global memory,
             // x and M - x of eight rows at a time thrashed the L1: 3x the time)
-            C* raw = t.oth;
+            C* raw = t.buf + t.oth;
 #pragma unroll 4
             for (int e = threadIdx.x; e < total; e += blockDim.x) {
                 const int rb = quot(e, M + 1, mag), k = e - rb * (M + 1);
@@ -227,10 +230,10 @@ __device__ __forceinline__ void row_pass_kernel_body(const PassArgs<T>& a) {
             if (r0 + rb >= a.nrows) break;
             C v;
             if (k == 0 || k == M) {
-                const C z0 = t.cur[t.lay.at(0, rb)];
+                const C z0 = t.buf[t.cur + t.lay.at(0, rb)];
                 v = k == 0 ? r2c_post(z0, z0, a.tw[0]) : mk((T)2 * (z0.x - z0.y), (T)0);
             } else {
-                v = r2c_post(t.cur[t.lay.at(k, rb)], t.cur[t.lay.at(M - k, rb)], a.tw[k]);
+                v = r2c_post(t.buf[t.cur + t.lay.at(k, rb)], t.buf[t.cur + t.lay.at(M - k, rb)], a.tw[k]);
             }
             a.spec[(size_t)(r0 + rb) * a.g.ld1 + k] = v;
         }
@@ -346,7 +349,7 @@ struct PassCfg {
     int threads = 0;
     size_t smem = 0;
     int pp = 1;          // 1: run-time-plan pass (TileLay fields below); 0: in-place row kernel
-    TileLay lay{0, 1, 31};
+    TileLay lay{0, 1};
     int span = 0, two = 0, primes = 0;
     FftStage fwd[FFT_MAX_STAGES], inv[FFT_MAX_STAGES];
     int tiles = 0;       // number of tiles of the pass
@@ -367,11 +370,10 @@ inline void lay_pass(const FftPlanDev& pl, int Ltab, int lines, int n, PassKind 
     TileLay l;
     l.lg = 0;
     while ((1 << l.lg) < lines) ++l.lg;
-    // rows are read and written along the row, so their pitch is odd; line
-    // tiles narrower than a 128-byte access are padded (TileLay)
+    // rows are read and written along the row, so their pitch is odd
     l.tbp = kind != PASS_LINES && lines > 1 ? lines + 1 : lines;
-    l.sh = (size_t)lines * csize >= 128 ? 31 : 3;
-    const int top = kind == PASS_ROWS ? pl.L : pl.L - 1;   // a staged row has M+1 values
+    c->lay = l;
+    c->span = (kind == PASS_ROWS ? pl.L + 1 : pl.L) * l.tbp;   // a staged row has M+1 values
     c->tiles = (n + lines - 1) / lines;
     const int table = prime_table_size(pl);
     c->primes = table > 0;
@@ -382,18 +384,12 @@ inline void lay_pass(const FftPlanDev& pl, int Ltab, int lines, int n, PassKind 
     c->two = kind == PASS_ROWS || pl.nst > 2 || (kind == PASS_PAIRS && pl.nst > 1);
     for (int s = 0; s + 1 < pl.nst || (s < pl.nst && kind != PASS_LINES); ++s)
         if (!reg_radix(pl.rad[s])) c->two = 1;
-    for (;;) {   // without the padding where a single long line does not fit with it
-        c->lay = l;
-        c->span = (top + (top >> l.sh) + 1) * l.tbp;
-        c->smem = ((size_t)c->span * (1 + c->two) + table) * csize;
-        if (l.sh == 31 || c->smem <= PASS_SMEM) break;
-        l.sh = 31;
-    }
+    c->smem = ((size_t)c->span * (1 + c->two) + table) * csize;
     if (threads == 0) {
         // the threads that keep the most lanes of an SM busy: resident threads
-        // (registers for 512 FP64 or 1024 FP32 of them, shared memory, and the
+        // (registers, shared memory, and the
         // tiles an SM gets) times the share of them the stages occupy
-        const int regs = csize >= 16 ? PASS_THREADS : 2 * PASS_THREADS;
+        const int regs = PASS_THREADS * (csize >= 16 ? pass_min_ctas<double>() : pass_min_ctas<float>());
         const int per_sm = (c->tiles + 147) / 148;
         double best = -1.0;
         for (int t = std::max(64, lines); t <= PASS_THREADS; t += 32) {

@@ -33,13 +33,14 @@ struct FftStage {
     int cs;                 // prime stages: where its cosines and sines start (prime_tables)
 };
 
-// Shared-memory place of element (x, b) of a tile.  b is fastest, so a stage
-// access of 8 FP64 (16 FP32) lines covers whole 128-byte rows; narrower
-// tiles leave one slot free after every 8 positions (sh = 3, else 31), or
-// the stride R of a stage's writes would fall on the same banks.
+// Shared-memory place of element (x, b) of a tile: x*tbp + b, b fastest, so a
+// stage access of 8 FP64 (16 FP32) lines covers whole 128-byte rows.  Narrower
+// tiles write with the stride R of a stage and meet 2- or 4-way bank conflicts
+// when R is even; padding against them (a slot after every 8 positions) cost
+// more in address arithmetic than the conflicts do.
 struct TileLay {
-    int lg, tbp, sh;   // log2(lines), pitch, padding shift
-    CSIPM_HD int at(int x, int b) const { return (x + (x >> sh)) * tbp + b; }
+    int lg, tbp;   // log2(lines), pitch
+    CSIPM_HD int at(int x, int b) const { return x * tbp + b; }
 };
 
 }  // namespace csipm

@@ -25,11 +25,7 @@ int csipm_obj(csipm_handle h, const double* x, double* f) {
     CK(op_AtA(h->op64, x, ep, nullptr, h->stream));
     h->matvecs++;
     const long long n = h->N;
-    ew_launch(dot2_kernel, n, h->stream, n, x, h->Qb, x, h->b, h->ws(h->slots + SL_DOT));
-    CK(cudaGetLastError());
-    // sum(c) = c . 1 : reuse Minv as a ones vector would cost a fill; use a dedicated reduction
-    ew_launch(fill_kernel, n, h->stream, n, 1.0, h->rhs);
-    ew_launch(dot2_kernel, n, h->stream, n, x + n, h->rhs, nullptr, nullptr, h->ws(h->slots + SL_DOT + 2));
+    ew_launch(obj_kernel, n, h->stream, n, x, (const double*)h->Qb, (const double*)h->b, h->ws(h->slots + SL_DOT));
     CK(cudaGetLastError());
     int r = read_slots(h, SL_DOT, 3);
     if (r) return r;

@@ -769,13 +769,27 @@ static __global__ void dot2_kernel(long long n, const double* __restrict__ a, co
 }
 
 // ------------------------------------------------------------------ NLPModels / KKT plugin
+// obj: beta.Qb, beta.b and sum(c) in one pass (a fill and two dot products
+// before: 720 x 462, 17 -> 7 us)
+static __global__ void obj_kernel(long long n, const double* __restrict__ x, const double* __restrict__ Qb,
+                                  const double* __restrict__ b, RedWorkspace ws) {
+    double acc[3] = {0.0, 0.0, 0.0};
+    CSIPM_GRID_LOOP(i, n) {
+        const double be = x[i];
+        acc[0] += be * Qb[i];
+        acc[1] += be * b[i];
+        acc[2] += x[n + i];
+    }
+    grid_reduce<3>(acc, ws, 0u, 0u);
+}
+
 // g = [AtA beta - Atz0 ; lambda] (beta part fused in the operator epilogue)
 struct EpiGrad {
     const double* b;
     double* g;
-    using Pre = NoPre;
-    __device__ __forceinline__ NoPre pre(int) const { return {}; }
-    __device__ __forceinline__ void put(int l, double v, const NoPre&) { g[l] = v - b[l]; }
+    using Pre = double;
+    __device__ __forceinline__ Pre pre(int l) const { return b[l]; }
+    __device__ __forceinline__ void put(int l, double v, Pre bl) { g[l] = v - bl; }
     __device__ __forceinline__ void finish() {}
 };
 
@@ -832,13 +846,14 @@ struct EpiCondensed {
     const double* L2;
     long long n;
     double alpha, beta;
-    using Pre = NoPre;
-    __device__ __forceinline__ NoPre pre(int) const { return {}; }
-    __device__ __forceinline__ void put(int l, double v, const NoPre&) {
-        const double xb = x[l], xz = x[n + l];
-        const double l1 = L1[l], l2 = L2[l];
-        y[l] = beta * y[l] + alpha * (v + l1 * xb + l2 * xz);
-        y[n + l] = beta * y[n + l] + alpha * (l2 * xb + l1 * xz);
+    // all six operands before any store: y may alias nothing the compiler
+    // knows of, so loads left in put() waited for the stores before them
+    // (256^3 product 0.81 -> 0.65 ms)
+    struct Pre { double xb, xz, l1, l2, yb, yz; };
+    __device__ __forceinline__ Pre pre(int l) const { return Pre{x[l], x[n + l], L1[l], L2[l], y[l], y[n + l]}; }
+    __device__ __forceinline__ void put(int l, double v, const Pre& r) {
+        y[l] = beta * r.yb + alpha * (v + r.l1 * r.xb + r.l2 * r.xz);
+        y[n + l] = beta * r.yz + alpha * (r.l2 * r.xb + r.l1 * r.xz);
     }
     __device__ __forceinline__ void finish() {}
 };
@@ -860,18 +875,25 @@ struct EpiKKT {
     double* y;          // 6N
     long long n;
     double alpha, beta;
-    using Pre = NoPre;
-    __device__ __forceinline__ NoPre pre(int) const { return {}; }
-    __device__ __forceinline__ void put(int l, double v, const NoPre&) {
+    struct Pre { double x[6], y[6]; };
+    __device__ __forceinline__ Pre pre(int l) const {
+        Pre r;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            r.x[q] = x[q * n + l];
+            r.y[q] = y[q * n + l];
+        }
+        return r;
+    }
+    __device__ __forceinline__ void put(int l, double v, const Pre& r) {
         const long long N = n;
-        const double xb = x[l], xz = x[N + l], xs1 = x[2 * N + l], xs2 = x[3 * N + l];
-        const double xy1 = x[4 * N + l], xy2 = x[5 * N + l];
-        y[l] = beta * y[l] + alpha * (v - xy1 + xy2);
-        y[N + l] = beta * y[N + l] - alpha * (xy1 + xy2);
-        y[2 * N + l] = beta * y[2 * N + l] - alpha * xy1;
-        y[3 * N + l] = beta * y[3 * N + l] - alpha * xy2;
-        y[4 * N + l] = beta * y[4 * N + l] + alpha * (-xb - xz - xs1);
-        y[5 * N + l] = beta * y[5 * N + l] + alpha * (xb - xz - xs2);
+        const double xb = r.x[0], xz = r.x[1], xs1 = r.x[2], xs2 = r.x[3], xy1 = r.x[4], xy2 = r.x[5];
+        y[l] = beta * r.y[0] + alpha * (v - xy1 + xy2);
+        y[N + l] = beta * r.y[1] - alpha * (xy1 + xy2);
+        y[2 * N + l] = beta * r.y[2] - alpha * xy1;
+        y[3 * N + l] = beta * r.y[3] - alpha * xy2;
+        y[4 * N + l] = beta * r.y[4] + alpha * (-xb - xz - xs1);
+        y[5 * N + l] = beta * r.y[5] + alpha * (xb - xz - xs2);
     }
     __device__ __forceinline__ void finish() {}
 };
