@@ -219,41 +219,38 @@ int ew_grid(const void* kernel, long long n) {
     return (int)std::max(1LL, std::min(b, (long long)wave));
 }
 
-int schur_cg(csipm_handle h, const double* rhs, double* x, bool has_x0, double rtol, int maxit, int* iters,
-             const double* r0v, const double* rtol_dev) {
+int schur_cg(csipm_handle h, const double* rhs, double* x, bool started, const double* x0, double rtol, int maxit,
+             int* iters, const double* rtol_dev) {
     const long long n = h->N;
     cudaStream_t st = h->stream;
     const double* Minv = h->opt.preconditioner ? h->Minv : nullptr;
     h->resid_kind = RESID_NONE;
-    CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
     const int ppp = passes_per_product(h->g);
-    const bool given = has_x0 && r0v != nullptr;
-    if (given) {
-        rhs = r0v;       // r = rhs - K x0 given: CG on it from x0 with no product
-        has_x0 = false;
-    } else if (has_x0) {
+    if (!started) {   // r = rhs - K x
+        CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
         EpiCG<double> ep{x, h->Db, h->cg_q, h->ws(h->slots + SL_DUMMY), 0.0};
         CK(solve_AtA(h, x, ep, nullptr, st));
         h->matvecs++;
-        h->launches += ppp;
-    } else if (!given) {
-        CK(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
+        ew_launch(cg_init_kernel<double>, n, st, n, rhs, h->cg_q, 1, Minv, h->cg_r, h->cg_p,
+                  h->ws(h->slots + SL_DUMMY), h->cgs, 0.0, DevScalar(rtol, rtol_dev));
+        CK(cudaGetLastError());
+        h->launches += ppp + 1;
     }
-    ew_launch(cg_init_kernel<double>, n, st, n, rhs, h->cg_q, has_x0 ? 1 : 0, Minv, h->cg_r, h->cg_p,
-                                                    h->ws(h->slots + SL_DUMMY), h->cgs, 0.0, DevScalar(rtol, rtol_dev));
-    CK(cudaGetLastError());
-    h->launches += 1;
     auto iteration = [&](cudaStream_t s, int it) -> cudaError_t {
         EpiCG<double> ep{h->cg_p, h->Db, h->cg_q, h->ws(&h->cgs->pq), 0.0};
         cudaError_t e = solve_AtA(h, h->cg_p, ep, &h->cgs->done, s);
         if (e != cudaSuccess) return e;
-        ew_launch(cg_update_kernel<double, double>, n, s, n, it, x, h->cg_r, h->cg_p, h->cg_q, Minv,
-                                                                   h->ws(h->slots + SL_DUMMY), h->cgs);
+        if (started)
+            ew_launch(cg_update_kernel<double, double, true>, n, s, n, it, x, x0, h->cg_r, h->cg_p, h->cg_q, Minv,
+                      h->ws(h->slots + SL_DUMMY), h->cgs);
+        else
+            ew_launch(cg_update_kernel<double, double, false>, n, s, n, it, x, x0, h->cg_r, h->cg_p, h->cg_q, Minv,
+                      h->ws(h->slots + SL_DUMMY), h->cgs);
         ew_launch(cg_pupdate_kernel<double>, n, s, n, it, h->cg_r, Minv, h->cg_p, h->cgs);
         return cudaGetLastError();
     };
-    // x is a kernel argument: a graph is only valid for the vector it was captured with
-    cudaGraphExec_t* ex = x == h->dba ? &h->cg_exec64[0] : (x == h->db ? &h->cg_exec64[1] : nullptr);
+    // a graph holds its vectors: one for the predictor's, one for the corrector's
+    cudaGraphExec_t* ex = !started ? nullptr : (x == h->dba ? &h->cg_exec64[0] : &h->cg_exec64[1]);
     const int r = cg_iterations(h, ex, maxit, iteration, ppp + 2);
     if (r) return r;
     CK(cudaMemcpyAsync(h->hcgs, h->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
@@ -294,8 +291,27 @@ static void ensure_diag64(csipm_handle h) {
     h->diag64_stale = false;
 }
 
+// h->rhs of the Newton solve under way, where a mixed solve needs it
+static int make_rhs(csipm_handle h) {
+    if (!h->rhs_due) return CSIPM_OK;
+    const long long n = h->N;
+    const double* bv = h->sorder ? h->bs : h->b;
+    const bool loose = h->opt.ipm_cg_rtol >= MIXED_FP32_WARM_RTOL;   // FP32 directions
+    const double* sm = h->slots + SL_SIGMU;
+    if (h->rhs_due == 2 && loose)
+        ew_launch(ipm_rhs_kernel<float>, n, h->stream, n, h->lambda, bv, (const double*)h->Qb, h->s1, h->s2, h->z1, h->z2,
+                  (const float*)h->f_dba, sm, h->rhs);
+    else
+        ew_launch(ipm_rhs_kernel<double>, n, h->stream, n, h->lambda, bv, (const double*)h->Qb, h->s1, h->s2, h->z1,
+                  h->z2, h->rhs_due == 2 ? (const double*)h->dba : nullptr, sm, h->rhs);
+    h->rhs_due = 0;
+    h->launches += 1;
+    CK(cudaGetLastError());
+    return CSIPM_OK;
+}
+
 int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, double rtol, int maxit, int* iters,
-                const double* r0v, float* xf, bool ready, const double* rin_dev) {
+                float* xf, bool started, const float* x0f, const double* rin_dev) {
     const long long n = h->N;
     cudaStream_t st = h->stream;
     const bool pc = h->opt.preconditioner != 0;
@@ -306,9 +322,7 @@ int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, doubl
     double r0 = -1.0, rn = -1.0;
     // loose Newton tolerances take the warm-start residual from the FP32
     // product: its rounding (~1e-7 relative) is far below what they ask
-    // a given warm-start residual serves round 0 with no product at all
-    const bool given = has_x0 && (r0v != nullptr || ready);
-    const bool fp32_warm = has_x0 && !given && rtol >= MIXED_FP32_WARM_RTOL;
+    const bool fp32_warm = has_x0 && !started && rtol >= MIXED_FP32_WARM_RTOL;
     h->resid_kind = RESID_NONE;
     // with xf, round 0 iterates on xf itself (no correction vector, no FP64
     // accumulation); any FP64 step (refinement, fallback) first takes the
@@ -320,16 +334,17 @@ int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, doubl
         h->launches += 1;
         in32 = false;
     };
-    if (!has_x0) {
+    if (!has_x0 && !started) {
         if (in32) CK(cudaMemsetAsync(xf, 0, sizeof(float) * n, st));
         else CK(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
     }
     int status = CSIPM_OK;
     for (int round = 0;; ++round) {
-        const double* res = given && round == 0 ? r0v : rhs;
+        const double* res = rhs;
         double rin = std::max(rtol, MIXED_INNER_RTOL);
-        if (round > 0 || (has_x0 && !fp32_warm && !given)) {
+        if (round > 0 || (has_x0 && !fp32_warm && !started)) {
             to64();
+            if (make_rhs(h)) return CSIPM_ERR_CUDA;
             ensure_diag64(h);
             EpiCG<double> ep{x, h->Db, h->cg_q, h->ws(h->slots + SL_DUMMY), 0.0};
             CK(solve_AtA(h, x, ep, nullptr, st));
@@ -355,10 +370,13 @@ int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, doubl
         }
         // FP32 PCG on K d = res: from d = 0 into f_x, or (in32) on xf from its start
         float* xi = in32 ? xf : h->f_x;
-        const bool started = ready && round == 0 && in32;   // r, p and the CG scalars already written
-        if (!started) CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
+        const bool go = started && round == 0;   // r, p and the CG scalars already written
+        if (!go) {
+            if (make_rhs(h)) return CSIPM_ERR_CUDA;
+            CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
+        }
         if (!in32) CK(cudaMemsetAsync(h->f_x, 0, sizeof(float) * n, st));
-        if (started) {
+        if (go) {
             // the FP32 CG starts from what the producing kernel wrote
         } else if (round == 0 && fp32_warm) {
             // warm-start residual rhs - K x0 with the FP32 product (x0 rounded to FP32)
@@ -380,21 +398,25 @@ int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, doubl
                                                              DevScalar(rin, round == 0 ? rin_dev : nullptr));
         }
         CK(cudaGetLastError());
-        if (!started) h->launches += 1;
+        if (!go) h->launches += 1;
         const int cap = std::min(maxit, MIXED_ROUND_MAXIT);
         auto iteration = [&](cudaStream_t s, int it) -> cudaError_t {
             EpiCG<float> ep{h->f_p, h->f_Db, h->f_q, h->ws(&h->cgs->pq), 0.0};
             cudaError_t e = solve_AtA32(h, h->f_p, ep, &h->cgs->done, s);
             if (e != cudaSuccess) return e;
-            ew_launch(cg_update_kernel<float, float>, n, s, n, it, xi, h->f_r, h->f_p, h->f_q, Minv32,
-                                                                    h->ws(h->slots + SL_DUMMY), h->cgs);
+            if (go)
+                ew_launch(cg_update_kernel<float, float, true>, n, s, n, it, xi, x0f, h->f_r, h->f_p, h->f_q, Minv32,
+                          h->ws(h->slots + SL_DUMMY), h->cgs);
+            else
+                ew_launch(cg_update_kernel<float, float, false>, n, s, n, it, xi, x0f, h->f_r, h->f_p, h->f_q, Minv32,
+                          h->ws(h->slots + SL_DUMMY), h->cgs);
             ew_launch(cg_pupdate_kernel<float>, n, s, n, it, h->f_r, Minv32, h->f_p, h->cgs);
             return cudaGetLastError();
         };
         {
             // a graph holds its vectors: one per iterate buffer
             cudaGraphExec_t* ex = xi == h->f_x ? &h->cg_exec32[0]
-                                  : (xi == h->f_dba ? &h->cg_exec32[1] : (xi == h->f_db ? &h->cg_exec32[2] : nullptr));
+                                  : (!go ? nullptr : (xi == h->f_dba ? &h->cg_exec32[1] : &h->cg_exec32[2]));
             const int r = cg_iterations(h, ex, cap, iteration, ppp + 2);
             if (r) return r;
         }
@@ -411,8 +433,9 @@ int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, doubl
         if (h->hcgs->breakdown) {
             to64();
             ensure_diag64(h);
+            if (make_rhs(h)) return CSIPM_ERR_CUDA;
             int its = 0;
-            status = schur_cg(h, rhs, x, true, std::min(0.5, rtol * r0 / rn), maxit, &its);
+            status = schur_cg(h, rhs, x, false, nullptr, std::min(0.5, rtol * r0 / rn), maxit, &its);
             total += its;
             h->fallbacks++;
             break;
@@ -517,7 +540,7 @@ int profile_impl(csipm_handle h, FftOperator<T>& op, const T* x, T* D, T* q, int
 // missing ones are allocated.
 int ensure_ipm_buffers(csipm_handle h) {
     const size_t n_ = (size_t)h->N;
-    double** f64[] = {&h->beta, &h->c, &h->s1, &h->s2, &h->z1, &h->z2, &h->rd, &h->Db, &h->Minv, &h->dba, &h->db,
+    double** f64[] = {&h->beta, &h->c, &h->s1, &h->s2, &h->z1, &h->z2, &h->Db, &h->Minv, &h->dba, &h->db,
                       &h->cg_r, &h->cg_p, &h->cg_q};
     for (double** q : f64)
         if (!*q && !h->alloc(q, n_)) return fail(h, CSIPM_ERR_OOM, h->err);
@@ -557,60 +580,60 @@ IpmMode ipm_mode(csipm_handle h) {
 }
 
 // The residual pass: the pending step on s and z (step), the dual residual,
-// the reductions of the stop test, the barrier diagonals and the predictor's
-// right-hand side; with FP32 directions also the start of the predictor's
-// FP32 CG at the tolerance *crtol.
+// the reductions of the stop test, the barrier diagonals and the start of the
+// predictor's CG at the tolerance *crtol (mixed precision at tight Newton
+// tolerances starts it from the right-hand side instead, make_rhs).
 cudaError_t launch_resid_pass(csipm_handle h, cudaStream_t st, const IpmMode& md, bool step, const double* crtol) {
     const long long n = h->N;
     const double lam = h->lambda;
-    const bool pc = h->opt.preconditioner != 0;
+    const int pc = h->opt.preconditioner != 0;
     const double* bv = h->sorder ? h->bs : h->b;
+    const DevScalar tol(0.0, crtol);
+    RedWorkspace ws = h->ws(h->slots + SL_RED);
+    const double *sm = h->slots + SL_SIGMU, *al = h->slots + SL_ALPHA;
+    h->rhs_due = md.mixed ? 1 : 0;
     if (md.dir32)
-        ew_launch(ipm_resdiag_kernel<float, float>, n, st, n, bv, h->Qb, lam, h->beta, h->s1, h->s2, h->z1, h->z2,
-                  step ? h->f_dba : nullptr, step ? h->f_db : nullptr, h->slots + SL_SIGMU, h->slots + SL_ALPHA,
-                  h->rd, (double*)nullptr, (double*)nullptr, h->f_Db, h->f_Minv, pc ? 1 : 0, h->rhs,
-                  h->ws(h->slots + SL_RED), h->f_r, h->f_p, h->cgs, DevScalar(0.0, crtol));
+        ew_launch(ipm_resdiag_kernel<float, float, float>, n, st, n, bv, h->Qb, lam, h->beta, h->s1, h->s2, h->z1, h->z2,
+                  step ? h->f_dba : nullptr, step ? h->f_db : nullptr, sm, al, (double*)nullptr, (double*)nullptr,
+                  h->f_Db, h->f_Minv, pc, ws, h->f_r, h->f_p, h->cgs, tol);
     else
-        ew_launch(ipm_resdiag_kernel<float, double>, n, st, n, bv, h->Qb, lam, h->beta, h->s1, h->s2, h->z1, h->z2,
-                  step ? h->dba : nullptr, step ? h->db : nullptr, h->slots + SL_SIGMU, h->slots + SL_ALPHA,
-                  h->rd, md.lazy64 ? nullptr : h->Db, md.lazy64 ? nullptr : h->Minv,
-                  md.mixed ? h->f_Db : nullptr, md.mixed ? h->f_Minv : nullptr, pc ? 1 : 0, h->rhs,
-                  h->ws(h->slots + SL_RED), (float*)nullptr, (float*)nullptr, (CgScalars*)nullptr, DevScalar());
+        ew_launch(ipm_resdiag_kernel<float, double, double>, n, st, n, bv, h->Qb, lam, h->beta, h->s1, h->s2, h->z1,
+                  h->z2, step ? h->dba : nullptr, step ? h->db : nullptr, sm, al, h->Db, h->Minv,
+                  md.mixed ? h->f_Db : nullptr, md.mixed ? h->f_Minv : nullptr, pc, ws,
+                  md.mixed ? nullptr : h->cg_r, md.mixed ? nullptr : h->cg_p, md.mixed ? nullptr : h->cgs, tol);
     return cudaGetLastError();
 }
 
-// The corrector's right-hand side after the predictor's step statistics and
-// centring target; rk says where the predictor left its residual (RESID_*),
-// from which the corrector's warm-start residual is formed with no product.
-// FP32 directions with a known residual: this pass also starts the
-// corrector's FP32 CG (r, p, scalars) at the tolerance *crtol.
-cudaError_t launch_corrector_rhs(csipm_handle h, cudaStream_t st, const IpmMode& md, int rk, const double* crtol) {
+// The start of the corrector's CG after the predictor's step statistics and
+// centring target, at the tolerance *crtol; rk says where the predictor left
+// its residual (RESID_*), from which the corrector's is formed with no
+// product.  Without one (mixed precision at tight tolerances, which refines
+// on exact residuals) only the start dba is copied; returns whether the CG
+// was started.
+cudaError_t launch_corrector_start(csipm_handle h, cudaStream_t st, const IpmMode& md, int rk, const double* crtol,
+                                   bool* started) {
     const long long n = h->N;
     const double lam = h->lambda;
-    const float* rp32 = rk == RESID_F32 ? h->f_r : nullptr;
-    const double* rp64 = rk == RESID_CG64 ? h->cg_r : nullptr;
-    const double* sigmu_d = h->slots + SL_SIGMU;
-    const bool cstart = md.dir32 && rk != RESID_NONE;
-    float* cr = cstart ? h->f_r : nullptr;
-    float* cp = cstart ? h->f_p : nullptr;
-    const float* cm = h->opt.preconditioner ? h->f_Minv : nullptr;
-    RedWorkspace cws = h->ws(h->slots + SL_DUMMY);
-    if (md.dir32 && rp32)
-        ew_launch(ipm_rhs_kernel<float, float>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, h->rd,
-                  (const float*)h->f_dba, sigmu_d, h->rhs, rp32, h->f_db, cr, cp, cm, h->cgs, cws,
-                  DevScalar(0.0, crtol));
+    const bool pc = h->opt.preconditioner != 0;
+    const double* sm = h->slots + SL_SIGMU;
+    RedWorkspace ws = h->ws(h->slots + SL_DUMMY);
+    const DevScalar tol(0.0, crtol);
+    *started = rk != RESID_NONE && (md.dir32 || !md.mixed);
+    if (md.mixed) h->rhs_due = 2;
+    if (!*started)
+        return md.dir32 ? cudaMemcpyAsync(h->f_db, h->f_dba, sizeof(float) * n, cudaMemcpyDeviceToDevice, st)
+                        : cudaMemcpyAsync(h->db, h->dba, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
+    if (md.dir32 && rk == RESID_F32)
+        ew_launch(ipm_corr_kernel<float, float, float>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, (const float*)h->f_dba,
+                  sm, (const float*)h->f_r, h->f_r, h->f_p, pc ? (const float*)h->f_Minv : nullptr, h->cgs, ws, tol);
     else if (md.dir32)
-        ew_launch(ipm_rhs_kernel<double, float>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, h->rd,
-                  (const float*)h->f_dba, sigmu_d, h->rhs, rp64, h->f_db, cr, cp, cm, h->cgs, cws,
-                  DevScalar(0.0, crtol));
-    else if (rp32)
-        ew_launch(ipm_rhs_kernel<float, double>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, h->rd,
-                  (const double*)h->dba, sigmu_d, h->rhs, rp32, h->db, (float*)nullptr, (float*)nullptr,
-                  (const float*)nullptr, (CgScalars*)nullptr, cws, DevScalar());
+        ew_launch(ipm_corr_kernel<double, float, float>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2,
+                  (const float*)h->f_dba, sm, (const double*)h->cg_r, h->f_r, h->f_p,
+                  pc ? (const float*)h->f_Minv : nullptr, h->cgs, ws, tol);
     else
-        ew_launch(ipm_rhs_kernel<double, double>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, h->rd,
-                  (const double*)h->dba, sigmu_d, h->rhs, rp64, h->db, (float*)nullptr, (float*)nullptr,
-                  (const float*)nullptr, (CgScalars*)nullptr, cws, DevScalar());
+        ew_launch(ipm_corr_kernel<double, double, double>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2,
+                  (const double*)h->dba, sm, (const double*)h->cg_r, h->cg_r, h->cg_p,
+                  pc ? (const double*)h->Minv : nullptr, h->cgs, ws, tol);
     return cudaGetLastError();
 }
 
@@ -710,9 +733,9 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
         ok = cudaGraphAddNode(&lnode, graph, nullptr, 0, &lp) == cudaSuccess;
     }
     // one CG loop over the iterate x (FP64) or xf (FP32)
-    auto cg_loop = [&](cudaStream_t s, cudaStream_t sb, double* x, float* xf) -> bool {
+    auto cg_loop = [&](cudaStream_t s, cudaStream_t sb, double* x, const double* x0, float* xf, const float* x0f) -> bool {
         auto arm = [&](cudaStream_t q, cudaGraphConditionalHandle hc) {
-            cg_arm_kernel<<<1, 1, 0, q>>>(hc, h->cgs);
+            cg_arm_kernel<<<1, 1, 0, q>>>(hc);
             ++kernels;
             return cudaGetLastError() == cudaSuccess;
         };
@@ -723,14 +746,14 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                     EpiCG<float> ep{h->f_p, h->f_Db, h->f_q, h->ws(&h->cgs->pq), 0.0};
                     e = solve_AtA32(h, h->f_p, ep, &h->cgs->done, q);
                     if (e != cudaSuccess) return false;
-                    ew_launch(cg_update_kernel<float, float>, n, q, n, it, xf, h->f_r, h->f_p, h->f_q, Minv32,
+                    ew_launch(cg_update_kernel<float, float, true>, n, q, n, it, xf, x0f, h->f_r, h->f_p, h->f_q, Minv32,
                               h->ws(h->slots + SL_DUMMY), h->cgs);
                     ew_launch(cg_pupdate_kernel<float>, n, q, n, it, h->f_r, Minv32, h->f_p, h->cgs);
                 } else {
                     EpiCG<double> ep{h->cg_p, h->Db, h->cg_q, h->ws(&h->cgs->pq), 0.0};
                     e = solve_AtA(h, h->cg_p, ep, &h->cgs->done, q);
                     if (e != cudaSuccess) return false;
-                    ew_launch(cg_update_kernel<double, double>, n, q, n, it, x, h->cg_r, h->cg_p, h->cg_q, Minv,
+                    ew_launch(cg_update_kernel<double, double, true>, n, q, n, it, x, x0, h->cg_r, h->cg_p, h->cg_q, Minv,
                               h->ws(h->slots + SL_DUMMY), h->cgs);
                     ew_launch(cg_pupdate_kernel<double>, n, q, n, it, h->cg_r, Minv, h->cg_p, h->cgs);
                 }
@@ -749,18 +772,8 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                                                cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
         cudaStream_t s0 = ss[0];
-        // ---- predictor from zero: FP32 directions start from the residual
-        // pass's CG start, FP64 ones from r = rhs
-        if (!md.dir32) {
-            ew_launch(fill_kernel, n, s0, n, 0.0, h->dba);
-            ew_launch(cg_init_kernel<double>, n, s0, n, (const double*)h->rhs, (const double*)nullptr, 0, Minv,
-                      h->cg_r, h->cg_p, h->ws(h->slots + SL_DUMMY), h->cgs, 0.0, DevScalar(0.0, rt_dev));
-            kernels += 2;
-        } else {
-            ew_launch(fill_f32_kernel, n, s0, n, 0.0f, h->f_dba);
-            kernels += 1;
-        }
-        ok = cg_loop(s0, ss[4], h->dba, h->f_dba);
+        // ---- predictor from zero: the residual pass started its CG
+        ok = cg_loop(s0, ss[4], h->dba, nullptr, h->f_dba, nullptr);
         ok = ok && capture_conditional(
                        s0, ss[1], cudaGraphCondTypeIf, [&](cudaStream_t q, cudaGraphConditionalHandle hi) { return check(1, hi, q); },
                        [&](cudaStream_t s1, cudaGraphConditionalHandle) -> bool {
@@ -774,18 +787,12 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                                          h->z2, (const double*)nullptr, (const double*)nullptr, h->dba,
                                          h->ws(h->slots + SL_SS));
                            ipm_sigma_kernel<<<1, 1, 0, s1>>>(h->slots + SL_SS, h->ctl, h->slots + SL_SIGMU);
-                           if (launch_corrector_rhs(h, s1, md, md.dir32 ? RESID_F32 : RESID_CG64, &h->ctl->rin) !=
-                               cudaSuccess)
+                           bool started = false;
+                           if (launch_corrector_start(h, s1, md, md.dir32 ? RESID_F32 : RESID_CG64,
+                                                      md.dir32 ? &h->ctl->rin : &h->ctl->rt, &started) != cudaSuccess)
                                return false;
                            kernels += 3;
-                           if (!md.dir32) {
-                               // r = rhs_c - K dba (written to rd by the rhs pass), from x = dba
-                               ew_launch(cg_init_kernel<double>, n, s1, n, (const double*)h->rd, (const double*)nullptr,
-                                         0, Minv, h->cg_r, h->cg_p, h->ws(h->slots + SL_DUMMY), h->cgs, 0.0,
-                                         DevScalar(0.0, rt_dev));
-                               ++kernels;
-                           }
-                           if (!cg_loop(s1, ss[4], h->db, h->f_db)) return false;
+                           if (!cg_loop(s1, ss[4], h->db, h->dba, h->f_db, h->f_dba)) return false;
                            return capture_conditional(
                                s1, ss[2], cudaGraphCondTypeIf,
                                [&](cudaStream_t q, cudaGraphConditionalHandle hi) { return check(2, hi, q); },
@@ -794,7 +801,7 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                                    if (launch_step(h, s2, md) != cudaSuccess) return false;
                                    EpiStore<double> ep{h->Qb};
                                    if (solve_AtA(h, h->beta, ep, nullptr, s2) != cudaSuccess) return false;
-                                   if (launch_resid_pass(h, s2, md, true, &h->ctl->rin_next) != cudaSuccess)
+                                   if (launch_resid_pass(h, s2, md, true, md.dir32 ? &h->ctl->rin_next : &h->ctl->rt_next) != cudaSuccess)
                                        return false;
                                    ipm_stop_kernel<<<1, 1, 0, s2>>>(h->slots + SL_RED, h->ctl, 1, loop);
                                    kernels += 3 + passes_per_product(h->g) + 2;
@@ -1118,19 +1125,20 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         qb_valid = false;
         h->diag64_stale = lazy64;
         {
-            // algorithmic bytes: b, Qb, beta, s1, s2, z1, z2 read; rd, rhs written;
-            // with the pending step the two directions read and s, z written;
-            // the barrier diagonals written in FP64 and/or FP32; with FP32
-            // directions the predictor CG's r and p written
+            // algorithmic bytes: b, Qb, beta, s1, s2, z1, z2 read; with the pending
+            // step the two directions read and s, z written; the barrier
+            // diagonals written in FP64 and/or FP32; the predictor CG's r and p
+            // written where the pass starts it
             const double td = dir32 ? 4.0 : 8.0;
-            const double per = 56.0 + 16.0 + (pending ? 2.0 * td + 32.0 : 0.0) + (lazy64 ? 0.0 : 16.0) +
-                               (mixed ? 8.0 : 0.0) + (dir32 ? 8.0 : 0.0);
+            const double per = 56.0 + (pending ? 2.0 * td + 32.0 : 0.0) + (lazy64 ? 0.0 : 16.0) +
+                               (mixed ? 8.0 : 0.0) + (dir32 ? 8.0 : (mixed ? 0.0 : 16.0));
             S.resid_pass_bytes += per * (double)n;
             S.resid_pass_launches += 1;
         }
         cudaEventRecord(h->ev_rp[0], st);
         // a resumed iteration restarts its predictor at this iteration's tolerance
-        CK(launch_resid_pass(h, st, md, pending, resume ? rin_dev : &h->ctl->rin_next));
+        CK(launch_resid_pass(h, st, md, pending,
+                             dir32 ? (resume ? rin_dev : &h->ctl->rin_next) : (resume ? rt_dev : &h->ctl->rt_next)));
         cudaEventRecord(h->ev_rp[1], st);
         pending = false;
         h->launches += 1;
@@ -1171,12 +1179,11 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
             }
         }
         const double rt = C.rt;                               // this iteration's Newton tolerance (host copy)
-        const double cg_rin = C.rin;
-        // ---- predictor (affine scaling): diagonals and right-hand side came with the residual
+        // ---- predictor (affine scaling): diagonals and the CG's start came with the residual
         int its = 0;
-        int cs = mixed ? schur_mixed(h, h->rhs, h->dba, false, rt, o.cg_maxit, &its, nullptr,
-                                     dir32 ? h->f_dba : nullptr, dir32, rin_dev)
-                       : schur_cg(h, h->rhs, h->dba, false, rt, o.cg_maxit, &its, nullptr, rt_dev);
+        int cs = mixed ? schur_mixed(h, h->rhs, h->dba, false, rt, o.cg_maxit, &its, dir32 ? h->f_dba : nullptr, dir32,
+                                     nullptr, rin_dev)
+                       : schur_cg(h, nullptr, h->dba, true, nullptr, rt, o.cg_maxit, &its, rt_dev);
         S.cg_iter += its;
         if (cs != CSIPM_OK && cs != CSIPM_ERR_CG_MAXITER) { status = cs; break; }
         // the centring target and the step length are computed on the device
@@ -1194,17 +1201,15 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         // product; mixed precision at tight Newton tolerances computes it
         // with an FP64 product instead, as refinement wants.
         const int rk = (!mixed || o.ipm_cg_rtol >= MIXED_FP32_WARM_RTOL) ? h->resid_kind : RESID_NONE;
-        CK(launch_corrector_rhs(h, st, md, rk, rin_dev));
-        const bool cstart = dir32 && rk != RESID_NONE;
-        const double* r0v = rk != RESID_NONE && !cstart ? h->rd : nullptr;
-        cs = mixed ? schur_mixed(h, h->rhs, h->db, true, rt, o.cg_maxit, &its, r0v, dir32 ? h->f_db : nullptr,
-                                 cstart, rin_dev)
-                   : schur_cg(h, h->rhs, h->db, true, rt, o.cg_maxit, &its, r0v, rt_dev);
+        bool cstart = false;
+        CK(launch_corrector_start(h, st, md, rk, dir32 ? rin_dev : rt_dev, &cstart));
+        cs = mixed ? schur_mixed(h, h->rhs, h->db, true, rt, o.cg_maxit, &its, dir32 ? h->f_db : nullptr, cstart,
+                                 dir32 ? h->f_dba : nullptr, rin_dev)
+                   : schur_cg(h, nullptr, h->db, true, h->dba, rt, o.cg_maxit, &its, rt_dev);
         S.cg_iter += its;
         if (cs != CSIPM_OK && cs != CSIPM_ERR_CG_MAXITER) { status = cs; break; }
-        (void)cg_rin;
         CK(launch_step(h, st, md));
-        h->launches += 6;   // sigma, corrector rhs, 2 step statistics, alpha, beta step (+ the Newton solves' launches)
+        h->launches += 6;   // sigma, corrector start, 2 step statistics, alpha, beta step (+ the Newton solves' launches)
         pending = true;
     }
     {
@@ -1284,7 +1289,6 @@ int csipm_admm(csipm_handle h, double rho, int maxt, double tol, double* z_out, 
         const double* x0 = X[(t + 1) & 1];
         // x-update: Krylov cg from zero, no preconditioner, atol = rtol = sqrt(eps) (src/admm.jl:35-37)
         CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
-        CK(cudaMemsetAsync(x1, 0, sizeof(double) * n, st));
         ew_launch(cg_init_kernel<double>, n, st, n, h->rhs, (const double*)nullptr, 0, (const double*)nullptr,
                                                         h->cg_r, h->cg_p, h->ws(h->slots + SL_DUMMY), h->cgs,
                                                         krylov_tol, krylov_tol);
@@ -1294,7 +1298,7 @@ int csipm_admm(csipm_handle h, double rho, int maxt, double tol, double* z_out, 
             EpiCG<double> ep{h->cg_p, h->Db, h->cg_q, h->ws(&h->cgs->pq), 0.0};
             cudaError_t e = solve_AtA(h, h->cg_p, ep, &h->cgs->done, s);
             if (e != cudaSuccess) return e;
-            ew_launch(cg_update_kernel<double, double>, n, s, n, it, x1, h->cg_r, h->cg_p, h->cg_q,
+            ew_launch(cg_update_kernel<double, double, true>, n, s, n, it, x1, (const double*)nullptr, h->cg_r, h->cg_p, h->cg_q,
                                                                        (const double*)nullptr,
                                                                        h->ws(h->slots + SL_DUMMY), h->cgs);
             ew_launch(cg_pupdate_kernel<double>, n, s, n, it, h->cg_r, (const double*)nullptr, h->cg_p,

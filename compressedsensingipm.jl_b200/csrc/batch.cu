@@ -36,7 +36,7 @@ struct BInst {
     int precond;
     int pad;
     const double* b;     // A^T z0, reference order
-    double *beta, *s1, *s2, *z1, *z2, *Qb, *rd, *Db, *Minv, *rhs, *dba, *db, *r, *p, *q, *c;
+    double *beta, *s1, *s2, *z1, *z2, *Qb, *Db, *Minv, *dba, *db, *r, *p, *q, *c;
     double* slots;
     double* partials;
     unsigned int* ticket;
@@ -83,11 +83,12 @@ __global__ void bk_ctl_start(const BInst* __restrict__ I, int count) {
 __global__ void __launch_bounds__(EW_THREADS, 3) bk_resid(const BInst* __restrict__ I, int step) {
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
-    ipm_resdiag_kernel_body<float, double>(q.n, q.b, q.Qb, q.lam, q.beta, q.s1, q.s2, q.z1, q.z2,
-                                           step ? q.dba : nullptr, step ? q.db : nullptr, q.slots + SL_SIGMU,
-                                           q.slots + SL_ALPHA, q.rd, q.Db, q.Minv, (float*)nullptr, (float*)nullptr,
-                                           q.precond, q.rhs, q.ws(q.slots + SL_RED), (float*)nullptr,
-                                           (float*)nullptr, (CgScalars*)nullptr, DevScalar());
+    // also starts the predictor's CG at the next iteration's tolerance
+    ipm_resdiag_kernel_body<float, double, double>(q.n, q.b, q.Qb, q.lam, q.beta, q.s1, q.s2, q.z1, q.z2,
+                                                   step ? q.dba : nullptr, step ? q.db : nullptr, q.slots + SL_SIGMU,
+                                                   q.slots + SL_ALPHA, q.Db, q.Minv, (float*)nullptr, (float*)nullptr,
+                                                   q.precond, q.ws(q.slots + SL_RED), q.r, q.p, q.cgs,
+                                                   DevScalar(0.0, &q.ctl->rt_next));
 }
 
 // stop test per instance; a stopped instance also closes its CG scalars so
@@ -101,27 +102,12 @@ __global__ void bk_stop(const BInst* __restrict__ I, int count) {
     if (q.ctl->status != IPM_RUNNING) q.cgs->done = 1;
 }
 
-__global__ void __launch_bounds__(EW_THREADS) bk_zero(const BInst* __restrict__ I, int which) {
-    const BInst& q = I[blockIdx.y];
-    if (!q.running()) return;
-    double* x = which ? q.db : q.dba;
-    CSIPM_GRID_LOOP(i, q.n) x[i] = 0.0;
-}
-
-// CG start r = rhs, p = Minv r at this iteration's Newton tolerance
-// (from = 0: the predictor's right-hand side; 1: the corrector's warm-start
-// residual, which the corrector right-hand side pass wrote to rd)
-__global__ void __launch_bounds__(EW_THREADS) bk_cg_init(const BInst* __restrict__ I, int from) {
-    const BInst& q = I[blockIdx.y];
-    if (!q.running()) return;
-    cg_init_kernel_body<double>(q.n, from ? q.rd : q.rhs, (const double*)nullptr, 0, q.precond ? q.Minv : nullptr,
-                                q.r, q.p, q.ws(q.slots + SL_DUMMY), q.cgs, 0.0, DevScalar(0.0, &q.ctl->rt));
-}
-
 __global__ void __launch_bounds__(EW_THREADS) bk_cg_update(const BInst* __restrict__ I, int it, int which) {
     const BInst& q = I[blockIdx.y];
-    cg_update_kernel_body<double, double>(q.n, it, which ? q.db : q.dba, q.r, q.p, q.q, q.precond ? q.Minv : nullptr,
-                                          q.ws(q.slots + SL_DUMMY), q.cgs);
+    // only an instance still running has a start of its own to copy
+    if (!q.running()) return;
+    cg_update_kernel_body<double, double, true>(q.n, it, which ? q.db : q.dba, which ? q.dba : nullptr, q.r, q.p, q.q,
+                                                q.precond ? q.Minv : nullptr, q.ws(q.slots + SL_DUMMY), q.cgs);
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_cg_pupdate(const BInst* __restrict__ I, int it) {
@@ -187,16 +173,14 @@ __global__ void bk_alpha(const BInst* __restrict__ I, int count) {
     ipm_alpha_kernel_body(q.slots + SL_SS, q.ctl, q.slots + SL_ALPHA);
 }
 
-// corrector right-hand side; rd receives the warm-start residual
-// rhs_c - K dba = rhs_c - rhs_p + r_p (r_p: the predictor CG's residual) and
-// db the warm start dba
-__global__ void __launch_bounds__(EW_THREADS) bk_rhs(const BInst* __restrict__ I) {
+// start of the corrector's CG from the predictor's residual, at the warm start dba
+__global__ void __launch_bounds__(EW_THREADS, 3) bk_corr(const BInst* __restrict__ I) {
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
-    ipm_rhs_kernel_body<double, double>(q.n, q.lam, q.s1, q.s2, q.z1, q.z2, q.rd, (const double*)q.dba,
-                                        q.slots + SL_SIGMU, q.rhs, (const double*)q.r, q.db, (float*)nullptr,
-                                        (float*)nullptr, (const float*)nullptr, (CgScalars*)nullptr,
-                                        q.ws(q.slots + SL_DUMMY), DevScalar());
+    ipm_corr_kernel_body<double, double, double>(q.n, q.lam, q.s1, q.s2, q.z1, q.z2, (const double*)q.dba,
+                                                 q.slots + SL_SIGMU, (const double*)q.r, q.r, q.p,
+                                                 q.precond ? (const double*)q.Minv : nullptr, q.cgs,
+                                                 q.ws(q.slots + SL_DUMMY), DevScalar(0.0, &q.ctl->rt));
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_beta_step(const BInst* __restrict__ I) {
@@ -513,8 +497,8 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
         q.lam = h->lambda;
         q.precond = h->opt.preconditioner ? 1 : 0;
         q.b = h->b;
-        q.beta = h->beta; q.s1 = h->s1; q.s2 = h->s2; q.z1 = h->z1; q.z2 = h->z2; q.Qb = h->Qb; q.rd = h->rd;
-        q.Db = h->Db; q.Minv = h->Minv; q.rhs = h->rhs; q.dba = h->dba; q.db = h->db;
+        q.beta = h->beta; q.s1 = h->s1; q.s2 = h->s2; q.z1 = h->z1; q.z2 = h->z2; q.Qb = h->Qb;
+        q.Db = h->Db; q.Minv = h->Minv; q.dba = h->dba; q.db = h->db;
         q.r = h->cg_r; q.p = h->cg_p; q.q = h->cg_q; q.c = h->c;
         q.slots = h->slots;
         q.partials = h->partials;
@@ -608,17 +592,13 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
         const int running = read_flag(B);
         if (running < 0) { status = fail(nullptr, CSIPM_ERR_CUDA, "batch synchronisation failed"); break; }
         if (running == 0) break;
-        // predictor from zero
-        bk_zero<<<ge, EW_THREADS, 0, st>>>(B.inst, 0);
-        bk_cg_init<<<ge, EW_THREADS, 0, st>>>(B.inst, 0);
-        B.launches += 2;
+        // predictor from zero (the residual pass started its CG)
         if ((status = batch_cg_loop(B, 0)) != CSIPM_OK) break;
         // centring target and corrector, warm-started at dba
         bk_stepstats<<<ge, EW_THREADS, 0, st>>>(B.inst, 0);
         bk_sigma<<<g1, 128, 0, st>>>(B.inst, count);
-        bk_rhs<<<ge, EW_THREADS, 0, st>>>(B.inst);
-        bk_cg_init<<<ge, EW_THREADS, 0, st>>>(B.inst, 1);
-        B.launches += 4;
+        bk_corr<<<ge, EW_THREADS, 0, st>>>(B.inst);
+        B.launches += 3;
         if ((status = batch_cg_loop(B, 1)) != CSIPM_OK) break;
         // step
         bk_stepstats<<<ge, EW_THREADS, 0, st>>>(B.inst, 1);

@@ -122,7 +122,7 @@ struct csipm_handle_s {
     double* b = nullptr;            // A^T z0
     bool sorder = false;            // solve runs in solver order (geometry.h)
     double* bs = nullptr;           // A^T z0 in solver order (when sorder)
-    double *beta = nullptr, *c = nullptr, *z1 = nullptr, *z2 = nullptr, *Qb = nullptr, *rd = nullptr;
+    double *beta = nullptr, *c = nullptr, *z1 = nullptr, *z2 = nullptr, *Qb = nullptr;
     double *s1 = nullptr, *s2 = nullptr;    // slacks c + beta, c - beta (stored; c is output scratch)
     double *Db = nullptr, *Minv = nullptr, *rhs = nullptr, *dba = nullptr, *db = nullptr;
     double *cg_r = nullptr, *cg_p = nullptr, *cg_q = nullptr;
@@ -152,6 +152,7 @@ struct csipm_handle_s {
     bool ipm_graph_off = false;     // its capture failed: csipm_solve runs plain iterations
     bool graphs_off = false;        // a capture failed: plain launches
     bool diag64_stale = false;      // FP64 Db/Minv not yet computed for this iterate (mixed precision)
+    int rhs_due = 0;                // the right-hand side rhs does not hold yet: 1 predictor, 2 corrector (mixed precision)
     int resid_kind = 0;             // where the last Newton solve left rhs - K x (RESID_*)
     int fallbacks = 0;              // mixed Newton solves finished in FP64 after an FP32 breakdown
 
@@ -398,22 +399,21 @@ constexpr double CG_FORCING_FLOOR = 1e-6;
 // the interior-point vectors of csipm_solve / csipm_admm, allocated on first use
 int ensure_ipm_buffers(csipm_handle h);
 
-// Newton solves of the condensed system K x = rhs.  has_x0: x holds a start;
-// r0v (optional, with has_x0): rhs - K x0 is already known and no product
-// is spent on it.  xf (schur_mixed, optional): the start and the result are
-// held in FP32 there instead of x (x is then scratch).  ready (with xf): the
-// kernel that produced the right-hand side (or the warm-start residual) also
-// wrote the FP32 CG start (f_r, f_p, h->cgs) for round 0.  On return
-// h->resid_kind says where the residual
-// rhs - K x of the result is held (RESID_*).
-// rtol_dev (optional): the device copy of rtol the CG thresholds are read
-// from (csipm_solve's control block: plain launches then read the same value
-// graph replays do); rin_dev likewise for round 0 of a mixed solve.
-int schur_cg(csipm_handle h, const double* rhs, double* x, bool has_x0, double rtol, int maxit, int* iters,
-             const double* r0v = nullptr, const double* rtol_dev = nullptr);
+// Newton solves of the condensed system K x = rhs.
+// schur_cg: started: the kernel before wrote the CG's start (cg_r, cg_p,
+// h->cgs) and the iterate starts at x0 (zero without); otherwise rhs is given
+// and x holds the start.  schur_mixed: xf (optional): the start and the
+// result are held in FP32 there instead of x (x is then scratch); started
+// (with xf): the FP32 CG's start (f_r, f_p, h->cgs) is written for round 0
+// and xf starts at x0f; has_x0: x (or xf) holds a start.  On return
+// h->resid_kind says where the residual rhs - K x of the result is held
+// (RESID_*).  rtol_dev (optional): the device copy of rtol the CG thresholds
+// are read from (csipm_solve's control block: plain launches then read the
+// same value graph replays do); rin_dev likewise for round 0 of a mixed solve.
+int schur_cg(csipm_handle h, const double* rhs, double* x, bool started, const double* x0, double rtol, int maxit,
+             int* iters, const double* rtol_dev = nullptr);
 int schur_mixed(csipm_handle h, const double* rhs, double* x, bool has_x0, double rtol, int maxit, int* iters,
-                const double* r0v = nullptr, float* xf = nullptr, bool ready = false,
-                const double* rin_dev = nullptr);
+                float* xf = nullptr, bool started = false, const float* x0f = nullptr, const double* rin_dev = nullptr);
 int ensure_kkt_buffers(csipm_handle h);
 int ensure_gondzio_buffers(csipm_handle h);
 

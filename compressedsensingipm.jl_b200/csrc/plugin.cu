@@ -123,14 +123,14 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
         // method's); the second halves of the 2N buffers hold the diagonals
         double *x = h->k_x, *r = h->k_r, *p = h->k_p, *q = h->k_q, *D = h->k_x + n, *M = h->k_r + n;
         const int so = h->sorder ? 1 : 0;
-        ew_launch(kkt_schur_init_kernel, so ? n / 2 : n, st, h->g, so, w, pr_diag, x, r, p, D, M,
+        ew_launch(kkt_schur_init_kernel, so ? n / 2 : n, st, h->g, so, w, pr_diag, r, p, D, M,
                   h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
         CK(cudaGetLastError());
         int chunk = 2, since = 0;
         for (int it = 0; it < maxit; ++it) {
             EpiCG<double> ep{p, D, q, h->ws(&h->cgs->pq), 0.0};
             CK(solve_AtA(h, p, ep, &h->cgs->done, st));
-            ew_launch(cg_update_kernel<double, double>, n, st, n, it, x, r, p, q, (const double*)M,
+            ew_launch(cg_update_kernel<double, double, true>, n, st, n, it, x, (const double*)nullptr, r, p, q, (const double*)M,
                       h->ws(h->slots + SL_DUMMY), h->cgs);
             ew_launch(cg_pupdate_kernel<double>, n, st, n, it, r, (const double*)M, p, h->cgs);
             CK(cudaGetLastError());

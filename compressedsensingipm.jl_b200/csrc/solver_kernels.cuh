@@ -102,15 +102,25 @@ static __global__ void cg_init_kernel(long long n, const double* __restrict__ rh
 }
 
 // alpha = rz/pq ; x += alpha p ; r -= alpha q ; rz' = r.(Minv r)
-template <typename TV, typename TX>
-__device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* __restrict__ x, TV* __restrict__ r, const TV* __restrict__ p,
-                                 const TV* __restrict__ q, const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
-    if (sc->done) return;
+// START: the first iteration takes its start from x0 (zero without one), so
+// nobody writes the start into x beforehand; a loop that is done before its
+// first step, or breaks down in it, copies the start.
+template <typename TV, typename TX, bool START>
+__device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* __restrict__ x, const TX* __restrict__ x0,
+                                 TV* __restrict__ r, const TV* __restrict__ p, const TV* __restrict__ q,
+                                 const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
+    const bool first = START && sc->iters == 0;
+    auto copy_start = [&]() { CSIPM_GRID_LOOP(k, n) x[k] = x0 ? x0[k] : (TX)0; };
+    if (sc->done) {
+        if (first && it == 0) copy_start();
+        return;
+    }
     const double pq = sc->full_pq();
     const double rz = sc->rz[it & 1];
-    // breakdown: every block sees the same p.q and returns before touching
-    // x or r, so the iterate stays the last good one
+    // breakdown: every block sees the same p.q and returns before stepping,
+    // so the iterate stays the last good one
     if (!(pq > 0.0) || !isfinite(pq)) {
+        if (first) copy_start();
         if (blockIdx.x == 0 && threadIdx.x == 0) { sc->breakdown = 1; sc->done = 1; }
         return;
     }
@@ -122,18 +132,24 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
         r[k] = (TV)rv;
         acc[0] += Minv ? rv * mv * rv : rv * rv;
     };
-    // two elements per trip with all loads issued first (load latency)
-    const long long G = (long long)gridDim.x * blockDim.x;
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    for (; i + G < n; i += 2 * G) {
-        const long long j = i + G;
-        const double xi = (double)x[i], xj = (double)x[j], ri = (double)r[i], rj = (double)r[j];
-        const double pi = (double)p[i], pj = (double)p[j], qi = (double)q[i], qj = (double)q[j];
-        const double mi = Minv ? (double)Minv[i] : 1.0, mj = Minv ? (double)Minv[j] : 1.0;
-        elem(i, xi, ri, pi, qi, mi);
-        elem(j, xj, rj, pj, qj, mj);
-    }
-    if (i < n) elem(i, (double)x[i], (double)r[i], (double)p[i], (double)q[i], Minv ? (double)Minv[i] : 1.0);
+    // two elements per trip with all loads issued first (load latency); one
+    // loop per source of x, so no branch sits between the loads
+    auto sweep = [&](auto&& xold) {
+        const long long G = (long long)gridDim.x * blockDim.x;
+        long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+        for (; i + G < n; i += 2 * G) {
+            const long long j = i + G;
+            const double xi = xold(i), xj = xold(j), ri = (double)r[i], rj = (double)r[j];
+            const double pi = (double)p[i], pj = (double)p[j], qi = (double)q[i], qj = (double)q[j];
+            const double mi = Minv ? (double)Minv[i] : 1.0, mj = Minv ? (double)Minv[j] : 1.0;
+            elem(i, xi, ri, pi, qi, mi);
+            elem(j, xj, rj, pj, qj, mj);
+        }
+        if (i < n) elem(i, xold(i), (double)r[i], (double)p[i], (double)q[i], Minv ? (double)Minv[i] : 1.0);
+    };
+    if (!first) sweep([&](long long k) { return (double)x[k]; });
+    else if (x0) sweep([&](long long k) { return (double)x0[k]; });
+    else sweep([&](long long) { return 0.0; });
     if (grid_reduce<1>(acc, ws, 0u, 0u) && threadIdx.x == 0) {
         // the last block: every other one has read sig and pq
         const double rho = sc->rho - alpha * sc->sig;
@@ -146,10 +162,10 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
         else if (sqrt(rzn) <= sc->thresh) sc->done = 1;
     }
 }
-template <typename TV, typename TX>
-static __global__ void cg_update_kernel(long long n, int it, TX* __restrict__ x, TV* __restrict__ r, const TV* __restrict__ p,
+template <typename TV, typename TX, bool START>
+static __global__ void cg_update_kernel(long long n, int it, TX* __restrict__ x, const TX* __restrict__ x0, TV* __restrict__ r, const TV* __restrict__ p,
                                  const TV* __restrict__ q, const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
-    cg_update_kernel_body<TV, TX>(n, it, x, r, p, q, Minv, ws, sc);
+    cg_update_kernel_body<TV, TX, START>(n, it, x, x0, r, p, q, Minv, ws, sc);
 }
 
 // p = Minv r + (rz'/rz) p
@@ -332,59 +348,85 @@ __device__ __forceinline__ ElemDir elem_affine(const ElemPre& e, double lam, dou
     return o;
 }
 
-// rhs = fb - L2 fc / L1 with fb = -rd + h1 - h2 (corrector: sigmu and the
-// second-order correction of the affine direction dba).  With rp (the
-// predictor solve's residual rhs_p - K dba) the corrector's warm-start
-// residual rhs - K dba = rhs - rhs_p + rp replaces rd (rd is not needed after
-// this pass; rhs still holds rhs_p on entry); with x0 the warm start
-// x0 = dba is written as well.
-//
-// With cr (FP32 corrector CG, rp given): the CG starts here instead of rd:
-// r = the warm-start residual, p = Minv r (cm: the rounded preconditioner,
-// null without one), r.(Minv r) reduced and the CG scalars set.  rp may be
-// the same vector as cr (read, then overwritten, by the same thread).
-template <typename TR, typename TD>
-__device__ __forceinline__ void ipm_rhs_kernel_body(long long n, double lam, const double* __restrict__ s1v, const double* __restrict__ s2v,
-                               const double* __restrict__ z1, const double* __restrict__ z2, double* rd,
-                               const TD* __restrict__ dba, const double* __restrict__ sigmu_p, double* rhs,
-                               const TR* rp, TD* __restrict__ x0, float* cr, float* __restrict__ cp,
-                               const float* __restrict__ cm, CgScalars* csc, RedWorkspace ws, DevScalar crtol) {
-    const double sigmu = sigmu_p ? *sigmu_p : 0.0;
-    double acc[1] = {0.0};
+// Right-hand side of a Newton solve, rhs = fb - L2 fc / L1 with
+// fb = -rd + h1 - h2 and rd = Qb - b - z1 + z2: the predictor's without dba,
+// else the corrector's (sigmu and the second-order correction of the affine
+// direction dba).  Mixed precision writes it for the solves that refine in
+// FP64; the others start their CG from the residual pass (predictor) and from
+// ipm_corr_kernel (corrector) and never form it.
+template <typename TD>
+__device__ __forceinline__ void ipm_rhs_kernel_body(long long n, double lam, const double* __restrict__ b,
+                               const double* __restrict__ Qb, const double* __restrict__ s1v, const double* __restrict__ s2v,
+                               const double* __restrict__ z1, const double* __restrict__ z2,
+                               const TD* __restrict__ dba, const double* __restrict__ sigmu_p, double* __restrict__ rhs) {
+    const double sigmu = dba ? *sigmu_p : 0.0;
     CSIPM_GRID_LOOP(i, n) {
         const ElemPre e = elem_pre(s1v[i], s2v[i], z1[i], z2[i]);
-        double cor1 = 0.0, cor2 = 0.0;
+        double h1 = -e.a, h2 = -e.d;
         if (dba) {
             const ElemDir f = elem_affine(e, lam, (double)dba[i]);
-            cor1 = f.ds1 * f.dz1;
-            cor2 = f.ds2 * f.dz2;
+            h1 += (sigmu - f.ds1 * f.dz1) * e.is1;
+            h2 += (sigmu - f.ds2 * f.dz2) * e.is2;
         }
-        const double h1 = (sigmu - cor1) * e.is1 - e.a;
-        const double h2 = (sigmu - cor2) * e.is2 - e.d;
-        const double fb = -rd[i] + h1 - h2;
+        const double fb = -(Qb[i] - b[i] - e.a + e.d) + h1 - h2;
         const double fc = -(lam - e.a - e.d) + h1 + h2;
-        const double rn = fb - e.L2 * fc * e.iL1;
-        if (cr) {
-            const double r0 = rn - rhs[i] + (double)rp[i];
-            const double zv = cm ? (double)cm[i] * r0 : r0;
-            cr[i] = (float)r0;
-            cp[i] = (float)zv;
-            acc[0] += r0 * zv;
-        } else if (rp) {
-            rd[i] = rn - rhs[i] + (double)rp[i];
-        }
-        rhs[i] = rn;
-        if (x0) x0[i] = dba[i];
+        rhs[i] = fb - e.L2 * fc * e.iL1;
     }
-    if (cr && grid_reduce<1>(acc, ws, 0u, 0u) && threadIdx.x == 0) cg_start(csc, ws.out[0], 0.0, crtol);
 }
-template <typename TR, typename TD>
-static __global__ void ipm_rhs_kernel(long long n, double lam, const double* __restrict__ s1v, const double* __restrict__ s2v,
-                               const double* __restrict__ z1, const double* __restrict__ z2, double* rd,
-                               const TD* __restrict__ dba, const double* __restrict__ sigmu_p, double* rhs,
-                               const TR* rp, TD* __restrict__ x0, float* cr, float* __restrict__ cp,
-                               const float* __restrict__ cm, CgScalars* csc, RedWorkspace ws, DevScalar crtol) {
-    ipm_rhs_kernel_body<TR, TD>(n, lam, s1v, s2v, z1, z2, rd, dba, sigmu_p, rhs, rp, x0, cr, cp, cm, csc, ws, crtol);
+template <typename TD>
+static __global__ void ipm_rhs_kernel(long long n, double lam, const double* __restrict__ b, const double* __restrict__ Qb,
+                               const double* __restrict__ s1v, const double* __restrict__ s2v,
+                               const double* __restrict__ z1, const double* __restrict__ z2,
+                               const TD* __restrict__ dba, const double* __restrict__ sigmu_p, double* __restrict__ rhs) {
+    ipm_rhs_kernel_body<TD>(n, lam, b, Qb, s1v, s2v, z1, z2, dba, sigmu_p, rhs);
+}
+
+// Start of the corrector's CG at the warm start dba: its residual is
+// rhs_c - K dba = rp + (rhs_c - rhs_p) with rp the predictor solve's residual,
+// and the difference of the right-hand sides is what the centring target and
+// the second-order correction add to h1 and h2,
+//     t1 - t2 - L2/L1 (t1 + t2),   t1 = (sigmu - ds1 dz1)/s1, t2 likewise,
+// so neither right-hand side nor the dual residual is read or written (they
+// were: 320^3 mixed 478 us and 16 bytes an element of the residual pass).
+// r = that residual, p = Minv r, r.(Minv r) and the CG scalars; cr may be rp.
+template <typename TR, typename TD, typename TC>
+__device__ __forceinline__ void ipm_corr_kernel_body(long long n, double lam, const double* __restrict__ s1v,
+                               const double* __restrict__ s2v, const double* __restrict__ z1, const double* __restrict__ z2,
+                               const TD* __restrict__ dba, const double* __restrict__ sigmu_p, const TR* rp, TC* cr,
+                               TC* __restrict__ cp, const TC* __restrict__ cm, CgScalars* csc, RedWorkspace ws,
+                               DevScalar crtol) {
+    const double sigmu = *sigmu_p;
+    double acc[1] = {0.0};
+    auto elem = [&](long long i, double s1, double s2, double a, double d, double xa, double rv, double mv) {
+        const ElemPre e = elem_pre(s1, s2, a, d);
+        const ElemDir f = elem_affine(e, lam, xa);
+        const double t1 = (sigmu - f.ds1 * f.dz1) * e.is1, t2 = (sigmu - f.ds2 * f.dz2) * e.is2;
+        const double r0 = rv + (t1 - t2 - e.L2 * (t1 + t2) * e.iL1);
+        const double zv = cm ? mv * r0 : r0;
+        cr[i] = (TC)r0;
+        cp[i] = (TC)zv;
+        acc[0] += r0 * zv;
+    };
+    const long long G = (long long)gridDim.x * blockDim.x;
+    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (; i + G < n; i += 2 * G) {   // two elements per trip, loads first
+        const long long j = i + G;
+        const double s1i = s1v[i], s1j = s1v[j], s2i = s2v[i], s2j = s2v[j], ai = z1[i], aj = z1[j], di = z2[i], dj = z2[j];
+        const double xi = (double)dba[i], xj = (double)dba[j], ri = (double)rp[i], rj = (double)rp[j];
+        const double mi = cm ? (double)cm[i] : 1.0, mj = cm ? (double)cm[j] : 1.0;
+        elem(i, s1i, s2i, ai, di, xi, ri, mi);
+        elem(j, s1j, s2j, aj, dj, xj, rj, mj);
+    }
+    if (i < n) elem(i, s1v[i], s2v[i], z1[i], z2[i], (double)dba[i], (double)rp[i], cm ? (double)cm[i] : 1.0);
+    if (grid_reduce<1>(acc, ws, 0u, 0u) && threadIdx.x == 0) cg_start(csc, ws.out[0], 0.0, crtol);
+}
+template <typename TR, typename TD, typename TC>
+static __global__ void __launch_bounds__(EW_THREADS, 3)
+ipm_corr_kernel(long long n, double lam, const double* __restrict__ s1v, const double* __restrict__ s2v,
+                const double* __restrict__ z1, const double* __restrict__ z2, const TD* __restrict__ dba,
+                const double* __restrict__ sigmu_p, const TR* rp, TC* cr, TC* __restrict__ cp,
+                const TC* __restrict__ cm, CgScalars* csc, RedWorkspace ws, DevScalar crtol) {
+    ipm_corr_kernel_body<TR, TD, TC>(n, lam, s1v, s2v, z1, z2, dba, sigmu_p, rp, cr, cp, cm, csc, ws, crtol);
 }
 
 // ------------------------------------------------------------------ IPM control
@@ -459,11 +501,10 @@ static __global__ void ipm_stop_kernel(const double* __restrict__ R, IpmCtl* __r
     ipm_stop_kernel_body(R, c, in_graph, hnd);
 }
 
-// Graph replays: opens a CG loop (a conditional while node) unless its start
-// already met the tolerance.  One thread.
-static __global__ void cg_arm_kernel(cudaGraphConditionalHandle hnd, const CgScalars* __restrict__ sc) {
-    cudaGraphSetConditional(hnd, sc->done ? 0u : 1u);
-}
+// Graph replays: opens a CG loop (a conditional while node), also one whose
+// start already met the tolerance: its passes return at once and the update
+// copies the start into the iterate.  One thread.
+static __global__ void cg_arm_kernel(cudaGraphConditionalHandle hnd) { cudaGraphSetConditional(hnd, 1u); }
 
 // Graph replays: after a CG loop, count its iterations and let the rest of
 // the iteration run only if it converged (a breakdown, or the loop's cap
@@ -617,16 +658,17 @@ static __global__ void admm_update_kernel(long long n, const double* __restrict_
 // rd = Qb - b - z1 + z2 and the scalar diagnostics (reductions RR_*), the
 // barrier diagonals of the condensed Schur system Db = 4 D1 D2/(D1 + D2),
 // Minv = 1/(1 + Db) (FP64 when Db is given, FP32 copies for mixed
-// precision), and the predictor right-hand side (h1 = -z1, h2 = -z2,
-// fc = -lambda).
-template <typename TV, typename TD>
+// precision), and the start of the predictor's CG from x = 0: r = the
+// predictor right-hand side (h1 = -z1, h2 = -z2, fc = -lambda), p = Minv r
+// and the CG scalars, in the precision TC of that CG.
+template <typename TV, typename TD, typename TC>
 __device__ __forceinline__ void ipm_resdiag_kernel_body(long long n, const double* __restrict__ b, const double* __restrict__ Qb, double lam,
                    const double* __restrict__ beta, double* __restrict__ s1v, double* __restrict__ s2v,
                    double* __restrict__ z1, double* __restrict__ z2, const TD* __restrict__ dba,
                    const TD* __restrict__ db, const double* __restrict__ sigmu_p,
-                   const double* __restrict__ alpha_p, double* __restrict__ rd, double* __restrict__ Db,
+                   const double* __restrict__ alpha_p, double* __restrict__ Db,
                    double* __restrict__ Minv, TV* __restrict__ Db_lo, TV* __restrict__ Minv_lo, int precond,
-                   double* __restrict__ rhs, RedWorkspace ws, TV* __restrict__ cr, TV* __restrict__ cp,
+                   RedWorkspace ws, TC* __restrict__ cr, TC* __restrict__ cp,
                    CgScalars* csc, DevScalar crtol) {
     double acc[RR_N] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     const bool step = db != nullptr;
@@ -649,7 +691,6 @@ __device__ __forceinline__ void ipm_resdiag_kernel_body(long long n, const doubl
         }
         const double ce = 0.5 * (s1 + s2);
         const double r = q - bb - a + d;
-        rd[i] = r;
         const double rc = lam - a - d;
         acc[RR_SZ] += s1 * a + s2 * d;
         acc[RR_BB] += bb * be;
@@ -663,14 +704,11 @@ __device__ __forceinline__ void ipm_resdiag_kernel_body(long long n, const doubl
         const double dbv = g.db, mi = g.mi;
         if (Db) { Db[i] = dbv; Minv[i] = mi; }
         if (Db_lo) { Db_lo[i] = (TV)dbv; Minv_lo[i] = (TV)mi; }
-        const double v = -r - a + d + lam * g.l2l1;
-        rhs[i] = v;
-        if (cr) {
-            // start of the predictor's FP32 CG (r = rhs, p = Minv r, from x = 0),
-            // with the rounded preconditioner the CG kernels read
-            const double zv = (double)(TV)mi * v;
-            cr[i] = (TV)v;
-            cp[i] = (TV)zv;
+        if (cr) {   // with the rounded preconditioner the CG kernels read
+            const double v = -r - a + d + lam * g.l2l1;
+            const double zv = (double)(TC)mi * v;
+            cr[i] = (TC)v;
+            cp[i] = (TC)zv;
             acc[RR_RZ] += v * zv;
         }
     };
@@ -692,17 +730,17 @@ __device__ __forceinline__ void ipm_resdiag_kernel_body(long long n, const doubl
              b[i]);
     if (grid_reduce<RR_N>(acc, ws, RR_MAXMASK, 0u) && csc && threadIdx.x == 0) cg_start(csc, ws.out[RR_RZ], 0.0, crtol);
 }
-template <typename TV, typename TD>
+template <typename TV, typename TD, typename TC>
 static __global__ void __launch_bounds__(EW_THREADS, 3)
 ipm_resdiag_kernel(long long n, const double* __restrict__ b, const double* __restrict__ Qb, double lam,
                    const double* __restrict__ beta, double* __restrict__ s1v, double* __restrict__ s2v,
                    double* __restrict__ z1, double* __restrict__ z2, const TD* __restrict__ dba,
                    const TD* __restrict__ db, const double* __restrict__ sigmu_p,
-                   const double* __restrict__ alpha_p, double* __restrict__ rd, double* __restrict__ Db,
+                   const double* __restrict__ alpha_p, double* __restrict__ Db,
                    double* __restrict__ Minv, TV* __restrict__ Db_lo, TV* __restrict__ Minv_lo, int precond,
-                   double* __restrict__ rhs, RedWorkspace ws, TV* __restrict__ cr, TV* __restrict__ cp,
+                   RedWorkspace ws, TC* __restrict__ cr, TC* __restrict__ cp,
                    CgScalars* csc, DevScalar crtol) {
-    ipm_resdiag_kernel_body<TV, TD>(n, b, Qb, lam, beta, s1v, s2v, z1, z2, dba, db, sigmu_p, alpha_p, rd, Db, Minv, Db_lo, Minv_lo, precond, rhs, ws, cr, cp, csc, crtol);
+    ipm_resdiag_kernel_body<TV, TD, TC>(n, b, Qb, lam, beta, s1v, s2v, z1, z2, dba, db, sigmu_p, alpha_p, Db, Minv, Db_lo, Minv_lo, precond, ws, cr, cp, csc, crtol);
 }
 
 // FP64 barrier diagonals alone (mixed precision at loose Newton tolerances
@@ -794,10 +832,6 @@ struct EpiGrad {
 };
 
 static __global__ void fill_kernel(long long n, double v, double* __restrict__ y) {
-    CSIPM_GRID_LOOP(i, n) y[i] = v;
-}
-
-static __global__ void fill_f32_kernel(long long n, float v, float* __restrict__ y) {
     CSIPM_GRID_LOOP(i, n) y[i] = v;
 }
 
@@ -982,10 +1016,10 @@ __device__ __forceinline__ void kkt_rhs(const double* __restrict__ w, long long 
     bz = w[n + i] - w3 - w4 - a - c;
 }
 
-// start: x = 0, r = r~, p = M r, the diagonals D and M, and the scalars
+// start from x = 0 (cg_update's START): r = r~, p = M r, the diagonals D and M, the scalars
 static __global__ void __launch_bounds__(EW_THREADS)
 kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const double* __restrict__ pr_diag,
-                      double* __restrict__ x, double* __restrict__ r, double* __restrict__ p, double* __restrict__ D,
+                      double* __restrict__ r, double* __restrict__ p, double* __restrict__ D,
                       double* __restrict__ M, RedWorkspace ws, CgScalars* sc, double atol, double rtol) {
     const long long n = g.N;
     double acc[2] = {0.0, 0.0};
@@ -995,7 +1029,6 @@ kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const do
         kkt_rhs(w, n, i, S1, S2, bb, bz);
         const double u = bz / l1, d = 4.0 * (S1 / l1) * S2, m = 1.0 / (1.0 + d);
         const double rv = sg * (bb - (S1 - S2) * u), z = m * rv;
-        x[s] = 0.0;
         r[s] = rv;
         p[s] = z;
         D[s] = d;
