@@ -70,6 +70,7 @@ namespace csipm_internal {
 // between beta entries and the sources of the half spectrum).
 template <bool TO_SOL>
 static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in, double* __restrict__ out) {
+    pdl_enter();
     const int64_t tail = g.N - 2 * g.NI;
     const int64_t total = g.NI + tail;
     const int pl = g.m1 - 1;
@@ -97,12 +98,12 @@ static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in
 }
 
 cudaError_t to_solver_order(const Geom& g, const double* ref, double* sol, cudaStream_t st) {
-    solver_order_kernel<true><<<ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st>>>(g, ref, sol);
+    launch_pdl(pdl_pays(g.dim, g.N), solver_order_kernel<true>, ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, ref, sol);
     return cudaGetLastError();
 }
 
 cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, cudaStream_t st) {
-    solver_order_kernel<false><<<ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st>>>(g, sol, ref);
+    launch_pdl(pdl_pays(g.dim, g.N), solver_order_kernel<false>, ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, sol, ref);
     return cudaGetLastError();
 }
 
@@ -122,6 +123,7 @@ cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, cu
 constexpr int CG_WHILE_CAP = 2000;
 
 static __global__ void cg_continue_kernel(cudaGraphConditionalHandle hnd, const CgScalars* __restrict__ sc, int cap) {
+    pdl_enter();
     cudaGraphSetConditional(hnd, (sc->done == 0 && sc->iters < cap) ? 1u : 0u);
 }
 
@@ -148,7 +150,7 @@ bool build_cg_while(csipm_handle h, cudaGraphExec_t* exec, int cap, Iter& iterat
              cudaSuccess;
         if (ok) {
             ok = iteration(cs, 0) == cudaSuccess && iteration(cs, 1) == cudaSuccess;
-            cg_continue_kernel<<<1, 1, 0, cs>>>(hnd, h->cgs, cap);
+            launch_pdl(true, cg_continue_kernel, 1, 1, 0, cs, hnd, h->cgs, cap);
             ok = cudaGetLastError() == cudaSuccess && ok;
             cudaGraph_t out = nullptr;
             ok = cudaStreamEndCapture(cs, &out) == cudaSuccess && ok;
@@ -650,7 +652,7 @@ cudaError_t launch_step(csipm_handle h, cudaStream_t st, const IpmMode& md) {
     else
         ew_launch(ipm_stepstats_kernel<double>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2, (const double*)h->dba,
                   sigmu_d, (const double*)h->db, h->ws(h->slots + SL_SS));
-    ipm_alpha_kernel<<<1, 1, 0, st>>>(h->slots + SL_SS, h->ctl, alpha_d);
+    launch_pdl(true, ipm_alpha_kernel, 1, 1, 0, st, h->slots + SL_SS, h->ctl, alpha_d);
     if (md.dir32)
         ew_launch(ipm_beta_step_kernel<float>, n, st, n, h->beta, (const float*)h->f_db, (const double*)alpha_d);
     else
@@ -735,7 +737,7 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
     // one CG loop over the iterate x (FP64) or xf (FP32)
     auto cg_loop = [&](cudaStream_t s, cudaStream_t sb, double* x, const double* x0, float* xf, const float* x0f) -> bool {
         auto arm = [&](cudaStream_t q, cudaGraphConditionalHandle hc) {
-            cg_arm_kernel<<<1, 1, 0, q>>>(hc);
+            launch_pdl(true, cg_arm_kernel, 1, 1, 0, q, hc);
             ++kernels;
             return cudaGetLastError() == cudaSuccess;
         };
@@ -758,13 +760,13 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                     ew_launch(cg_pupdate_kernel<double>, n, q, n, it, h->cg_r, Minv, h->cg_p, h->cgs);
                 }
             }
-            cg_continue_kernel<<<1, 1, 0, q>>>(hc, h->cgs, cap);
+            launch_pdl(true, cg_continue_kernel, 1, 1, 0, q, hc, h->cgs, cap);
             return cudaGetLastError() == cudaSuccess;
         };
         return capture_conditional(s, sb, cudaGraphCondTypeWhile, arm, body);
     };
     auto check = [&](int which, cudaGraphConditionalHandle hi, cudaStream_t q) {
-        ipm_cg_check_kernel<<<1, 1, 0, q>>>(h->cgs, h->ctl, which, cap_is_limit, hi, loop);
+        launch_pdl(true, ipm_cg_check_kernel, 1, 1, 0, q, h->cgs, h->ctl, which, cap_is_limit, hi, loop);
         ++kernels;
         return cudaGetLastError() == cudaSuccess;
     };
@@ -786,7 +788,7 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                                ew_launch(ipm_stepstats_kernel<double>, n, s1, n, h->lambda, h->s1, h->s2, h->z1,
                                          h->z2, (const double*)nullptr, (const double*)nullptr, h->dba,
                                          h->ws(h->slots + SL_SS));
-                           ipm_sigma_kernel<<<1, 1, 0, s1>>>(h->slots + SL_SS, h->ctl, h->slots + SL_SIGMU);
+                           launch_pdl(true, ipm_sigma_kernel, 1, 1, 0, s1, h->slots + SL_SS, h->ctl, h->slots + SL_SIGMU);
                            bool started = false;
                            if (launch_corrector_start(h, s1, md, md.dir32 ? RESID_F32 : RESID_CG64,
                                                       md.dir32 ? &h->ctl->rin : &h->ctl->rt, &started) != cudaSuccess)
@@ -803,7 +805,7 @@ bool build_ipm_graph(csipm_handle h, const IpmMode& md) {
                                    if (solve_AtA(h, h->beta, ep, nullptr, s2) != cudaSuccess) return false;
                                    if (launch_resid_pass(h, s2, md, true, md.dir32 ? &h->ctl->rin_next : &h->ctl->rt_next) != cudaSuccess)
                                        return false;
-                                   ipm_stop_kernel<<<1, 1, 0, s2>>>(h->slots + SL_RED, h->ctl, 1, loop);
+                                   launch_pdl(true, ipm_stop_kernel, 1, 1, 0, s2, h->slots + SL_RED, h->ctl, 1, loop);
                                    kernels += 3 + passes_per_product(h->g) + 2;
                                    return cudaGetLastError() == cudaSuccess;
                                });
@@ -1143,7 +1145,7 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         pending = false;
         h->launches += 1;
         if (!resume) {
-            ipm_stop_kernel<<<1, 1, 0, st>>>(h->slots + SL_RED, h->ctl, 0, 0);
+            launch_pdl(true, ipm_stop_kernel, 1, 1, 0, st, h->slots + SL_RED, h->ctl, 0, 0);
             CK(cudaGetLastError());
             h->launches += 1;
         }
@@ -1194,7 +1196,7 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         else
             ew_launch(ipm_stepstats_kernel<double>, n, st, n, lam, h->s1, h->s2, h->z1, h->z2,
                       (const double*)nullptr, (const double*)nullptr, h->dba, h->ws(h->slots + SL_SS));
-        ipm_sigma_kernel<<<1, 1, 0, st>>>(h->slots + SL_SS, h->ctl, h->slots + SL_SIGMU);
+        launch_pdl(true, ipm_sigma_kernel, 1, 1, 0, st, h->slots + SL_SS, h->ctl, h->slots + SL_SIGMU);
         // ---- corrector, warm-started at dba.  Its starting residual
         // rhs_c - K dba = rhs_c - rhs_p + (rhs_p - K dba) comes from the
         // predictor solve's residual (kept by CG's recurrence) with no

@@ -62,17 +62,20 @@ struct BPass {
 // csipm_solve launches; an instance that has stopped returns at once (all
 // its blocks alike, so no reduction waits on it).
 __global__ void __launch_bounds__(EW_THREADS) bk_init1(const BInst* __restrict__ I) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     ipm_init1_kernel_body(q.n, q.b, q.lam, q.beta, q.ws(q.slots + SL_MAXB));
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_init2(const BInst* __restrict__ I) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     ipm_init2_kernel_body(q.n, q.b, q.Qb, q.lam, q.beta, q.slots + SL_MAXB, q.s1, q.s2, q.z1, q.z2);
 }
 
 // control blocks take ||z0||^2 and the KKT scale from the slots (one thread per instance)
 __global__ void bk_ctl_start(const BInst* __restrict__ I, int count) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const BInst& q = I[k];
@@ -81,6 +84,7 @@ __global__ void bk_ctl_start(const BInst* __restrict__ I, int count) {
 }
 
 __global__ void __launch_bounds__(EW_THREADS, 3) bk_resid(const BInst* __restrict__ I, int step) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
     // also starts the predictor's CG at the next iteration's tolerance
@@ -94,6 +98,7 @@ __global__ void __launch_bounds__(EW_THREADS, 3) bk_resid(const BInst* __restric
 // stop test per instance; a stopped instance also closes its CG scalars so
 // the CG loops of the step skip it
 __global__ void bk_stop(const BInst* __restrict__ I, int count) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const BInst& q = I[k];
@@ -103,6 +108,7 @@ __global__ void bk_stop(const BInst* __restrict__ I, int count) {
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_cg_update(const BInst* __restrict__ I, int it, int which) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     // only an instance still running has a start of its own to copy
     if (!q.running()) return;
@@ -111,6 +117,7 @@ __global__ void __launch_bounds__(EW_THREADS) bk_cg_update(const BInst* __restri
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_cg_pupdate(const BInst* __restrict__ I, int it) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     cg_pupdate_kernel_body<double>(q.n, it, q.r, q.precond ? q.Minv : nullptr, q.p, q.cgs);
 }
@@ -118,6 +125,7 @@ __global__ void __launch_bounds__(EW_THREADS) bk_cg_pupdate(const BInst* __restr
 // after a CG loop: count its iterations; a breakdown stops the instance
 // (csipm_solve reports it as non-finite); one thread per instance
 __global__ void bk_cg_post(const BInst* __restrict__ I, int count) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const BInst& q = I[k];
@@ -128,6 +136,7 @@ __global__ void bk_cg_post(const BInst* __restrict__ I, int count) {
 
 // instances still iterating a CG loop (done clear) -> *out
 __global__ void bk_cg_active(const BInst* __restrict__ I, int count, int* __restrict__ out) {
+    pdl_enter();
     __shared__ int s;
     if (threadIdx.x == 0) s = 0;
     __syncthreads();
@@ -139,6 +148,7 @@ __global__ void bk_cg_active(const BInst* __restrict__ I, int count, int* __rest
 }
 
 __global__ void bk_running(const BInst* __restrict__ I, int count, int* __restrict__ out) {
+    pdl_enter();
     __shared__ int s;
     if (threadIdx.x == 0) s = 0;
     __syncthreads();
@@ -150,6 +160,7 @@ __global__ void bk_running(const BInst* __restrict__ I, int count, int* __restri
 }
 
 __global__ void __launch_bounds__(EW_THREADS, 3) bk_stepstats(const BInst* __restrict__ I, int corrector) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
     ipm_stepstats_kernel_body<double>(q.n, q.lam, q.s1, q.s2, q.z1, q.z2, corrector ? q.dba : nullptr,
@@ -158,6 +169,7 @@ __global__ void __launch_bounds__(EW_THREADS, 3) bk_stepstats(const BInst* __res
 }
 
 __global__ void bk_sigma(const BInst* __restrict__ I, int count) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const BInst& q = I[k];
@@ -166,6 +178,7 @@ __global__ void bk_sigma(const BInst* __restrict__ I, int count) {
 }
 
 __global__ void bk_alpha(const BInst* __restrict__ I, int count) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const BInst& q = I[k];
@@ -175,6 +188,7 @@ __global__ void bk_alpha(const BInst* __restrict__ I, int count) {
 
 // start of the corrector's CG from the predictor's residual, at the warm start dba
 __global__ void __launch_bounds__(EW_THREADS, 3) bk_corr(const BInst* __restrict__ I) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
     ipm_corr_kernel_body<double, double, double>(q.n, q.lam, q.s1, q.s2, q.z1, q.z2, (const double*)q.dba,
@@ -184,6 +198,7 @@ __global__ void __launch_bounds__(EW_THREADS, 3) bk_corr(const BInst* __restrict
 }
 
 __global__ void __launch_bounds__(EW_THREADS) bk_beta_step(const BInst* __restrict__ I) {
+    pdl_enter();
     const BInst& q = I[blockIdx.y];
     if (!q.running()) return;
     ipm_beta_step_kernel_body<double>(q.n, q.beta, q.db, q.slots + SL_ALPHA);
@@ -196,6 +211,7 @@ constexpr int BATCH_THREADS = 256;
 
 template <bool INV, int IN, int OUT, class Epi>
 __global__ void __launch_bounds__(BATCH_THREADS) bk_strided(const BPass<Epi>* __restrict__ B) {
+    pdl_enter();
     const BPass<Epi>& e = B[blockIdx.y];
     const PassArgs<double>& a = e.a;
     strided_pass_kernel_body<double, INV, IN, OUT, double, Epi>(a, e.src, e.epi);
@@ -203,12 +219,14 @@ __global__ void __launch_bounds__(BATCH_THREADS) bk_strided(const BPass<Epi>* __
 
 template <bool MASK, class Epi>
 __global__ void __launch_bounds__(BATCH_THREADS) bk_row(const BPass<Epi>* __restrict__ B) {
+    pdl_enter();
     const PassArgs<double>& a = B[blockIdx.y].a;
     row_pass_kernel_body<double, IN_SPEC, OUT_SPEC, MASK>(a);
 }
 
 template <class Epi>
 __global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_first(const BPass<Epi>* __restrict__ B) {
+    pdl_enter();
     const BPass<Epi>& e = B[blockIdx.y];
     const PassArgs<double>& a = e.a;
     l1d_first_kernel_body<double, double>(a, e.src, e.twN, e.P);
@@ -216,6 +234,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_first(const BPass<Epi>* 
 
 template <bool MASK, class Epi>
 __global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_row(const BPass<Epi>* __restrict__ B) {
+    pdl_enter();
     const BPass<Epi>& e = B[blockIdx.y];
     const PassArgs<double>& a = e.a;
     l1d_row_kernel_body<double, IN_SPEC, OUT_SPEC, MASK>(a, e.twN, e.P, e.Q);
@@ -223,6 +242,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_row(const BPass<Epi>* __
 
 template <class Epi>
 __global__ void __launch_bounds__(BATCH_THREADS) bk_l1d_last(const BPass<Epi>* __restrict__ B) {
+    pdl_enter();
     const BPass<Epi>& e = B[blockIdx.y];
     const PassArgs<double>& a = e.a;
     l1d_last_kernel_body<double, Epi>(a, e.twN, e.P, e.Q, e.epi);
@@ -380,7 +400,7 @@ cudaError_t launch_bpass(K kernel, const BProduct<Epi>& P, int pass, cudaStream_
     const cudaError_t e = smem_optin(kernel, P.smem[pass]);
     if (e != cudaSuccess) return e;
     const int gx = batch_grid(kernel, BATCH_THREADS, P.smem[pass], P.count, P.gx[pass]);
-    kernel<<<dim3(gx, P.count), BATCH_THREADS, P.smem[pass], st>>>(P.tab[pass]);
+    launch_pdl(true, kernel, dim3(gx, P.count), BATCH_THREADS, P.smem[pass], st, P.tab[pass]);
     return cudaGetLastError();
 }
 
@@ -424,20 +444,20 @@ int batch_cg_loop(BatchState& B, int which) {
     for (int it = 0; it < BATCH_CG_CAP; ++it) {
         cudaError_t e = batch_product(B, B.pc);
         if (e != cudaSuccess) return fail(nullptr, CSIPM_ERR_CUDA, std::string("batch CG product: ") + cudaGetErrorString(e));
-        bk_cg_update<<<ge, EW_THREADS, 0, B.st>>>(B.inst, it, which);
-        bk_cg_pupdate<<<ge, EW_THREADS, 0, B.st>>>(B.inst, it);
+        launch_pdl(true, bk_cg_update, ge, EW_THREADS, 0, B.st, B.inst, it, which);
+        launch_pdl(true, bk_cg_pupdate, ge, EW_THREADS, 0, B.st, B.inst, it);
         B.launches += 2;
         if (++since >= chunk) {
             since = 0;
             if (chunk < 8) chunk *= 2;
-            bk_cg_active<<<1, 256, 0, B.st>>>(B.inst, B.count, B.flag);
+            launch_pdl(true, bk_cg_active, 1, 256, 0, B.st, B.inst, B.count, B.flag);
             B.launches += 1;
             const int active = read_flag(B);
             if (active < 0) return fail(nullptr, CSIPM_ERR_CUDA, std::string("batch CG loop: ") + cudaGetErrorString(cudaGetLastError()));
             if (active == 0) break;
         }
     }
-    bk_cg_post<<<(B.count + 127) / 128, 128, 0, B.st>>>(B.inst, B.count);
+    launch_pdl(true, bk_cg_post, (B.count + 127) / 128, 128, 0, B.st, B.inst, B.count);
     B.launches += 1;
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CSIPM_OK : fail(nullptr, CSIPM_ERR_CUDA, std::string("batch CG loop: ") + cudaGetErrorString(e));
@@ -567,13 +587,13 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
     const dim3 ge(B.gx_elem, count);
     const int g1 = (count + 127) / 128;
     // ---- initial point (as csipm_solve)
-    bk_init1<<<ge, EW_THREADS, 0, st>>>(B.inst);
+    launch_pdl(true, bk_init1, ge, EW_THREADS, 0, st, B.inst);
     {
         const cudaError_t e = batch_product(B, B.pq);
         if (e != cudaSuccess) return done(fail(nullptr, CSIPM_ERR_CUDA, std::string("batch product: ") + cudaGetErrorString(e)));
     }
-    bk_init2<<<ge, EW_THREADS, 0, st>>>(B.inst);
-    bk_ctl_start<<<g1, 128, 0, st>>>(B.inst, count);
+    launch_pdl(true, bk_init2, ge, EW_THREADS, 0, st, B.inst);
+    launch_pdl(true, bk_ctl_start, g1, 128, 0, st, B.inst, count);
     B.launches += 3;
     int status = CSIPM_OK;
     bool pending = false;
@@ -585,9 +605,9 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
                 break;
             }
         }
-        bk_resid<<<ge, EW_THREADS, 0, st>>>(B.inst, pending ? 1 : 0);
-        bk_stop<<<g1, 128, 0, st>>>(B.inst, count);
-        bk_running<<<1, 256, 0, st>>>(B.inst, count, B.flag);
+        launch_pdl(true, bk_resid, ge, EW_THREADS, 0, st, B.inst, pending ? 1 : 0);
+        launch_pdl(true, bk_stop, g1, 128, 0, st, B.inst, count);
+        launch_pdl(true, bk_running, 1, 256, 0, st, B.inst, count, B.flag);
         B.launches += 3;
         const int running = read_flag(B);
         if (running < 0) { status = fail(nullptr, CSIPM_ERR_CUDA, "batch synchronisation failed"); break; }
@@ -595,15 +615,15 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
         // predictor from zero (the residual pass started its CG)
         if ((status = batch_cg_loop(B, 0)) != CSIPM_OK) break;
         // centring target and corrector, warm-started at dba
-        bk_stepstats<<<ge, EW_THREADS, 0, st>>>(B.inst, 0);
-        bk_sigma<<<g1, 128, 0, st>>>(B.inst, count);
-        bk_corr<<<ge, EW_THREADS, 0, st>>>(B.inst);
+        launch_pdl(true, bk_stepstats, ge, EW_THREADS, 0, st, B.inst, 0);
+        launch_pdl(true, bk_sigma, g1, 128, 0, st, B.inst, count);
+        launch_pdl(true, bk_corr, ge, EW_THREADS, 0, st, B.inst);
         B.launches += 3;
         if ((status = batch_cg_loop(B, 1)) != CSIPM_OK) break;
         // step
-        bk_stepstats<<<ge, EW_THREADS, 0, st>>>(B.inst, 1);
-        bk_alpha<<<g1, 128, 0, st>>>(B.inst, count);
-        bk_beta_step<<<ge, EW_THREADS, 0, st>>>(B.inst);
+        launch_pdl(true, bk_stepstats, ge, EW_THREADS, 0, st, B.inst, 1);
+        launch_pdl(true, bk_alpha, g1, 128, 0, st, B.inst, count);
+        launch_pdl(true, bk_beta_step, ge, EW_THREADS, 0, st, B.inst);
         B.launches += 3;
         {
             const cudaError_t e = cudaGetLastError();

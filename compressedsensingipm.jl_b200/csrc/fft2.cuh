@@ -64,6 +64,7 @@ template <typename T, int A, int B, bool INV, int IN, int OUT, typename TS, clas
 __global__ void __launch_bounds__(fft2_tb<T, A * B>() * (A > B ? A : B),
                                   (fft2_min_ctas<T, IN, OUT, fft2_tb<T, A * B>() * (A > B ? A : B)>()))
 strided2_kernel(PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
+    pdl_enter();
     using C = cplx_t<T>;
     constexpr int L = A * B;
     constexpr int TB = fft2_tb<T, L>();
@@ -230,6 +231,7 @@ template <typename T, int A, int B> struct Row2Shape {
 template <typename T, int A, int B, int IN, int OUT, bool MASK>
 __global__ void __launch_bounds__(Row2Shape<T, A, B>::ROWS * Row2Shape<T, A, B>::NTL, Row2Shape<T, A, B>::MINB)
 row2_kernel(PassArgs<T> a) {
+    pdl_enter();
     using C = cplx_t<T>;
     using Sh = Row2Shape<T, A, B>;
     constexpr int M = Sh::M;
@@ -374,6 +376,7 @@ static __device__ int g_row2b_timeouts;
 template <typename T, int A, int B, bool MASK>
 __global__ void __launch_bounds__(Row2Shape<T, A, B>::ROWS * Row2Shape<T, A, B>::NTL, Row2Shape<T, A, B>::MINB_B)
 row2b_kernel(PassArgs<T> a, int ntiles) {
+    pdl_enter();
     using C = cplx_t<T>;
     using Sh = Row2Shape<T, A, B>;
     constexpr int M = Sh::M;

@@ -13,8 +13,7 @@ cudaError_t launch_strided2(int A, int B, const PassArgs<T>& a, const TS* src, c
     if (A == AA && B == BB) {                                                                              \
         constexpr int TB = fft2_tb<T, AA * BB>();                                                          \
         const dim3 grid((a.n_lines + TB - 1) / TB, a.n_outer, 1);                                          \
-        strided2_kernel<T, AA, BB, INV, IN, OUT, TS, Epi><<<grid, TB * (AA > BB ? AA : BB), 0, st>>>(a, src, epi); \
-        return cudaGetLastError();                                                                         \
+        return launch_pdl(pdl_pays(a.g.dim, a.g.N), strided2_kernel<T, AA, BB, INV, IN, OUT, TS, Epi>, grid, TB * (AA > BB ? AA : BB), 0, st, a, src, epi); \
     }
     CSIPM_FFT2_SPAIRS(CSIPM_S2)
 #undef CSIPM_S2
@@ -35,8 +34,7 @@ bool launch_row2b(const PassArgs<T>& a, cudaStream_t st, cudaError_t* err) {
     if (*err != cudaSuccess) return true;
     const int ntiles = a.nrows / Sh::ROWS;
     const int grid = persistent_grid((const void*)k, threads, dyn, ntiles);
-    k<<<grid, threads, dyn, st>>>(a, ntiles);
-    *err = cudaGetLastError();
+    *err = launch_pdl(pdl_pays(a.g.dim, a.g.N), k, grid, threads, dyn, st, a, ntiles);
     return true;
 }
 
@@ -50,8 +48,7 @@ cudaError_t launch_row2(int A, int B, const PassArgs<T>& a, cudaStream_t st) {
             if (launch_row2b<T, AA, BB, MASK>(a, st, &e)) return e;                                        \
         }                                                                                                  \
         const dim3 grid((a.nrows + Sh::ROWS - 1) / Sh::ROWS, 1, 1);                                        \
-        row2_kernel<T, AA, BB, IN, OUT, MASK><<<grid, Sh::ROWS * Sh::NTL, 0, st>>>(a);                     \
-        return cudaGetLastError();                                                                         \
+        return launch_pdl(pdl_pays(a.g.dim, a.g.N), row2_kernel<T, AA, BB, IN, OUT, MASK>, grid, Sh::ROWS * Sh::NTL, 0, st, a);      \
     }
     CSIPM_FFT2_RPAIRS(CSIPM_R2)
 #undef CSIPM_R2

@@ -13,6 +13,7 @@ namespace csipm_internal {
 
 // obj: [0] = r.r, [1] = sum(p) + sum(q)
 static __global__ void gz_obj_kernel(long long n, const double* __restrict__ x, RedWorkspace ws) {
+    pdl_enter();
     double acc[2] = {0.0, 0.0};
     CSIPM_GRID_LOOP(i, n) {
         const double r = x[2 * n + i];
@@ -23,6 +24,7 @@ static __global__ void gz_obj_kernel(long long n, const double* __restrict__ x, 
 }
 
 static __global__ void gz_grad_kernel(long long n, const double* __restrict__ x, double lam, double* __restrict__ g) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         g[i] = lam;
         g[n + i] = lam;
@@ -32,12 +34,14 @@ static __global__ void gz_grad_kernel(long long n, const double* __restrict__ x,
 
 // d = a[0:n) - a[n:2n)   (sign = +1), or a[n:2n) - a[0:n) (sign = -1)
 static __global__ void gz_diff_kernel(long long n, const double* __restrict__ a, double sign, double* __restrict__ d) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) d[i] = sign * (a[i] - a[n + i]);
 }
 
 // c = z0 - Ux - r
 static __global__ void gz_cons_kernel(long long n, const double* __restrict__ z0, const double* __restrict__ ux,
                                       const double* __restrict__ x, double* __restrict__ c) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) c[i] = z0[i] - ux[i] - x[2 * n + i];
 }
 
@@ -45,6 +49,7 @@ static __global__ void gz_cons_kernel(long long n, const double* __restrict__ z0
 static __global__ void gz_build_kernel(long long n, const double* __restrict__ pr_diag, double* __restrict__ Dp,
                                        double* __restrict__ Dq, double* __restrict__ P11, double* __restrict__ P12,
                                        double* __restrict__ P22) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double rp = pr_diag[i], rq = pr_diag[n + i];
         const double ip = 1.0 / (1.0 + rp);
@@ -100,6 +105,7 @@ struct EpiGzCG {
 // kkt mul! body, first part: t = A'x_y arrives; y_p, y_q, y_r updated and d = x_q - x_p
 static __global__ void gz_kktmul1_kernel(long long n, const double* __restrict__ x, const double* __restrict__ t,
                                          double* __restrict__ y, double alpha, double beta, double* __restrict__ d) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double tv = t[i];
         y[i] = -alpha * tv + beta * y[i];
@@ -112,12 +118,14 @@ static __global__ void gz_kktmul1_kernel(long long n, const double* __restrict__
 // second part: y_y = alpha (A d - x_r) + beta y_y
 static __global__ void gz_kktmul2_kernel(long long n, const double* __restrict__ x, const double* __restrict__ ad,
                                          double* __restrict__ y, double alpha, double beta) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) y[3 * n + i] = alpha * (ad[i] - x[2 * n + i]) + beta * y[3 * n + i];
 }
 
 // jtprod!: y = [-t; t; -x]
 static __global__ void gz_jtprod_kernel(long long n, const double* __restrict__ x, const double* __restrict__ t,
                                         double* __restrict__ y) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         y[i] = -t[i];
         y[n + i] = t[i];
@@ -127,12 +135,14 @@ static __global__ void gz_jtprod_kernel(long long n, const double* __restrict__ 
 
 // solve_kkt!: buffer3 = w_r + w_y
 static __global__ void gz_sum_kernel(long long n, const double* __restrict__ w, double* __restrict__ s) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) s[i] = w[2 * n + i] + w[3 * n + i];
 }
 
 // rhs = [w_p - t; w_q + t]
 static __global__ void gz_rhs_kernel(long long n, const double* __restrict__ w, const double* __restrict__ t,
                                      double* __restrict__ b) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         b[i] = w[i] - t[i];
         b[n + i] = w[n + i] + t[i];
@@ -142,6 +152,7 @@ static __global__ void gz_rhs_kernel(long long n, const double* __restrict__ w, 
 // w_x = x (and d = x_p - x_q for U dx)
 static __global__ void gz_setx_kernel(long long n, const double* __restrict__ x, double* __restrict__ w,
                                       double* __restrict__ d) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double a = x[i], b = x[n + i];
         w[i] = a;
@@ -152,6 +163,7 @@ static __global__ void gz_setx_kernel(long long n, const double* __restrict__ x,
 
 // dr = -w_y - U dx ; dy = dr - w_r(old)
 static __global__ void gz_back_kernel(long long n, const double* __restrict__ udx, double* __restrict__ w) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double wr = w[2 * n + i], wy = w[3 * n + i];
         const double dr = -wy - udx[i];

@@ -72,7 +72,7 @@ int ew_grid(const void* kernel, long long n);
 
 template <typename... P, typename... A>
 inline void ew_launch(void (*kernel)(P...), long long n, cudaStream_t st, A&&... args) {
-    kernel<<<ew_grid((const void*)kernel, n), EW_THREADS, 0, st>>>(std::forward<A>(args)...);
+    launch_pdl(pdl_pays(0, n), kernel, ew_grid((const void*)kernel, n), EW_THREADS, 0, st, std::forward<A>(args)...);
 }
 
 inline bool valid_dims(int dim, const int* size, std::string* err, int* status) {

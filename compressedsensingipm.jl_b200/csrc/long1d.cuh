@@ -83,6 +83,7 @@ __device__ __forceinline__ void l1d_first_kernel_body(const PassArgs<T>& a, cons
 template <typename T, typename TS>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
 l1d_first_kernel(const __grid_constant__ PassArgs<T> a, const TS* __restrict__ src, const cplx_t<T>* __restrict__ twN, int P) {
+    pdl_enter();
     l1d_first_kernel_body<T, TS>(a, src, twN, P);
 }
 
@@ -186,6 +187,7 @@ __device__ __forceinline__ void l1d_row_kernel_body(const PassArgs<T>& a, const 
 template <typename T, int IN, int OUT, bool MASK>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
 l1d_row_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P, int Q) {
+    pdl_enter();
     l1d_row_kernel_body<T, IN, OUT, MASK>(a, twN, P, Q);
 }
 
@@ -253,6 +255,7 @@ __device__ __forceinline__ void l1d_last_kernel_body(const PassArgs<T>& a, const
 template <typename T, class Epi>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
 l1d_last_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN, int P, int Q, Epi epi) {
+    pdl_enter();
     l1d_last_kernel_body<T, Epi>(a, twN, P, Q, epi);
 }
 
@@ -280,7 +283,7 @@ cudaError_t l1d_first(const FftOperator<T>& op, const TS* src, const int* skip, 
     const PassCfg& c = op.f_cfg;
     const cudaError_t e = smem_optin(k, c.smem);
     if (e != cudaSuccess) return e;
-    k<<<c.tiles, c.threads, c.smem, st>>>(l1d_args(op, 0, 1.0, skip), src, op.tw1, op.l1P);
+    launch_pdl(pdl_pays(1, op.g.N), k, c.tiles, c.threads, c.smem, st, l1d_args(op, 0, 1.0, skip), src, op.tw1, op.l1P);
     return cudaGetLastError();
 }
 
@@ -294,7 +297,7 @@ cudaError_t l1d_row(const FftOperator<T>& op, double scale, const T* real_in, T*
     PassArgs<T> a = l1d_args(op, 1, scale, skip);
     a.real_in = real_in;
     a.real_out = real_out;
-    k<<<c.tiles, c.threads, c.smem, st>>>(a, op.tw1, op.l1P, op.l1Q);
+    launch_pdl(pdl_pays(1, op.g.N), k, c.tiles, c.threads, c.smem, st, a, op.tw1, op.l1P, op.l1Q);
     return cudaGetLastError();
 }
 
@@ -304,7 +307,7 @@ cudaError_t l1d_last(const FftOperator<T>& op, const Epi& epi, const int* skip, 
     const PassCfg& c = op.q_cfg;
     const cudaError_t e = smem_optin(k, c.smem);
     if (e != cudaSuccess) return e;
-    k<<<c.tiles, c.threads, c.smem, st>>>(l1d_args(op, 2, 1.0, skip), op.tw1, op.l1P, op.l1Q, epi);
+    launch_pdl(pdl_pays(1, op.g.N), k, c.tiles, c.threads, c.smem, st, l1d_args(op, 2, 1.0, skip), op.tw1, op.l1P, op.l1Q, epi);
     return cudaGetLastError();
 }
 

@@ -68,6 +68,47 @@ struct PassArgs {
     const int* skip;         // when non-null and *skip != 0 the pass returns at once (converged CG)
 };
 
+// ------------------------------------------------------------- dependent launches
+// A solve is a chain of some hundred kernels of a few microseconds, each
+// reading what the one before wrote.  They are launched with programmatic
+// stream serialisation: a kernel's blocks may be placed while the one before
+// still drains, and wait in pdl_enter (its first statement, before any memory
+// is read) until that one has completed and its writes are visible; then the
+// next kernel may be placed in turn.  Every kernel of a chain waits, so the
+// order of the stream holds throughout.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Whether a kernel on N samples is launched that way (dim 0: an element
+// kernel).  It hides 1-3 us a launch, and costs when early blocks sit beside a
+// pass that fills the shared memory or the HBM queues.  A'A in FP64, plain ->
+// early (B200, us): 1D 4096 21.6 -> 18.2, 131072 28.7 -> 25.4, 259200 32.2 ->
+// 30.0, 524288 41.0 -> 53.1; 256^2 22.6 -> 17.7, 1024^2 46.6 -> 41.4; 64^3 30.8
+// -> 22.8, 160^3 115 -> 105, 256^3 384 -> 398.
+inline bool pdl_pays(int dim, long long N) { return N <= (dim == 1 ? 1LL << 18 : 1LL << 22); }
+
+// Not inside a capture: a graph's kernels already follow one another closely,
+// and programmatic edges made its replays slower (1024^2 solve 3.47 -> 3.88 ms,
+// 320^3 mixed 42.0 -> 46.4 ms).
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (early) cudaStreamIsCapturing(st, &cap);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = early && cap == cudaStreamCaptureStatusNone;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+
 // ------------------------------------------------------------- epilogues
 // Two-phase epilogues: pre(l) loads what put(l, v, pre) needs, so a scatter
 // loop can issue the loads of several elements before it consumes them.

@@ -89,6 +89,7 @@ template <typename T> constexpr int pass_min_ctas() { return sizeof(T) == 8 ? 1 
 template <typename T, bool INV, int IN, int OUT, typename TS, class Epi>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
 strided_pass_kernel(const __grid_constant__ PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
+    pdl_enter();
     strided_pass_kernel_body<T, INV, IN, OUT, TS, Epi>(a, src, epi);
 }
 
@@ -242,6 +243,7 @@ __device__ __forceinline__ void row_pass_kernel_body(const PassArgs<T>& a) {
 }
 template <typename T, int IN, int OUT, bool MASK>
 __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>()) row_pass_kernel(const __grid_constant__ PassArgs<T> a) {
+    pdl_enter();
     row_pass_kernel_body<T, IN, OUT, MASK>(a);
 }
 
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>()) row_pass_ker
 // with N1 above about 12000): one row a CTA, register-staged stages.
 template <typename T, int IN, int OUT, bool MASK>
 __global__ void __launch_bounds__(1024) row_pass_ip_kernel(PassArgs<T> a) {
+    pdl_enter();
     using C = cplx_t<T>;
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -729,7 +732,7 @@ cudaError_t launch_strided(const PassCfg& c, const PassArgs<T>& a, const TS* src
     auto k = strided_pass_kernel<T, INV, IN, OUT, TS, Epi>;
     const cudaError_t e = smem_optin(k, c.smem);
     if (e != cudaSuccess) return e;
-    k<<<pass_grid((const void*)k, c), c.threads, c.smem, st>>>(a, src, epi);
+    launch_pdl(pdl_pays(a.g.dim, a.g.N), k, pass_grid((const void*)k, c), c.threads, c.smem, st, a, src, epi);
     return cudaGetLastError();
 }
 
@@ -739,12 +742,12 @@ cudaError_t launch_row(const PassCfg& c, const PassArgs<T>& a, cudaStream_t st) 
         auto k = row_pass_kernel<T, IN, OUT, MASK>;
         const cudaError_t e = smem_optin(k, c.smem);
         if (e != cudaSuccess) return e;
-        k<<<pass_grid((const void*)k, c), c.threads, c.smem, st>>>(a);
+        launch_pdl(pdl_pays(a.g.dim, a.g.N), k, pass_grid((const void*)k, c), c.threads, c.smem, st, a);
     } else {
         auto k = row_pass_ip_kernel<T, IN, OUT, MASK>;
         const cudaError_t e = smem_optin(k, c.smem);
         if (e != cudaSuccess) return e;
-        k<<<c.grid, c.threads, c.smem, st>>>(a);
+        launch_pdl(pdl_pays(a.g.dim, a.g.N), k, c.grid, c.threads, c.smem, st, a);
     }
     return cudaGetLastError();
 }

@@ -98,6 +98,7 @@ template <typename TV>
 static __global__ void cg_init_kernel(long long n, const double* __restrict__ rhs, const TV* __restrict__ q, int has_x0,
                                const TV* __restrict__ Minv, TV* __restrict__ r, TV* __restrict__ p,
                                RedWorkspace ws, CgScalars* sc, double atol, DevScalar rtol_s) {
+    pdl_enter();
     cg_init_kernel_body<TV>(n, rhs, q, has_x0, Minv, r, p, ws, sc, atol, rtol_s);
 }
 
@@ -165,6 +166,7 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
 template <typename TV, typename TX, bool START>
 static __global__ void cg_update_kernel(long long n, int it, TX* __restrict__ x, const TX* __restrict__ x0, TV* __restrict__ r, const TV* __restrict__ p,
                                  const TV* __restrict__ q, const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
+    pdl_enter();
     cg_update_kernel_body<TV, TX, START>(n, it, x, x0, r, p, q, Minv, ws, sc);
 }
 
@@ -188,12 +190,14 @@ __device__ __forceinline__ void cg_pupdate_kernel_body(long long n, int it, cons
 template <typename TV>
 static __global__ void cg_pupdate_kernel(long long n, int it, const TV* __restrict__ r, const TV* __restrict__ Minv, TV* __restrict__ p,
                                   const CgScalars* sc) {
+    pdl_enter();
     cg_pupdate_kernel_body<TV>(n, it, r, Minv, p, sc);
 }
 
 // Mixed precision: r = rhs - q in FP64 with r.(Minv r) (the refinement residual)
 static __global__ void resid64_kernel(long long n, const double* __restrict__ rhs, const double* __restrict__ q,
                                       const double* __restrict__ Minv, double* __restrict__ r, RedWorkspace ws) {
+    pdl_enter();
     double acc[1] = {0.0};
     CSIPM_GRID_LOOP(i, n) {
         const double rv = rhs[i] - q[i];
@@ -205,6 +209,7 @@ static __global__ void resid64_kernel(long long n, const double* __restrict__ rh
 
 // x += d (FP32 correction into the FP64 iterate)
 static __global__ void add_f32_kernel(long long n, const float* __restrict__ d, double* __restrict__ x) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) x[i] += (double)d[i];
 }
 
@@ -229,6 +234,7 @@ __device__ __forceinline__ void ipm_init1_kernel_body(long long n, const double*
 }
 static __global__ void ipm_init1_kernel(long long n, const double* __restrict__ b, double lam, double* __restrict__ beta,
                                  RedWorkspace ws) {
+    pdl_enter();
     ipm_init1_kernel_body(n, b, lam, beta, ws);
 }
 
@@ -260,6 +266,7 @@ static __global__ void ipm_init2_kernel(long long n, const double* __restrict__ 
                                  const double* __restrict__ beta, const double* __restrict__ mx,
                                  double* __restrict__ s1, double* __restrict__ s2, double* __restrict__ z1,
                                  double* __restrict__ z2) {
+    pdl_enter();
     ipm_init2_kernel_body(n, b, Qb, lam, beta, mx, s1, s2, z1, z2);
 }
 
@@ -378,6 +385,7 @@ static __global__ void ipm_rhs_kernel(long long n, double lam, const double* __r
                                const double* __restrict__ s1v, const double* __restrict__ s2v,
                                const double* __restrict__ z1, const double* __restrict__ z2,
                                const TD* __restrict__ dba, const double* __restrict__ sigmu_p, double* __restrict__ rhs) {
+    pdl_enter();
     ipm_rhs_kernel_body<TD>(n, lam, b, Qb, s1v, s2v, z1, z2, dba, sigmu_p, rhs);
 }
 
@@ -426,6 +434,7 @@ ipm_corr_kernel(long long n, double lam, const double* __restrict__ s1v, const d
                 const double* __restrict__ z1, const double* __restrict__ z2, const TD* __restrict__ dba,
                 const double* __restrict__ sigmu_p, const TR* rp, TC* cr, TC* __restrict__ cp,
                 const TC* __restrict__ cm, CgScalars* csc, RedWorkspace ws, DevScalar crtol) {
+    pdl_enter();
     ipm_corr_kernel_body<TR, TD, TC>(n, lam, s1v, s2v, z1, z2, dba, sigmu_p, rp, cr, cp, cm, csc, ws, crtol);
 }
 
@@ -498,13 +507,15 @@ __device__ __forceinline__ void ipm_stop_kernel_body(const double* __restrict__ 
 }
 static __global__ void ipm_stop_kernel(const double* __restrict__ R, IpmCtl* __restrict__ c, int in_graph,
                                        cudaGraphConditionalHandle hnd) {
+    pdl_enter();
     ipm_stop_kernel_body(R, c, in_graph, hnd);
 }
 
 // Graph replays: opens a CG loop (a conditional while node), also one whose
 // start already met the tolerance: its passes return at once and the update
 // copies the start into the iterate.  One thread.
-static __global__ void cg_arm_kernel(cudaGraphConditionalHandle hnd) { cudaGraphSetConditional(hnd, 1u); }
+static __global__ void cg_arm_kernel(cudaGraphConditionalHandle hnd) {
+    pdl_enter(); cudaGraphSetConditional(hnd, 1u); }
 
 // Graph replays: after a CG loop, count its iterations and let the rest of
 // the iteration run only if it converged (a breakdown, or the loop's cap
@@ -512,6 +523,7 @@ static __global__ void cg_arm_kernel(cudaGraphConditionalHandle hnd) { cudaGraph
 static __global__ void ipm_cg_check_kernel(const CgScalars* __restrict__ sc, IpmCtl* __restrict__ c, int which,
                                            int cap_is_limit, cudaGraphConditionalHandle if_hnd,
                                            cudaGraphConditionalHandle loop_hnd) {
+    pdl_enter();
     const bool ok = !sc->breakdown && (sc->done || cap_is_limit);
     c->cg_iter += sc->iters;
     if (!ok) {
@@ -584,6 +596,7 @@ static __global__ void __launch_bounds__(EW_THREADS, 3)
 ipm_stepstats_kernel(long long n, double lam, const double* __restrict__ s1v, const double* __restrict__ s2v,
                      const double* __restrict__ z1, const double* __restrict__ z2, const TD* __restrict__ dba,
                      const double* __restrict__ sigmu_p, const TD* __restrict__ db, RedWorkspace ws) {
+    pdl_enter();
     ipm_stepstats_kernel_body<TD>(n, lam, s1v, s2v, z1, z2, dba, sigmu_p, db, ws);
 }
 
@@ -600,6 +613,7 @@ __device__ __forceinline__ void ipm_sigma_kernel_body(const double* __restrict__
 }
 static __global__ void ipm_sigma_kernel(const double* __restrict__ q, const IpmCtl* __restrict__ c,
                                         double* __restrict__ sigmu) {
+    pdl_enter();
     ipm_sigma_kernel_body(q, c, sigmu);
 }
 
@@ -615,6 +629,7 @@ __device__ __forceinline__ void ipm_alpha_kernel_body(const double* __restrict__
 }
 static __global__ void ipm_alpha_kernel(const double* __restrict__ q, const IpmCtl* __restrict__ c,
                                         double* __restrict__ alpha) {
+    pdl_enter();
     ipm_alpha_kernel_body(q, c, alpha);
 }
 
@@ -622,6 +637,7 @@ static __global__ void ipm_alpha_kernel(const double* __restrict__ q, const IpmC
 // b = A'z0 + rho z - y
 static __global__ void admm_rhs_kernel(long long n, const double* __restrict__ bv, const double* __restrict__ z,
                                        const double* __restrict__ y, double rho, double* __restrict__ b) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) b[i] = bv[i] + rho * z[i] - y[i];
 }
 
@@ -632,6 +648,7 @@ static __global__ void admm_update_kernel(long long n, const double* __restrict_
                                           const double* __restrict__ x0, double* __restrict__ z,
                                           double* __restrict__ y, double rho, double lam, double* __restrict__ b,
                                           RedWorkspace ws) {
+    pdl_enter();
     double acc[3] = {0.0, 0.0, 0.0};
     const double thre = lam / rho;
     CSIPM_GRID_LOOP(i, n) {
@@ -740,6 +757,7 @@ ipm_resdiag_kernel(long long n, const double* __restrict__ b, const double* __re
                    double* __restrict__ Minv, TV* __restrict__ Db_lo, TV* __restrict__ Minv_lo, int precond,
                    RedWorkspace ws, TC* __restrict__ cr, TC* __restrict__ cp,
                    CgScalars* csc, DevScalar crtol) {
+    pdl_enter();
     ipm_resdiag_kernel_body<TV, TD, TC>(n, b, Qb, lam, beta, s1v, s2v, z1, z2, dba, db, sigmu_p, alpha_p, Db, Minv, Db_lo, Minv_lo, precond, ws, cr, cp, csc, crtol);
 }
 
@@ -749,6 +767,7 @@ ipm_resdiag_kernel(long long n, const double* __restrict__ b, const double* __re
 static __global__ void ipm_diag64_kernel(long long n, const double* __restrict__ s1, const double* __restrict__ s2,
                                          const double* __restrict__ z1, const double* __restrict__ z2,
                                          double* __restrict__ Db, double* __restrict__ Minv, int precond) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const ElemDiag g = elem_diag(s1[i], s2[i], z1[i], z2[i], precond);   // as in ipm_resdiag_kernel
         Db[i] = g.db;
@@ -767,6 +786,7 @@ __device__ __forceinline__ void ipm_beta_step_kernel_body(long long n, double* _
 template <typename TD>
 static __global__ void ipm_beta_step_kernel(long long n, double* __restrict__ beta, const TD* __restrict__ db,
                                             const double* __restrict__ alpha_p) {
+    pdl_enter();
     ipm_beta_step_kernel_body<TD>(n, beta, db, alpha_p);
 }
 
@@ -777,27 +797,32 @@ __device__ __forceinline__ void half_sum_kernel_body(long long n, const double* 
 }
 static __global__ void half_sum_kernel(long long n, const double* __restrict__ s1, const double* __restrict__ s2,
                                        double* __restrict__ c) {
+    pdl_enter();
     half_sum_kernel_body(n, s1, s2, c);
 }
 
 // ------------------------------------------------------------------ utilities
 template <typename TA, typename TB>
 static __global__ void convert_kernel(long long n, const TA* __restrict__ a, TB* __restrict__ b) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) b[i] = (TB)a[i];
 }
 
 static __global__ void axpy_kernel(long long n, double alpha, const double* __restrict__ x, double* __restrict__ y) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) y[i] += alpha * x[i];
 }
 
 // y = x - y  (residual r = rhs - Kx in place on y)
 static __global__ void sub_from_kernel(long long n, const double* __restrict__ x, double* __restrict__ y) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) y[i] = x[i] - y[i];
 }
 
 // dot products on the device
 static __global__ void dot2_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b,
                             const double* __restrict__ c2, const double* __restrict__ d2, RedWorkspace ws) {
+    pdl_enter();
     double acc[2] = {0.0, 0.0};
     CSIPM_GRID_LOOP(i, n) {
         acc[0] += a[i] * b[i];
@@ -811,6 +836,7 @@ static __global__ void dot2_kernel(long long n, const double* __restrict__ a, co
 // before: 720 x 462, 17 -> 7 us)
 static __global__ void obj_kernel(long long n, const double* __restrict__ x, const double* __restrict__ Qb,
                                   const double* __restrict__ b, RedWorkspace ws) {
+    pdl_enter();
     double acc[3] = {0.0, 0.0, 0.0};
     CSIPM_GRID_LOOP(i, n) {
         const double be = x[i];
@@ -832,11 +858,13 @@ struct EpiGrad {
 };
 
 static __global__ void fill_kernel(long long n, double v, double* __restrict__ y) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) y[i] = v;
 }
 
 // cons!: c = [-beta - c ; beta - c]   (src/fft_model.jl:91-101)
 static __global__ void cons_kernel(long long n, const double* __restrict__ x, double* __restrict__ out) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double be = x[i], ce = x[n + i];
         out[i] = -be - ce;
@@ -858,6 +886,7 @@ struct EpiScale {
 static __global__ void kkt_build_kernel(long long n, const double* __restrict__ pr_diag, double* __restrict__ L1,
                                  double* __restrict__ L2, double* __restrict__ P11, double* __restrict__ P12,
                                  double* __restrict__ P22) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i];
         const double l1 = S1 + S2, l2 = S1 - S2;
@@ -896,6 +925,7 @@ struct EpiCondensed {
 static __global__ void precond_mul_kernel(long long n, double* __restrict__ y, const double* __restrict__ x,
                                    const double* __restrict__ P11, const double* __restrict__ P12,
                                    const double* __restrict__ P22, double alpha, double beta) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double xb = x[i], xz = x[n + i];
         y[i] = beta * y[i] + alpha * (P11[i] * xb + P12[i] * xz);
@@ -934,6 +964,7 @@ struct EpiKKT {
 
 // jtprod!  (src/fft_kkt.jl:253-275)
 static __global__ void jtprod_kernel(long long n, double* __restrict__ y, const double* __restrict__ x) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double y1 = x[i], y2 = x[n + i];
         y[i] = -y1 + y2;
@@ -946,6 +977,7 @@ static __global__ void jtprod_kernel(long long n, double* __restrict__ y, const 
 // solve_kkt! right-hand side (src/fft_kkt.jl:334-335): b = [w1 - w3 + w4 - S1 w5 + S2 w6 ; w2 - w3 - w4 - S1 w5 - S2 w6]
 static __global__ void kkt_rhs_kernel(long long n, const double* __restrict__ w, const double* __restrict__ pr_diag,
                                double* __restrict__ b) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i];
         const double w1 = w[i], w2 = w[n + i], w3 = w[2 * n + i], w4 = w[3 * n + i], w5 = w[4 * n + i], w6 = w[5 * n + i];
@@ -957,6 +989,7 @@ static __global__ void kkt_rhs_kernel(long long n, const double* __restrict__ w,
 // solve_kkt! back-substitution (src/fft_kkt.jl:345-350)
 static __global__ void kkt_back_kernel(long long n, double* __restrict__ w, const double* __restrict__ x,
                                 const double* __restrict__ pr_diag) {
+    pdl_enter();
     CSIPM_GRID_LOOP(i, n) {
         const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i];
         const double w1 = x[i], w2 = x[n + i];
@@ -1021,6 +1054,7 @@ static __global__ void __launch_bounds__(EW_THREADS)
 kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const double* __restrict__ pr_diag,
                       double* __restrict__ r, double* __restrict__ p, double* __restrict__ D,
                       double* __restrict__ M, RedWorkspace ws, CgScalars* sc, double atol, double rtol) {
+    pdl_enter();
     const long long n = g.N;
     double acc[2] = {0.0, 0.0};
     for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
@@ -1048,6 +1082,7 @@ kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const do
 static __global__ void __launch_bounds__(EW_THREADS)
 kkt_schur_back_kernel(Geom g, int sorder, double* __restrict__ w, const double* __restrict__ x,
                       const double* __restrict__ pr_diag, const CgScalars* __restrict__ sc) {
+    pdl_enter();
     const long long n = g.N;
     const double left = 1.0 - sc->rho;
     for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
@@ -1083,6 +1118,7 @@ __device__ __forceinline__ void pblock(const double* P11, const double* P12, con
 static __global__ void kcg_init_kernel(long long n, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r,
                                 double* __restrict__ p, const double* __restrict__ P11, const double* __restrict__ P12,
                                 const double* __restrict__ P22, RedWorkspace ws, CgScalars* sc, double atol, double rtol) {
+    pdl_enter();
     double acc[1] = {0.0};
     CSIPM_GRID_LOOP(i, n) {
         const double rb = b[i], rzv = b[n + i];
@@ -1134,6 +1170,7 @@ static __global__ void kcg_update_kernel(long long n, int it, double* __restrict
                                   const double* __restrict__ p, const double* __restrict__ q,
                                   const double* __restrict__ P11, const double* __restrict__ P12,
                                   const double* __restrict__ P22, RedWorkspace ws, CgScalars* sc) {
+    pdl_enter();
     if (sc->done) return;
     const double pq = sc->pq;
     const double alpha = sc->rz[it & 1] / pq;
@@ -1161,6 +1198,7 @@ static __global__ void kcg_update_kernel(long long n, int it, double* __restrict
 static __global__ void kcg_pupdate_kernel(long long n, int it, const double* __restrict__ r, double* __restrict__ p,
                                    const double* __restrict__ P11, const double* __restrict__ P12,
                                    const double* __restrict__ P22, const CgScalars* sc) {
+    pdl_enter();
     if (sc->done) return;
     const double b = sc->rz[(it + 1) & 1] / sc->rz[it & 1];
     CSIPM_GRID_LOOP(i, n) {
