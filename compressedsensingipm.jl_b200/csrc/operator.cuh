@@ -46,7 +46,7 @@ struct PassArgs {
     FftPlanDev pl;
     const cplx_t<T>* tw;     // Ltab-th roots of unity (global memory)
     int Ltab;
-    FftStage fwd[FFT_MAX_STAGES], inv[FFT_MAX_STAGES];   // the plan's stages, in order and (rows) reversed
+    FftStage fwd[PASS_STAGES], inv[PASS_STAGES];   // the plan's stages, in order and (rows) reversed
     cplx_t<T>* spec;
     // strided passes
     int n_lines;             // number of dim-1 positions (M1+1)

@@ -354,7 +354,7 @@ struct PassCfg {
     int pp = 1;          // 1: run-time-plan pass (TileLay fields below); 0: in-place row kernel
     TileLay lay{0, 1};
     int span = 0, two = 0, primes = 0;
-    FftStage fwd[FFT_MAX_STAGES], inv[FFT_MAX_STAGES];
+    FftStage fwd[PASS_STAGES], inv[PASS_STAGES];
     int tiles = 0;       // number of tiles of the pass
     dim3 grid;           // one CTA per tile (persistent grids are capped at launch)
 };
@@ -370,11 +370,17 @@ inline void lay_pass(const FftPlanDev& pl, int Ltab, int lines, int n, PassKind 
                      PassCfg* c) {
     c->tb = lines;
     c->pp = 1;
+    if (pl.L * csize > PASS_SMEM) {   // longer than a tile: PASS_STAGES and 16 bits may not hold it
+        c->smem = ~(size_t)0;
+        return;
+    }
     TileLay l;
     l.lg = 0;
     while ((1 << l.lg) < lines) ++l.lg;
-    // rows are read and written along the row, so their pitch is odd
-    l.tbp = kind != PASS_LINES && lines > 1 ? lines + 1 : lines;
+    // rows are read and written along the row, so their pitch is odd; 1D pairs
+    // are read like strided lines (padded by one they met 2-way bank conflicts:
+    // last pass of 777600, 27.5 -> 26.0 us)
+    l.tbp = kind == PASS_ROWS && lines > 1 ? lines + 1 : lines;
     c->lay = l;
     c->span = (kind == PASS_ROWS ? pl.L + 1 : pl.L) * l.tbp;   // a staged row has M+1 values
     c->tiles = (n + lines - 1) / lines;
@@ -690,8 +696,8 @@ public:
         a->span = c.span;
         a->two = c.two;
         a->primes = c.primes;
-        std::copy(c.fwd, c.fwd + FFT_MAX_STAGES, a->fwd);
-        std::copy(c.inv, c.inv + FFT_MAX_STAGES, a->inv);
+        std::copy(c.fwd, c.fwd + PASS_STAGES, a->fwd);
+        std::copy(c.inv, c.inv + PASS_STAGES, a->inv);
     }
     PassArgs<T> row_args(double scale, const T* real_in, T* real_out) const {
         PassArgs<T> a{};

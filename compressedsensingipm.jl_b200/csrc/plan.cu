@@ -65,13 +65,13 @@ void fill_stages(const FftPlanDev& pl, int Ltab, bool rev, FftStage* out) {
     for (int s = 0; s < pl.nst; ++s) {
         const int q = rev ? pl.nst - 1 - s : s;
         FftStage& o = out[s];
-        o.R = pl.rad[q];
-        o.Ns = Ns;
-        o.m = pl.L / o.R;
+        o.R = (unsigned short)pl.rad[q];
+        o.Ns = (unsigned short)Ns;
+        o.m = (unsigned short)(pl.L / o.R);
         o.step = Ltab / (Ns * o.R);
         o.mag_ns = 0xffffffffu / (unsigned)Ns + 1u;
         o.mag_m = 0xffffffffu / (unsigned)o.m + 1u;
-        o.cs = cs[q];
+        o.cs = (unsigned short)cs[q];
         Ns *= o.R;
     }
 }

@@ -12,6 +12,9 @@
 namespace csipm {
 
 constexpr int FFT_MAX_STAGES = 12;
+// Stages of a run-time-plan pass: lengths up to 46874 have at most 6, and a
+// line of 25601 values does not fit a tile (lay_pass).
+constexpr int PASS_STAGES = 6;
 
 struct FftPlanDev {
     int L;                       // transform length
@@ -25,12 +28,16 @@ struct FftPlanDev {
 // more in instruction fetches than the third stage of a 256-point line.
 CSIPM_HD constexpr bool reg_radix(int r) { return r <= 10; }
 
-// One stage of a plan as the kernels read it (fill_stages, plan.cu).
+// One stage of a plan as the kernels read it (fill_stages, plan.cu).  It
+// travels in every pass's arguments, which each block reads cold from the
+// constant bank before anything else: 12 + 12 stages of 28 bytes -> 6 + 6 of 20
+// took an A'A on 4096 samples from 18.3 to 16.7 us, on 777600 from 61.7 to 57.3
+// (B200, with the unpadded pair tiles of lay_pass).
 struct FftStage {
-    int R, Ns, m;           // radix, product of the earlier radices, L/R
-    int step;               // Ltab/(Ns*R): table stride of the stage's twiddles
-    unsigned mag_ns, mag_m; // reciprocals of Ns and m (quot)
-    int cs;                 // prime stages: where its cosines and sines start (prime_tables)
+    unsigned short R, Ns, m;    // radix, product of the earlier radices, L/R (quot: below 2^16)
+    unsigned short cs;          // prime stages: where its cosines and sines start (prime_tables)
+    int step;                   // Ltab/(Ns*R): table stride of the stage's twiddles
+    unsigned mag_ns, mag_m;     // reciprocals of Ns and m (quot)
 };
 
 // Shared-memory place of element (x, b) of a tile: x*tbp + b, b fastest, so a

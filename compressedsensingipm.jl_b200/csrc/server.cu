@@ -90,7 +90,7 @@ size_t footprint_bytes(int dim, const int* size, int precision, int64_t n_missin
     b += 16 * Nh;                                 // FP64 spectrum
     if (precision == CSIPM_MIXED) b += 8 * 4 * N + 8 * Nh;   // FP32 CG vectors and directions + FP32 spectrum
     if (n_missing > 0) b += (size_t)((n1 + 31) / 32) * 4 * (size_t)(n2 * n3) * (precision == CSIPM_MIXED ? 2 : 1);
-    b += 2 * 16 * (size_t)(n2 * n3);              // plane map
+    b += 2 * 16 * (size_t)(n2 * n3);              // headroom (twiddle tables of long axes)
     b += 8 * 8 * 65536 + (1 << 20);               // reduction partials, slots, twiddles (upper bound)
     b += 2 * 8 * N;                               // the server's z0 / beta staging
     return b;
