@@ -68,7 +68,9 @@ namespace csipm_internal {
 // One thread per solver-order pair (NI of them) and per tail entry; every
 // reference index is read or written exactly once (the packing is a bijection
 // between beta entries and the sources of the half spectrum).
-template <bool TO_SOL>
+// SIGNED: the vector changes sign with beta; bounds of |beta| such as c do
+// not, and move without the pairs' signs.
+template <bool TO_SOL, bool SIGNED>
 static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in, double* __restrict__ out) {
     pdl_enter();
     const int64_t tail = g.N - 2 * g.NI;
@@ -80,7 +82,7 @@ static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in
             const int64_t r = idx / pl;
             const int j = (int)(r % g.n2), k = (int)(r / g.n2);
             const MapEntry e = decode_interior(g, i, j, k);
-            const double sg = e.kind == KIND_MINUS ? -1.0 : 1.0;
+            const double sg = SIGNED && e.kind == KIND_MINUS ? -1.0 : 1.0;
             if (TO_SOL) {
                 reinterpret_cast<double2*>(out)[idx] = make_double2(in[e.re], sg * in[e.im]);
             } else {
@@ -98,12 +100,13 @@ static __global__ void solver_order_kernel(Geom g, const double* __restrict__ in
 }
 
 cudaError_t to_solver_order(const Geom& g, const double* ref, double* sol, cudaStream_t st) {
-    launch_pdl(pdl_pays(g.dim, g.N), solver_order_kernel<true>, ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, ref, sol);
+    launch_pdl(pdl_pays(g.dim, g.N), solver_order_kernel<true, true>, ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, ref, sol);
     return cudaGetLastError();
 }
 
-cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, cudaStream_t st) {
-    launch_pdl(pdl_pays(g.dim, g.N), solver_order_kernel<false>, ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, sol, ref);
+cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, bool is_signed, cudaStream_t st) {
+    launch_pdl(pdl_pays(g.dim, g.N), is_signed ? solver_order_kernel<false, true> : solver_order_kernel<false, false>,
+               ew_blocks(g.N / 2 + 1), EW_THREADS, 0, st, g, sol, ref);
     return cudaGetLastError();
 }
 
@@ -1233,8 +1236,8 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         h->launches += 1;
     }
     if (h->sorder) {
-        CK(to_reference_order(h->g, h->beta, beta_out, st));
-        if (c_out) CK(to_reference_order(h->g, h->c, c_out, st));
+        CK(to_reference_order(h->g, h->beta, beta_out, true, st));
+        if (c_out) CK(to_reference_order(h->g, h->c, c_out, false, st));
         h->launches += c_out ? 2 : 1;
     } else {
         CK(cudaMemcpyAsync(beta_out, h->beta, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
@@ -1327,7 +1330,7 @@ int csipm_admm(csipm_handle h, double rho, int maxt, double tol, double* z_out, 
         if (!std::isfinite(err)) { status = fail(h, CSIPM_ERR_NONFINITE, "non-finite ADMM iterate"); break; }
         ++t;
     }
-    if (h->sorder) CK(to_reference_order(h->g, z, z_out, st));
+    if (h->sorder) CK(to_reference_order(h->g, z, z_out, true, st));
     else CK(cudaMemcpyAsync(z_out, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     cudaEventRecord(h->ev1, st);
     CK(cudaEventSynchronize(h->ev1));

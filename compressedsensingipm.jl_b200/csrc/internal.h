@@ -388,7 +388,8 @@ cudaError_t solve_AtA32(csipm_handle h, const float* x, const Epi& epi, const in
 
 // signed permutation reference order <-> solver order (n = N entries)
 cudaError_t to_solver_order(const Geom& g, const double* ref, double* sol, cudaStream_t st);
-cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, cudaStream_t st);
+// is_signed: the vector changes sign with beta (c and other bounds of |beta| do not)
+cudaError_t to_reference_order(const Geom& g, const double* sol, double* ref, bool is_signed, cudaStream_t st);
 
 enum { RESID_NONE = 0, RESID_CG64 = 1, RESID_F32 = 2 };   // none / FP64 in cg_r / FP32 in f_r
 
