@@ -342,7 +342,8 @@ int build_product(BatchState& B, BProduct<Epi>& P, const std::vector<csipm_handl
     P.mask = hs[0]->op64.maskw != nullptr;
     std::vector<std::vector<BPass<Epi>>> t;
     // an instance's pass: its tile at the handle's lines (or rows) per CTA,
-    // laid out for the batch's block size
+    // laid out for the batch's block size (csipm_solve_batch has refused
+    // in-place rows)
     auto add = [&](int pass, const FftOperator<double>& op, PassArgs<double> a, const PassCfg& cfg, PassKind kind,
                    const double* src, const Epi& e, const int* sk) -> bool {
         if ((int)t.size() <= pass) t.resize(pass + 1);
@@ -364,7 +365,7 @@ int build_product(BatchState& B, BProduct<Epi>& P, const std::vector<csipm_handl
         t[pass].push_back(bp);
         P.smem[pass] = std::max(P.smem[pass], c.smem);
         P.gx[pass] = std::max(P.gx[pass], c.tiles);
-        return cfg.pp && c.smem <= FftOperator<double>::smem_limit();
+        return c.smem <= FftOperator<double>::smem_limit();
     };
     for (int k = 0; k < K; ++k) {
         FftOperator<double>& op = hs[k]->op64;
@@ -477,6 +478,11 @@ int csipm_solve_batch(csipm_handle* hs_in, int count, double* const* beta_out, c
         if (batch_kind(hs[k]) != batch_kind(hs[0]) || (hs[k]->op64.maskw != nullptr) != (hs[0]->op64.maskw != nullptr))
             return fail(nullptr, CSIPM_ERR_INVALID,
                         "a batch shares the dimension count, the long-row 1D passes and the presence of missing samples");
+        // rows longer than a tile run in place, in a kernel and with plans of
+        // their own that a batch's passes do not take
+        if (hs[k]->g.dim >= 2 && !hs[k]->op64.row_cfg.pp)
+            return fail(nullptr, CSIPM_ERR_UNSUPPORTED,
+                        "dimension 1 of an instance is too long for the batch's row pass; solve it alone");
         for (int j = 0; j < k; ++j)
             if (hs[j] == hs[k]) return fail(nullptr, CSIPM_ERR_INVALID, "a handle appears twice in the batch");
     }

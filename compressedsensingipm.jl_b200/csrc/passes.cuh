@@ -370,7 +370,10 @@ inline void lay_pass(const FftPlanDev& pl, int Ltab, int lines, int n, PassKind 
                      PassCfg* c) {
     c->tb = lines;
     c->pp = 1;
-    if (pl.L * csize > PASS_SMEM) {   // longer than a tile: PASS_STAGES and 16 bits may not hold it
+    // Refused before its stages are written: a line longer than a tile (16 bits
+    // may not hold it) and a plan of more stages than the arguments carry (the
+    // in-place rows' plans, radices up to 8, have up to 8 for lengths of a tile).
+    if (pl.L * csize > PASS_SMEM || pl.nst > PASS_STAGES) {
         c->smem = ~(size_t)0;
         return;
     }

@@ -19,7 +19,8 @@ bool make_fft_plan(int L, FftPlanDev* out, std::string* err);
 bool make_row_plan(int L, FftPlanDev* out, std::string* err);
 
 // The plan's stages in plan order (rev: reversed, as the inverse half of a row
-// pass runs it) with twiddles from a table of Ltab-th roots.
+// pass runs it) with twiddles from a table of Ltab-th roots.  Writes pl.nst of
+// them: the caller has checked that out holds as many.
 void fill_stages(const FftPlanDev& pl, int Ltab, bool rev, FftStage* out);
 
 // Complex values of the plan's prime tables (prime_tables, fft_device.cuh).

@@ -259,7 +259,9 @@ CSIPM_API int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm
  * block) and every element kernel runs all instances at once (gridDim.y =
  * instance).  Any sizes mix; the handles must share the dimension count,
  * whether they have missing samples, and for 1D whether the rows take the
- * long-row passes (N1/2 > 2048).  Each instance solves with its own options
+ * long-row passes (N1/2 > 2048).  2D and 3D instances whose rows are longer
+ * than an on-chip tile (N1 above about 12800) are refused with
+ * CSIPM_ERR_UNSUPPORTED; csipm_solve takes them.  Each instance solves with its own options
  * (tol, max_iter, ipm_cg_rtol, ipm_cg_forcing, preconditioner) by
  * csipm_solve's FP64 method in the reference packing: its iterates equal
  * csipm_solve's up to the order of floating-point sums.  Runs on hs[0]'s

@@ -1,0 +1,35 @@
+"""Batches of recoveries whose rows run in place (longer than an on-chip tile):
+refused as a batch before anything runs, solved one by one."""
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _problems(dims):
+    import csipm.problems as P
+    op0 = O.Operator(dims)
+    return [P.finalize(P.make_spec("2d", dims=dims, seed=60 + k), op0.A, op0.At) for k in range(2)]
+
+
+def _model(torch, prob):
+    import csipm
+    params = csipm.FFTParameters(2, prob.size, torch.tensor(prob.z0, device="cuda"), prob.lam, prob.missing)
+    return csipm.FFTNLPModel(params, rdft=True, tol=1e-8, ipm_cg_rtol=1e-2)
+
+
+# half rows of 6561 = 3^8 (8 stages in place) and 6480 (7)
+@pytest.mark.parametrize("dims", [(13122, 4), (12960, 6)], ids=lambda s: "x".join(map(str, s)))
+def test_batch_refuses_in_place_rows(cuda, dims):
+    import csipm
+    from csipm import _native
+    torch = cuda
+    models = [_model(torch, p) for p in _problems(dims)]
+    with pytest.raises(_native.CsipmError) as e:
+        csipm.ipm_solve_batch(models)
+    assert e.value.status == _native.CSIPM_ERR_UNSUPPORTED and "solve it alone" in str(e.value)
+    for m in models:
+        r = csipm.ipm_solve(m)
+        assert r.status == 0, r.stats
+        m.op_fft.close()
