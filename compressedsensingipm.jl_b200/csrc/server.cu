@@ -168,7 +168,8 @@ static void set_message(csipm_result* r, const char* msg) {
 }
 
 // Solves an admitted group on the slot's stream — one request through
-// csipm_solve, several through csipm_solve_batch — and fills one result per
+// csipm_solve, several through csipm_solve_batch (or one by one where that
+// does not take them) — and fills one result per
 // member (status, stats, message).  Members stage z0 and beta through one
 // pinned buffer, each at its own offset.
 static void run_group(const std::vector<Pending>& g, int cuda_graphs, cudaStream_t st, cudaMemPool_t pool,
@@ -243,9 +244,18 @@ static void run_group(const std::vector<Pending>& g, int cuda_graphs, cudaStream
                 bl.push_back(beta[k]);
             }
         if (!hl.empty()) {
+            // a batch that ends before its results are copied leaves the stats
+            // as they are: its members carry its error
             std::vector<csipm_stats> S(hl.size());
+            for (csipm_stats& x : S) x.status = CSIPM_ERR_CUDA;
             const int r = csipm_solve_batch(hl.data(), (int)hl.size(), bl.data(), S.data());
             const std::string batch_err = r != CSIPM_OK ? csipm_last_error(nullptr) : "";
+            if (r == CSIPM_ERR_UNSUPPORTED) {   // nothing ran: one by one
+                for (size_t j = 0; j < live.size(); ++j) {
+                    S[j].status = csipm_solve(hl[j], bl[j], nullptr, &S[j]);
+                    res[live[j]].group = 1;
+                }
+            }
             for (size_t j = 0; j < live.size(); ++j) {
                 const int k = live[j];
                 res[k].stats = S[j];

@@ -33,3 +33,24 @@ def test_batch_refuses_in_place_rows(cuda, dims):
         r = csipm.ipm_solve(m)
         assert r.status == 0, r.stats
         m.op_fft.close()
+
+
+def test_server_solves_them_one_by_one(cuda):
+    """A batching server gets such requests solved all the same: equal to the
+    solve alone (deterministic kernels), never an unsolved buffer with status 0."""
+    from csipm.serving import Server
+    import csipm
+    torch = cuda
+    dims = (13122, 4)
+    probs = _problems(dims)
+    with Server(slots=1, batch=4) as srv:
+        for k in range(3):   # the first keeps the one slot busy while the others queue
+            p = probs[k % 2]
+            srv.submit(p.size, p.z0, p.lam, p.missing, tag=k, tol=1e-8, ipm_cg_rtol=1e-2)
+        got = {r.tag: r for r in srv.drain()}
+    for k in range(3):
+        assert got[k].status == 0 and got[k].group == 1, got[k].message
+        m = _model(torch, probs[k % 2])
+        b = csipm.ipm_solve(m).beta.cpu().numpy()
+        assert abs(got[k].beta - b).max() <= 1e-12 * abs(b).max()
+        m.op_fft.close()
