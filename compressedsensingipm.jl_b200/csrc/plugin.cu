@@ -118,13 +118,15 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
         return CSIPM_OK;
     };
     cudaEventRecord(h->ev0, st);
-    if (h->opt.preconditioner) {
+    const bool pc = h->opt.preconditioner != 0;
+    bool other = false;   // the N-unknown start found diagonals that are not the built ones
+    if (pc) {
         // on N unknowns (kkt_schur_init_kernel says why the iterates are the 2N
         // method's); the second halves of the 2N buffers hold the diagonals
         double *x = h->k_x, *r = h->k_r, *p = h->k_p, *q = h->k_q, *D = h->k_x + n, *M = h->k_r + n;
         const int so = h->sorder ? 1 : 0;
-        ew_launch(kkt_schur_init_kernel, so ? n / 2 : n, st, h->g, so, w, pr_diag, r, p, D, M,
-                  h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
+        ew_launch(kkt_schur_init_kernel, so ? n / 2 : n, st, h->g, so, w, pr_diag, (const double*)h->L1,
+                  (const double*)h->L2, r, p, D, M, h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
         CK(cudaGetLastError());
         int chunk = 2, since = 0;
         for (int it = 0; it < maxit; ++it) {
@@ -142,27 +144,32 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
                 if (h->hcgs->done) break;
             }
         }
-        CK(cudaMemcpyAsync(h->hcgs, h->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
-        ew_launch(kkt_schur_back_kernel, so ? n / 2 : n, st, h->g, so, w, (const double*)x, pr_diag,
-                  (const CgScalars*)h->cgs);
-        CK(cudaGetLastError());
-        const int f = finish();
-        h->matvecs += h->hcgs->iters;
-        return f;
+        other = h->hcgs->other != 0;
+        if (!other) {
+            CK(cudaMemcpyAsync(h->hcgs, h->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
+            ew_launch(kkt_schur_back_kernel, so ? n / 2 : n, st, h->g, so, w, (const double*)x, pr_diag,
+                      (const CgScalars*)h->cgs);
+            CK(cudaGetLastError());
+            const int f = finish();
+            h->matvecs += h->hcgs->iters;
+            return f;
+        }
     }
-    const double* none = nullptr;   // no preconditioner: 2N vectors, reference packing
+    // the 2N method, reference packing: without the preconditioner, or on
+    // diagonals other than pr_diag's
+    const double *P11 = pc ? h->P11 : nullptr, *P12 = pc ? h->P12 : nullptr, *P22 = pc ? h->P22 : nullptr;
     ew_launch(kkt_rhs_kernel, n, st, n, w, pr_diag, h->k_b);
     CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));
-    ew_launch(kcg_init_kernel, n, st, n, h->k_b, h->k_x, h->k_r, h->k_p, none, none, none,
+    ew_launch(kcg_init_kernel, n, st, n, h->k_b, h->k_x, h->k_r, h->k_p, P11, P12, P22,
                                               h->ws(h->slots + SL_DUMMY), h->cgs, h->opt.cg_atol, h->opt.cg_rtol);
     CK(cudaGetLastError());
     int chunk = 2, since = 0;
     for (int it = 0; it < maxit; ++it) {
         EpiKcg ep{h->k_p, h->k_q, h->L1, h->L2, n, h->ws(&h->cgs->pq), 0.0};
         CK(op_AtA(h->op64, h->k_p, ep, &h->cgs->done, st));
-        ew_launch(kcg_update_kernel, n, st, n, it, h->k_x, h->k_r, h->k_p, h->k_q, none, none, none,
+        ew_launch(kcg_update_kernel, n, st, n, it, h->k_x, h->k_r, h->k_p, h->k_q, P11, P12, P22,
                                                      h->ws(h->slots + SL_DUMMY), h->cgs);
-        ew_launch(kcg_pupdate_kernel, n, st, n, it, h->k_r, h->k_p, none, none, none, h->cgs);
+        ew_launch(kcg_pupdate_kernel, n, st, n, it, h->k_r, h->k_p, P11, P12, P22, h->cgs);
         CK(cudaGetLastError());
         if (++since >= chunk || it + 1 == maxit) {
             since = 0;

@@ -43,7 +43,7 @@ struct CgScalars {
     int done;           // 1: converged or broke down (later kernels of the solve return at once)
     int iters;          // iterations completed
     int breakdown;      // 1: p'q <= 0 or non-finite
-    int pad;
+    int other;          // kkt_schur_init_kernel: 1: the solve is the 2N method's
     // Newton solves of the KKT plugin (kkt_schur_init_kernel): the eliminated
     // half's share of the scalars, zero elsewhere
     double S, rho, sig;
@@ -1049,16 +1049,23 @@ __device__ __forceinline__ void kkt_rhs(const double* __restrict__ w, long long 
     bz = w[n + i] - w3 - w4 - a - c;
 }
 
-// start from x = 0 (cg_update's START): r = r~, p = M r, the diagonals D and M, the scalars
+// start from x = 0 (cg_update's START): r = r~, p = M r, the diagonals D and M, the scalars.
+// K and P are the ones kkt_build stored (L1, L2).  D comes from pr_diag, which
+// gives 4 S1 S2/(S1 + S2) without the cancellation of L1 - L2^2/L1; where
+// pr_diag is not what was built from, the start is marked `other` and closed,
+// and the 2N method runs on the stored K.  (Two vectors read of some 27 at the
+// start and 14 in each iteration.)
 static __global__ void __launch_bounds__(EW_THREADS)
 kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const double* __restrict__ pr_diag,
+                      const double* __restrict__ L1, const double* __restrict__ L2,
                       double* __restrict__ r, double* __restrict__ p, double* __restrict__ D,
                       double* __restrict__ M, RedWorkspace ws, CgScalars* sc, double atol, double rtol) {
     pdl_enter();
     const long long n = g.N;
-    double acc[2] = {0.0, 0.0};
+    double acc[3] = {0.0, 0.0, 0.0};
     for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
         const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i], l1 = S1 + S2;
+        if (!(l1 == L1[i] && S1 - S2 == L2[i])) acc[2] += 1.0;
         double bb, bz;
         kkt_rhs(w, n, i, S1, S2, bb, bz);
         const double u = bz / l1, d = 4.0 * (S1 / l1) * S2, m = 1.0 / (1.0 + d);
@@ -1070,11 +1077,13 @@ kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const do
         acc[0] += rv * z;
         acc[1] += bz * u;
     });
-    if (grid_reduce<2>(acc, ws, 0u, 0u) && threadIdx.x == 0) {
+    if (grid_reduce<3>(acc, ws, 0u, 0u) && threadIdx.x == 0) {
         const double S = ws.out[1];
         cg_start(sc, ws.out[0] + S, atol, DevScalar(rtol));
         sc->S = S;
         sc->rho = sc->sig = 1.0;
+        sc->other = ws.out[2] > 0.0 ? 1 : 0;
+        if (sc->other) sc->done = 1;
     }
 }
 
