@@ -119,7 +119,7 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
     };
     cudaEventRecord(h->ev0, st);
     const bool pc = h->opt.preconditioner != 0;
-    bool other = false;   // the N-unknown start found diagonals that are not the built ones
+    bool other = false;   // the N-unknown start found diagonals it does not serve
     if (pc) {
         // on N unknowns (kkt_schur_init_kernel says why the iterates are the 2N
         // method's); the second halves of the 2N buffers hold the diagonals
@@ -132,7 +132,7 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
         for (int it = 0; it < maxit; ++it) {
             EpiCG<double> ep{p, D, q, h->ws(&h->cgs->pq), 0.0};
             CK(solve_AtA(h, p, ep, &h->cgs->done, st));
-            ew_launch(cg_update_kernel<double, double, true>, n, st, n, it, x, (const double*)nullptr, r, p, q, (const double*)M,
+            ew_launch(cg_update_kernel<double, double, true, false>, n, st, n, it, x, (const double*)nullptr, r, p, q, (const double*)M,
                       h->ws(h->slots + SL_DUMMY), h->cgs);
             ew_launch(cg_pupdate_kernel<double>, n, st, n, it, r, (const double*)M, p, h->cgs);
             CK(cudaGetLastError());
@@ -155,8 +155,8 @@ int csipm_kkt_solve(csipm_handle h, double* w, const double* pr_diag, int* cg_it
             return f;
         }
     }
-    // the 2N method, reference packing: without the preconditioner, or on
-    // diagonals other than pr_diag's
+    // the 2N method, reference packing: without the preconditioner, or on the
+    // diagonals kkt_schur_init_kernel leaves to it
     const double *P11 = pc ? h->P11 : nullptr, *P12 = pc ? h->P12 : nullptr, *P22 = pc ? h->P22 : nullptr;
     ew_launch(kkt_rhs_kernel, n, st, n, w, pr_diag, h->k_b);
     CK(cudaMemsetAsync(h->cgs, 0, sizeof(CgScalars), st));

@@ -106,7 +106,10 @@ static __global__ void cg_init_kernel(long long n, const double* __restrict__ rh
 // START: the first iteration takes its start from x0 (zero without one), so
 // nobody writes the start into x beforehand; a loop that is done before its
 // first step, or breaks down in it, copies the start.
-template <typename TV, typename TX, bool START>
+// POSITIVE: a p.q that is not positive is a breakdown (K is positive definite);
+// the plugin's solves go on, as the 2N method does (kcg_update_kernel), until
+// something is not finite.
+template <typename TV, typename TX, bool START, bool POSITIVE = true>
 __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* __restrict__ x, const TX* __restrict__ x0,
                                  TV* __restrict__ r, const TV* __restrict__ p, const TV* __restrict__ q,
                                  const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
@@ -120,7 +123,7 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
     const double rz = sc->rz[it & 1];
     // breakdown: every block sees the same p.q and returns before stepping,
     // so the iterate stays the last good one
-    if (!(pq > 0.0) || !isfinite(pq)) {
+    if (POSITIVE && (!(pq > 0.0) || !isfinite(pq))) {
         if (first) copy_start();
         if (blockIdx.x == 0 && threadIdx.x == 0) { sc->breakdown = 1; sc->done = 1; }
         return;
@@ -163,11 +166,11 @@ __device__ __forceinline__ void cg_update_kernel_body(long long n, int it, TX* _
         else if (sqrt(rzn) <= sc->thresh) sc->done = 1;
     }
 }
-template <typename TV, typename TX, bool START>
+template <typename TV, typename TX, bool START, bool POSITIVE = true>
 static __global__ void cg_update_kernel(long long n, int it, TX* __restrict__ x, const TX* __restrict__ x0, TV* __restrict__ r, const TV* __restrict__ p,
                                  const TV* __restrict__ q, const TV* __restrict__ Minv, RedWorkspace ws, CgScalars* sc) {
     pdl_enter();
-    cg_update_kernel_body<TV, TX, START>(n, it, x, x0, r, p, q, Minv, ws, sc);
+    cg_update_kernel_body<TV, TX, START, POSITIVE>(n, it, x, x0, r, p, q, Minv, ws, sc);
 }
 
 // p = Minv r + (rz'/rz) p
@@ -1052,8 +1055,9 @@ __device__ __forceinline__ void kkt_rhs(const double* __restrict__ w, long long 
 // start from x = 0 (cg_update's START): r = r~, p = M r, the diagonals D and M, the scalars.
 // K and P are the ones kkt_build stored (L1, L2).  D comes from pr_diag, which
 // gives 4 S1 S2/(S1 + S2) without the cancellation of L1 - L2^2/L1; where
-// pr_diag is not what was built from, the start is marked `other` and closed,
-// and the 2N method runs on the stored K.  (Two vectors read of some 27 at the
+// pr_diag is not what was built from, or an entry is negative, not finite or
+// leaves S1 + S2 = 0 to divide by, the start is marked `other` and closed, and
+// the 2N method runs on the stored K.  (Two vectors read of some 27 at the
 // start and 14 in each iteration.)
 static __global__ void __launch_bounds__(EW_THREADS)
 kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const double* __restrict__ pr_diag,
@@ -1065,7 +1069,7 @@ kkt_schur_init_kernel(Geom g, int sorder, const double* __restrict__ w, const do
     double acc[3] = {0.0, 0.0, 0.0};
     for_solver_entries(g, sorder, [&](long long i, long long s, double sg) {
         const double S1 = pr_diag[2 * n + i], S2 = pr_diag[3 * n + i], l1 = S1 + S2;
-        if (!(l1 == L1[i] && S1 - S2 == L2[i])) acc[2] += 1.0;
+        if (!(l1 == L1[i] && S1 - S2 == L2[i] && S1 >= 0.0 && S2 >= 0.0 && l1 > 0.0 && isfinite(l1))) acc[2] += 1.0;
         double bb, bz;
         kkt_rhs(w, n, i, S1, S2, bb, bz);
         const double u = bz / l1, d = 4.0 * (S1 / l1) * S2, m = 1.0 / (1.0 + d);

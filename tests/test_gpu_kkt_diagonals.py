@@ -52,3 +52,54 @@ def test_diagonals_other_than_the_built_ones(cuda, size, pc, layout, entries):
     assert kkt.krylov_iterations[-1] == it
     assert _close(wt.cpu().numpy(), sol)
     nlp.op_fft.close()
+
+
+def _cg_2n(op, K, b, steps):
+    """`steps` iterations of the preconditioned CG on 2N unknowns, whatever the
+    signs of p.q and r.z."""
+    n2 = b.size
+    mul = lambda v: OI.condensed_mul(op, K, np.zeros(n2), v, 1.0, 0.0)
+    pre = lambda v: OI.precond_mul(K, np.zeros(n2), v, 1.0, 0.0)
+    x, r = np.zeros(n2), b.copy()
+    p = pre(r)
+    rz = r @ p
+    for _ in range(steps):
+        q = mul(p)
+        a = rz / (p @ q)
+        x += a * p
+        r -= a * q
+        z = pre(r)
+        rz, old = r @ z, rz
+        p = z + rz / old * p
+    return x
+
+
+@pytest.mark.parametrize("size", [(200,), (62, 82), (22, 14, 34)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("layout", ["solver", "reference"])
+@pytest.mark.parametrize("diag", ["negative", "opposite", "zero"])
+def test_diagonals_that_are_not_positive(cuda, size, layout, diag):
+    """K is indefinite (negative), a pair of diagonals sums to zero (opposite),
+    or one of each pair is zero: three iterations and no error, as the 2N method."""
+    torch = cuda
+    nlp, kkt, op, rng = _system(torch, size, cg_rtol=0.0, cg_maxit=3, layout=layout)
+    N = op.N
+    S1, S2 = 1.0 + rng.random(N), 1.0 + rng.random(N)
+    if diag == "negative":
+        S1, S2 = -2.0 - S1, -2.0 - S2
+    elif diag == "opposite":
+        S2[::7] = -S1[::7]
+    else:
+        S2[::3] = 0.0
+    pr = np.concatenate([np.ones(2 * N), S1, S2])
+    prt = torch.tensor(pr, device="cuda")
+    kkt.build_kkt(prt)
+    # w3, w5 and w6 zero: b = [w1 + w4; w2 - w4], and no 0/0 in the back-substitution
+    w = rng.standard_normal((6, N))
+    w[2] = w[4] = w[5] = 0.0
+    wt = torch.tensor(w.reshape(-1), device="cuda")
+    kkt.solve_kkt(wt, prt)
+    assert kkt.krylov_iterations == [3]
+    x = _cg_2n(op, OI.kkt_build(pr, N), np.concatenate([w[0] + w[3], w[1] - w[3]]), 3)
+    got = wt.cpu().numpy()
+    assert _close(got[:2 * N], x)
+    nlp.op_fft.close()
