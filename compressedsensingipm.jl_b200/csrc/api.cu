@@ -588,7 +588,10 @@ IpmMode ipm_mode(csipm_handle h) {
 // the reductions of the stop test, the barrier diagonals and the start of the
 // predictor's CG at the tolerance *crtol (mixed precision at tight Newton
 // tolerances starts it from the right-hand side instead, make_rhs).
-cudaError_t launch_resid_pass(csipm_handle h, cudaStream_t st, const IpmMode& md, bool step, const double* crtol) {
+// This one and the two below are also recorded into build_ipm_graph's graph,
+// where nothing runs: they take the handle const, and the state of the solve
+// (rhs_due) is set beside their calls in csipm_solve.
+cudaError_t launch_resid_pass(const csipm_handle_s* h, cudaStream_t st, const IpmMode& md, bool step, const double* crtol) {
     const long long n = h->N;
     const double lam = h->lambda;
     const int pc = h->opt.preconditioner != 0;
@@ -596,7 +599,6 @@ cudaError_t launch_resid_pass(csipm_handle h, cudaStream_t st, const IpmMode& md
     const DevScalar tol(0.0, crtol);
     RedWorkspace ws = h->ws(h->slots + SL_RED);
     const double *sm = h->slots + SL_SIGMU, *al = h->slots + SL_ALPHA;
-    h->rhs_due = md.mixed ? 1 : 0;
     if (md.dir32)
         ew_launch(ipm_resdiag_kernel<float, float, float>, n, st, n, bv, h->Qb, lam, h->beta, h->s1, h->s2, h->z1, h->z2,
                   step ? h->f_dba : nullptr, step ? h->f_db : nullptr, sm, al, (double*)nullptr, (double*)nullptr,
@@ -615,7 +617,7 @@ cudaError_t launch_resid_pass(csipm_handle h, cudaStream_t st, const IpmMode& md
 // product.  Without one (mixed precision at tight tolerances, which refines
 // on exact residuals) only the start dba is copied; returns whether the CG
 // was started.
-cudaError_t launch_corrector_start(csipm_handle h, cudaStream_t st, const IpmMode& md, int rk, const double* crtol,
+cudaError_t launch_corrector_start(const csipm_handle_s* h, cudaStream_t st, const IpmMode& md, int rk, const double* crtol,
                                    bool* started) {
     const long long n = h->N;
     const double lam = h->lambda;
@@ -624,7 +626,6 @@ cudaError_t launch_corrector_start(csipm_handle h, cudaStream_t st, const IpmMod
     RedWorkspace ws = h->ws(h->slots + SL_DUMMY);
     const DevScalar tol(0.0, crtol);
     *started = rk != RESID_NONE && (md.dir32 || !md.mixed);
-    if (md.mixed) h->rhs_due = 2;
     if (!*started)
         return md.dir32 ? cudaMemcpyAsync(h->f_db, h->f_dba, sizeof(float) * n, cudaMemcpyDeviceToDevice, st)
                         : cudaMemcpyAsync(h->db, h->dba, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
@@ -644,7 +645,7 @@ cudaError_t launch_corrector_start(csipm_handle h, cudaStream_t st, const IpmMod
 
 // After the corrector: its step statistics, the step length and the beta
 // step (s and z take the same step inside the next residual pass).
-cudaError_t launch_step(csipm_handle h, cudaStream_t st, const IpmMode& md) {
+cudaError_t launch_step(const csipm_handle_s* h, cudaStream_t st, const IpmMode& md) {
     const long long n = h->N;
     const double lam = h->lambda;
     const double* sigmu_d = h->slots + SL_SIGMU;
@@ -1144,6 +1145,7 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         // a resumed iteration restarts its predictor at this iteration's tolerance
         CK(launch_resid_pass(h, st, md, pending,
                              dir32 ? (resume ? rin_dev : &h->ctl->rin_next) : (resume ? rt_dev : &h->ctl->rt_next)));
+        h->rhs_due = mixed ? 1 : 0;
         cudaEventRecord(h->ev_rp[1], st);
         pending = false;
         h->launches += 1;
@@ -1208,6 +1210,7 @@ int csipm_solve(csipm_handle h, double* beta_out, double* c_out, csipm_stats* st
         const int rk = (!mixed || o.ipm_cg_rtol >= MIXED_FP32_WARM_RTOL) ? h->resid_kind : RESID_NONE;
         bool cstart = false;
         CK(launch_corrector_start(h, st, md, rk, dir32 ? rin_dev : rt_dev, &cstart));
+        if (mixed) h->rhs_due = 2;
         cs = mixed ? schur_mixed(h, h->rhs, h->db, true, rt, o.cg_maxit, &its, dir32 ? h->f_db : nullptr, cstart,
                                  dir32 ? h->f_dba : nullptr, rin_dev)
                    : schur_cg(h, nullptr, h->db, true, h->dba, rt, o.cg_maxit, &its, rt_dev);
