@@ -15,7 +15,9 @@
 // processes: the file's choices are read at the first tuning, and every new
 // choice is appended to it as one JSON object per line,
 //   {"elem": 4, "dim": 3, "n": [320, 320, 320], "masked": 1,
-//    "s3_two": 1, "s3_tb": 0, "s2_tb": 0, "row_two": 1, "row_rb": 0, "s2_two": 1}
+//    "s3_two": 1, "s3_tb": 0, "s2_tb": 0, "row_two": 1, "row_rb": 0, "s2_two": 1, "gen": 2}
+// A choice holds for the kernels it was timed on: lines of another generation
+// (or of none) are passed over, and the size is tuned and appended anew.
 #pragma once
 #include <cstdio>
 #include <cstdlib>
@@ -27,6 +29,10 @@
 #include "internal.h"
 
 namespace csipm_internal {
+
+// Counted up whenever the kernels that are tuned change (2: the run-time-plan
+// passes of passes.cuh; lines before them carry none).
+constexpr int TUNE_GEN = 2;
 
 struct TuneChoice {
     int s3_two = 1, s3_tb = 0;     // 1: two-level; else run-time-plan tb (0: the heuristic's)
@@ -59,7 +65,11 @@ inline const std::string& tune_cache_path() {
     return p;
 }
 
-// Reads the persisted choices once (tune_mu held); lines that do not parse are skipped.
+// a width the tuner can have written: 0 (the heuristic's) or a power of two up to 16
+inline bool tune_width(int w) { return w >= 0 && w <= 16 && (w & (w - 1)) == 0; }
+
+// Reads the persisted choices once (tune_mu held); lines that do not parse, or
+// that no tuning of these kernels wrote, are skipped.
 inline void tune_cache_load() {
     static bool loaded = false;
     if (loaded) return;
@@ -72,12 +82,13 @@ inline void tune_cache_load() {
     while (std::fgets(line, sizeof(line), f)) {
         int elem, dim, n1, n2, n3, masked;
         TuneChoice c;
-        // lines without s2_two (written before it was tuned) keep the two-level kernel
+        int gen = 0;
         if (std::sscanf(line,
                         " {\"elem\": %d, \"dim\": %d, \"n\": [%d, %d, %d], \"masked\": %d, \"s3_two\": %d, "
-                        "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d",
+                        "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d, \"gen\": %d}",
                         &elem, &dim, &n1, &n2, &n3, &masked, &c.s3_two, &c.s3_tb, &c.s2_tb, &c.row_two,
-                        &c.row_rb, &c.s2_two) >= 11)
+                        &c.row_rb, &c.s2_two, &gen) == 13 &&
+            gen == TUNE_GEN && tune_width(c.s3_tb) && tune_width(c.s2_tb) && tune_width(c.row_rb))
             tune_cache()[TuneKey{elem, dim, n1, n2, n3, masked}] = c;
     }
     std::fclose(f);
@@ -91,9 +102,9 @@ inline void tune_cache_append(const TuneKey& k, const TuneChoice& c) {
     if (!f) return;
     std::fprintf(f,
                  "{\"elem\": %d, \"dim\": %d, \"n\": [%d, %d, %d], \"masked\": %d, \"s3_two\": %d, "
-                 "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d}\n",
+                 "\"s3_tb\": %d, \"s2_tb\": %d, \"row_two\": %d, \"row_rb\": %d, \"s2_two\": %d, \"gen\": %d}\n",
                  std::get<0>(k), std::get<1>(k), std::get<2>(k), std::get<3>(k), std::get<4>(k), std::get<5>(k),
-                 c.s3_two, c.s3_tb, c.s2_tb, c.row_two, c.row_rb, c.s2_two);
+                 c.s3_two, c.s3_tb, c.s2_tb, c.row_two, c.row_rb, c.s2_two, TUNE_GEN);
     std::fclose(f);
 }
 
