@@ -145,19 +145,20 @@ float tune_time(cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1, F&& launch) {
     return best;
 }
 
+// A width that does not fit leaves the heuristic's configuration (the
+// configurations are filled in while they are tried).
 template <typename T>
 void apply_choice(FftOperator<T>& op, const TuneChoice& c) {
     const Geom& g = op.g;
+    PassCfg t;
     if (g.dim == 3) {
         if (!c.s3_two) op.s3_A = op.s3_B = 0;
-        if (c.s3_tb) strided_cfg_tb<T>(op.plan3, g.m1 + 1, g.n2, c.s3_tb, &op.s3_cfg);
+        if (c.s3_tb && strided_cfg_tb<T>(op.plan3, g.m1 + 1, g.n2, c.s3_tb, &t)) op.s3_cfg = t;
     }
     if (!c.s2_two) op.s2_A = op.s2_B = 0;
-    if (g.dim >= 2 && c.s2_tb) strided_cfg_tb<T>(op.plan2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, c.s2_tb, &op.s2_cfg);
-    if (g.dim >= 2) {
-        if (!c.row_two) op.r_A = op.r_B = 0;
-        if (c.row_rb) row_cfg_rb(op, g.n2 * g.n3, c.row_rb, &op.row_cfg);
-    }
+    if (c.s2_tb && strided_cfg_tb<T>(op.plan2, g.m1 + 1, g.dim == 3 ? g.n3 : 1, c.s2_tb, &t)) op.s2_cfg = t;
+    if (!c.row_two) op.r_A = op.r_B = 0;
+    if (c.row_rb && op.row_cfg.pp && row_cfg_rb(op, g.n2 * g.n3, c.row_rb, &t)) op.row_cfg = t;
 }
 
 // Tunes op (2D/3D; 1D keeps its heuristic) on stream st; op.spec holds scratch.

@@ -1,7 +1,9 @@
 """The persisted tuning choices (CSIPM_TUNE_CACHE): lines that no tuning of the
-present kernels wrote are passed over and their sizes tuned again."""
+present kernels wrote are passed over and their sizes tuned again, and a width
+that does not fit leaves the heuristic's configuration."""
 import json
 import os
+import re
 import subprocess
 import sys
 
@@ -48,3 +50,18 @@ def test_lines_of_other_kernels_are_tuned_again(cuda, tmp_path):
         _write(path, entry)
         lines = _open(path, size)
         assert len(lines) == 2 and lines[0] == entry and lines[1]["gen"] == gen, entry
+
+
+@pytest.mark.parametrize("size,fits_not", [((4, 4, 1000), {"s3_two": 0, "s3_tb": 16}), ((6, 2000), {"s2_two": 0, "s2_tb": 8}),
+                                           ((3000, 64), {"row_two": 0, "row_rb": 16}), ((12804, 4), {"row_two": 0, "row_rb": 1})],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+def test_a_choice_that_does_not_fit(cuda, tmp_path, size, fits_not):
+    """The heuristic's configuration stays, so the product runs and is right."""
+    with open(os.path.join(PKG, "csrc", "tune.cuh")) as f:
+        gen = int(re.search(r"TUNE_GEN = (\d+)", f.read()).group(1))
+    n = list(size) + [1] * (3 - len(size))
+    entry = dict(elem=8, dim=len(size), n=n, masked=0, s3_two=1, s3_tb=0, s2_tb=0, row_two=1, row_rb=0, s2_two=1, gen=gen)
+    path = tmp_path / "f.jsonl"
+    entry.update(fits_not)
+    _write(path, entry)
+    assert len(_open(path, size)) == 1   # taken, not tuned again
