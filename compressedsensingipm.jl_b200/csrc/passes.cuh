@@ -257,7 +257,11 @@ __global__ void __launch_bounds__(1024) row_pass_ip_kernel(PassArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* buf = reinterpret_cast<C*>(smem_raw);
     const int M = a.g.m1;
-    constexpr int RB = 1, TBP = 1;
+    // One row a CTA.  The layout comes in at run time: with RB = TBP = 1 known to
+    // the compiler it unrolled the engine's stages into twice the spills at the
+    // 64 registers that 1024 threads leave (5888 bytes for 3392): A'A on
+    // 12804 x 4 samples (rows of 2 3 11 97) 1310 us, so 720.
+    const int RB = 1 << a.lay.lg, TBP = a.lay.tbp;
     __shared__ int s_rad[FFT_MAX_STAGES];
     load_radices(a.pl, s_rad);
     const C* tw = a.tw;
@@ -623,6 +627,7 @@ public:
         }
         cfg->pp = 0;
         cfg->tb = 1;
+        cfg->lay = TileLay{0, 1};
         cfg->threads = thr;
         cfg->smem = o1;
         cfg->tiles = nrows;
