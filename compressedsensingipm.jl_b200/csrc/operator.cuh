@@ -76,8 +76,9 @@ struct PassArgs {
 // is read) until that one has completed and its writes are visible; then the
 // next kernel may be placed in turn.  Every kernel of a chain waits, so the
 // order of the stream holds throughout.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
