@@ -24,7 +24,9 @@
 // range sit in L2), so what counts is launches and the chain inside one:
 // three launches where four kernels ran (a plain lines pass, then the post-
 // processing over all k), and register-radix stages (fft_device.cuh) with
-// loads and stores attached to the first and last stage.
+// loads and stores attached to the first and last stage.  Epilogues with many
+// operands on long vectors take the post-processing out of the last pass again
+// (l1d_last).
 #pragma once
 #include "passes.cuh"
 
@@ -259,6 +261,41 @@ l1d_last_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restri
     l1d_last_kernel_body<T, Epi>(a, twN, P, Q, epi);
 }
 
+// ----------------------------------------------------------------- post pass
+// R2C post-processing and epilogue of Z[k] and Z[M-k] from the spectrum, one
+// thread a pair of positions: the last pass of the plugins' epilogues on long
+// vectors (l1d_last says when).
+template <typename T, class Epi>
+__global__ void __launch_bounds__(256) l1d_post_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN,
+                                                       Epi epi) {
+    pdl_enter();
+    using C = cplx_t<T>;
+    if (a.skip && *a.skip) return;
+    const int M = a.g.m1;
+    Epi ep = epi;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; 2 * k <= M; k += gridDim.x * blockDim.x) {
+        const C zk = a.spec[k];
+        if (k == 0) {
+            scatter1<T>(M, 0, r2c_post(zk, zk, twN[0]), ep);
+            scatter1<T>(M, M, mk((T)2 * (zk.x - zk.y), (T)0), ep);
+        } else if (2 * k == M) {
+            scatter1<T>(M, k, r2c_post(zk, zk, twN[k]), ep);
+        } else {
+            // the operands of both entries of a position before either is stored
+            const C zm = a.spec[M - k];
+            const C v[2] = {r2c_post(zk, zm, twN[k]), r2c_post(zm, zk, twN[M - k])};
+            const int at[2] = {k, M - k};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const typename Epi::Pre pr = ep.pre(at[q] + 1), pi = ep.pre(M + at[q]);
+                ep.put(at[q] + 1, SQRT2_D * (double)v[q].x, pr);
+                ep.put(M + at[q], SQRT2_D * (double)v[q].y, pi);
+            }
+        }
+    }
+    ep.finish();
+}
+
 // ---------------------------------------------------------------- launchers
 // pass: 0 first, 1 row, 2 last
 template <typename T>
@@ -301,8 +338,32 @@ cudaError_t l1d_row(const FftOperator<T>& op, double scale, const T* real_in, T*
     return cudaGetLastError();
 }
 
+// The last pass.  An epilogue with many operands (the KKT plugins': 4 to 12
+// values an entry) meets a tile of two to eight lines badly: every operand is
+// read 8 to 32 bytes at a time, a few hundred threads wait for them, and long
+// vectors have only tiles of two lines.  From L1D_POST_N samples such an epilogue
+// takes a pass of its own, after the lines went through in place.  Measured on
+// B200, in the last pass -> in its own, us waited for: condensed product 16384
+// 29.4 -> 31.6, 32768 32.9 -> 32.4, 65536 39.2 -> 33.0, 262144 62.8 -> 38.2,
+// 777600 102 -> 59; the plugin's 6N product 16384 31.4 -> 32.7, 32768 36.9 ->
+// 33.9, 262144 89.5 -> 41.3; 20 CG iterations on 2N vectors 16384 776 -> 780,
+// 32768 802 -> 791, 262144 1251 -> 1038.
+constexpr long long L1D_POST_N = 1LL << 15;
 template <typename T, class Epi>
 cudaError_t l1d_last(const FftOperator<T>& op, const Epi& epi, const int* skip, cudaStream_t st) {
+    if constexpr (sizeof(typename Epi::Pre) > 2 * sizeof(double)) {
+        if (op.g.N >= L1D_POST_N) {
+            PassArgs<T> a = l1d_args(op, 0, 1.0, skip);
+            a.n_lines = a.sx = op.l1P;
+            a.n_outer = 1;
+            cudaError_t e = launch_strided<T, false, IN_SPEC, OUT_SPEC>(op.f_cfg, a, (const double*)nullptr,
+                                                                       EpiStore<double>{nullptr}, st);
+            if (e != cudaSuccess) return e;
+            const int blocks = std::min(1024, op.g.m1 / 512 + 1);
+            launch_pdl(pdl_pays(1, op.g.N), l1d_post_kernel<T, Epi>, blocks, 256, 0, st, a, op.tw1, epi);
+            return cudaGetLastError();
+        }
+    }
     auto k = l1d_last_kernel<T, Epi>;
     const PassCfg& c = op.q_cfg;
     const cudaError_t e = smem_optin(k, c.smem);
