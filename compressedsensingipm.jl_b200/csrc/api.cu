@@ -491,7 +491,11 @@ int profile_impl(csipm_handle h, FftOperator<T>& op, const T* x, T* D, T* q, int
         return CSIPM_OK;
     };
     int r = 0;
-    if (g.dim == 1) {
+    if (op.l1_one) {
+        r = timeit([&] { return op_AtA(op, x, ecg, nullptr, st); }, 4 * w * N + maskb,
+                   f32 ? "fp32 row: gather+FFT+scatter+CG" : "row: gather+C2R+mask+R2C+scatter+CG");
+        if (r) return r;
+    } else if (g.dim == 1) {
         const double M = (double)g.m1;
         r = timeit([&] { return l1d_first(op, x, nullptr, st); }, w * N + cw * M,
                    f32 ? "fp32 1D lines: gather+C2R+inverse" : "1D lines: gather+C2R+inverse");

@@ -279,6 +279,9 @@ cudaError_t op_AtA(FftOperator<T>& op, const TS* x, const Epi& epi, const int* s
     constexpr int SOUT = SOL ? OUT_SSCATTER : OUT_SCATTER;
     if constexpr (SOL) {
         if (!solver_order_ok(op)) return cudaErrorInvalidValue;
+    } else if (op.l1_one) {
+        return mask ? l1d_one<T, IN_GATHER, OUT_SCATTER, true>(op, x, epi, sc, nullptr, nullptr, skip, st)
+                    : l1d_one<T, IN_GATHER, OUT_SCATTER, false>(op, x, epi, sc, nullptr, nullptr, skip, st);
     } else if (g.dim == 1) {
         e = l1d_first(op, x, skip, st);
         if (e != cudaSuccess) return e;
@@ -322,6 +325,9 @@ cudaError_t op_A(FftOperator<T>& op, const TS* beta, T* x, cudaStream_t st) {
     EpiStore<double> none{nullptr};
     PassArgs<T> ra = op.row_args(1.0 / std::sqrt((double)g.N), nullptr, x);
     cudaError_t e;
+    if (op.l1_one)
+        return mask ? l1d_one<T, IN_GATHER, OUT_REAL, true>(op, beta, none, ra.scale, nullptr, x, nullptr, st)
+                    : l1d_one<T, IN_GATHER, OUT_REAL, false>(op, beta, none, ra.scale, nullptr, x, nullptr, st);
     if (g.dim == 1) {
         e = l1d_first(op, beta, nullptr, st);
         if (e != cudaSuccess) return e;
@@ -347,6 +353,8 @@ cudaError_t op_At(FftOperator<T>& op, const T* z, const Epi& epi, cudaStream_t s
     EpiStore<double> none{nullptr};
     PassArgs<T> ra = op.row_args(1.0 / (2.0 * std::sqrt((double)g.N)), z, nullptr);
     cudaError_t e;
+    if (op.l1_one)
+        return l1d_one<T, IN_REAL, OUT_SCATTER, false>(op, (const T*)nullptr, epi, ra.scale, z, nullptr, nullptr, st);
     if (g.dim == 1) {
         e = l1d_row<T, IN_REAL, OUT_SPEC, false>(op, ra.scale, z, nullptr, nullptr, st);
         if (e != cudaSuccess) return e;
@@ -363,7 +371,7 @@ cudaError_t op_At(FftOperator<T>& op, const T* z, const Epi& epi, cudaStream_t s
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 inline int passes_per_product(const Geom& g) {
-    return g.dim == 3 ? 5 : 3;
+    return g.dim == 3 ? 5 : (g.dim == 1 && g.n1 <= L1D_ONE_N ? 1 : 3);
 }
 
 inline int read_slots(csipm_handle h, int first, int count) {

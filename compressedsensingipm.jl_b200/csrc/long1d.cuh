@@ -23,7 +23,7 @@
 // The passes are bound by latency, not bandwidth (1D vectors of the serving
 // range sit in L2), so what counts is launches and the chain inside one:
 // three launches where four kernels ran (a plain lines pass, then the post-
-// processing over all k), and register-radix stages (fft_device.cuh) with
+// processing over all k), one for short rows (l1d_one_kernel), and register-radix stages (fft_device.cuh) with
 // loads and stores attached to the first and last stage.  Epilogues with many
 // operands on long vectors take the post-processing out of the last pass again
 // (l1d_last).
@@ -261,39 +261,82 @@ l1d_last_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restri
     l1d_last_kernel_body<T, Epi>(a, twN, P, Q, epi);
 }
 
-// ----------------------------------------------------------------- post pass
-// R2C post-processing and epilogue of Z[k] and Z[M-k] from the spectrum, one
-// thread a pair of positions: the last pass of the plugins' epilogues on long
-// vectors (l1d_last says when).
+// ------------------------------------------------- post-processing of a pair
+// R2C post-processing and epilogue of positions k and M-k (0 <= 2k <= M) from
+// Z[k] and Z[M-k], which z(k) reads.
+template <typename T, class Epi, class Z>
+__device__ __forceinline__ void l1d_post_pair(int M, int k, Z&& z, const cplx_t<T>* __restrict__ twN, Epi& ep) {
+    using C = cplx_t<T>;
+    const C zk = z(k);
+    if (k == 0) {
+        scatter1<T>(M, 0, r2c_post(zk, zk, twN[0]), ep);
+        scatter1<T>(M, M, mk((T)2 * (zk.x - zk.y), (T)0), ep);
+    } else if (2 * k == M) {
+        scatter1<T>(M, k, r2c_post(zk, zk, twN[k]), ep);
+    } else {
+        // the operands of both entries of a position before either is stored
+        const C zm = z(M - k);
+        const C v[2] = {r2c_post(zk, zm, twN[k]), r2c_post(zm, zk, twN[M - k])};
+        const int at[2] = {k, M - k};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const typename Epi::Pre pr = ep.pre(at[q] + 1), pi = ep.pre(M + at[q]);
+            ep.put(at[q] + 1, SQRT2_D * (double)v[q].x, pr);
+            ep.put(M + at[q], SQRT2_D * (double)v[q].y, pi);
+        }
+    }
+}
+
+// Post pass: one thread a pair of positions, Z from the spectrum.  The last pass
+// of the plugins' epilogues on long vectors (l1d_last says when).
 template <typename T, class Epi>
 __global__ void __launch_bounds__(256) l1d_post_kernel(const __grid_constant__ PassArgs<T> a, const cplx_t<T>* __restrict__ twN,
                                                        Epi epi) {
     pdl_enter();
-    using C = cplx_t<T>;
     if (a.skip && *a.skip) return;
     const int M = a.g.m1;
     Epi ep = epi;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; 2 * k <= M; k += gridDim.x * blockDim.x) {
-        const C zk = a.spec[k];
-        if (k == 0) {
-            scatter1<T>(M, 0, r2c_post(zk, zk, twN[0]), ep);
-            scatter1<T>(M, M, mk((T)2 * (zk.x - zk.y), (T)0), ep);
-        } else if (2 * k == M) {
-            scatter1<T>(M, k, r2c_post(zk, zk, twN[k]), ep);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; 2 * k <= M; k += gridDim.x * blockDim.x)
+        l1d_post_pair<T>(M, k, [&](int x) { return a.spec[x]; }, twN, ep);
+    ep.finish();
+}
+
+// ------------------------------------------------------- short rows, one launch
+// A whole product of a row of up to L1D_ONE_N samples in one CTA: the row plan
+// of M from the gather (or the real samples) to the scatter (or the samples),
+// with the C2R and R2C steps at its ends and no spectrum in HBM.
+template <typename T, int IN, int OUT, bool MASK, typename TS, class Epi>
+__global__ void __launch_bounds__(PASS_THREADS, pass_min_ctas<T>())
+l1d_one_kernel(const __grid_constant__ PassArgs<T> a, const TS* __restrict__ src, Epi epi) {
+    pdl_enter();
+    using C = cplx_t<T>;
+    if (a.skip && *a.skip) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FftTile<C> t = make_tile(a, smem_raw);
+    const int M = a.g.m1;
+    const L1dRow<T, MASK> base{nullptr, a.real_in, a.real_out, a.maskw, nullptr, 0, 1, (T)a.scale, true};
+    L1dRowReal<T, MASK> re{base};
+    if constexpr (IN == IN_REAL) {
+        first_stage<T, false>(t, re);
+    } else {
+        t.st = a.inv;
+        L1dFirst<T, TS> in{src, nullptr, a.tw, M, 1, 0};
+        first_stage<T, true>(t, in);
+        mid_stages<T, true>(t, 1, t.nst - 1);
+        if constexpr (OUT == OUT_REAL) {
+            last_stage<T, true>(t, re);
         } else {
-            // the operands of both entries of a position before either is stored
-            const C zm = a.spec[M - k];
-            const C v[2] = {r2c_post(zk, zm, twN[k]), r2c_post(zm, zk, twN[M - k])};
-            const int at[2] = {k, M - k};
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const typename Epi::Pre pr = ep.pre(at[q] + 1), pi = ep.pre(M + at[q]);
-                ep.put(at[q] + 1, SQRT2_D * (double)v[q].x, pr);
-                ep.put(M + at[q], SQRT2_D * (double)v[q].y, pi);
-            }
+            chain_stage<T>(t, [&](int n, int, C z) { return base.keep(n, z); });
+            t.st = a.fwd;
         }
     }
-    ep.finish();
+    if constexpr (OUT == OUT_SCATTER) {
+        mid_stages<T, false>(t, 1, t.nst);
+        Epi ep = epi;
+        for (int k = threadIdx.x; 2 * k <= M; k += blockDim.x)
+            l1d_post_pair<T>(M, k, [&](int x) { return t.buf[t.cur + t.lay.at(x, 0)]; }, a.tw, ep);
+        ep.finish();
+    }
 }
 
 // ---------------------------------------------------------------- launchers
@@ -372,6 +415,20 @@ cudaError_t l1d_last(const FftOperator<T>& op, const Epi& epi, const int* skip, 
     return cudaGetLastError();
 }
 
+// A whole product of a short row (op.l1_one).
+template <typename T, int IN, int OUT, bool MASK, typename TS, class Epi>
+cudaError_t l1d_one(const FftOperator<T>& op, const TS* src, const Epi& epi, double scale, const T* real_in, T* real_out,
+                    const int* skip, cudaStream_t st) {
+    auto k = l1d_one_kernel<T, IN, OUT, MASK, TS, Epi>;
+    const PassCfg& c = op.row_cfg;
+    const cudaError_t e = smem_optin(k, c.smem);
+    if (e != cudaSuccess) return e;
+    PassArgs<T> a = op.row_args(scale, real_in, real_out);
+    a.skip = skip;
+    launch_pdl(pdl_pays(1, op.g.N), k, 1, c.threads, c.smem, st, a, src, epi);
+    return cudaGetLastError();
+}
+
 // compiled once (passes_r*.cu): the kernels of one precision, and the last
 // pass's epilogues
 #define CSIPM_1D_LIST64(X) X(double, EpiStore<double>, EpiCG<double>)
@@ -379,7 +436,14 @@ cudaError_t l1d_last(const FftOperator<T>& op, const Epi& epi, const int* skip, 
 #define CSIPM_PASS_1D_ROW(EXT, T, IN, OUT, MASK)                                                                      \
     EXT template cudaError_t l1d_row<T, IN, OUT, MASK>(const FftOperator<T>&, double, const T*, T*, const int*,        \
                                                        cudaStream_t);
+#define CSIPM_PASS_1D_ONE(EXT, T, IN, OUT, MASK, EPI)                                                                 \
+    EXT template cudaError_t l1d_one<T, IN, OUT, MASK, T, EPI>(const FftOperator<T>&, const T*, const EPI&, double,    \
+                                                               const T*, T*, const int*, cudaStream_t);
 #define CSIPM_PASS_1D(EXT, T, EPI1, EPI2)                                                                              \
+    CSIPM_PASS_1D_ONE(EXT, T, IN_GATHER, OUT_SCATTER, true, EPI1)                                                      \
+    CSIPM_PASS_1D_ONE(EXT, T, IN_GATHER, OUT_SCATTER, false, EPI1)                                                     \
+    CSIPM_PASS_1D_ONE(EXT, T, IN_GATHER, OUT_SCATTER, true, EPI2)                                                      \
+    CSIPM_PASS_1D_ONE(EXT, T, IN_GATHER, OUT_SCATTER, false, EPI2)                                                     \
     EXT template cudaError_t l1d_first<T, T>(const FftOperator<T>&, const T*, const int*, cudaStream_t);               \
     CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_SPEC, true)                                                                 \
     CSIPM_PASS_1D_ROW(EXT, T, IN_SPEC, OUT_SPEC, false)                                                                \

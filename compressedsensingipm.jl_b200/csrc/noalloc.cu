@@ -89,8 +89,8 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
     op.g = g;
     op.stream = (cudaStream_t)stream;
     std::string err;
-    const bool long1d = dim == 1;   // the handle path's four-step rows
     if (!op.make_plans(&err)) return static_fail(CSIPM_ERR_UNSUPPORTED, err);
+    const bool long1d = dim == 1 && !op.l1_one;   // the handle path's four-step rows
 
     const size_t spec_b = align256(sizeof(C) * (size_t)g.ld1 * g.n2 * g.n3);
     const size_t tw1_b = align256(sizeof(C) * (size_t)g.n1);
@@ -127,13 +127,16 @@ int csipm_apply_AtA_static(int dim, const int* size, const uint32_t* keep_bits, 
     if (e == cudaSuccess && long1d) e = put_twiddles(op.l1Q, op.twQ, s);
     if (e != cudaSuccess) return static_fail(CSIPM_ERR_CUDA, std::string("twiddle kernel: ") + cudaGetErrorString(e));
 
-    // the fused passes of A^T A: five (3D) or three (2D, 1D)
+    // the fused passes of A^T A: five (3D), three (2D, 1D) or one (short 1D rows)
     const double sc = 1.0 / (2.0 * (double)g.N);
     const bool mask = keep_bits != nullptr;
     EpiStore<double> none{nullptr};
     EpiStore<double> out{y};
     PassArgs<double> ra = op.row_args(sc, nullptr, nullptr);
-    if (long1d) {
+    if (op.l1_one) {
+        e = mask ? l1d_one<double, IN_GATHER, OUT_SCATTER, true>(op, x, out, sc, nullptr, nullptr, nullptr, s)
+                 : l1d_one<double, IN_GATHER, OUT_SCATTER, false>(op, x, out, sc, nullptr, nullptr, nullptr, s);
+    } else if (long1d) {
         e = l1d_first(op, x, nullptr, s);
         if (e == cudaSuccess)
             e = mask ? l1d_row<double, IN_SPEC, OUT_SPEC, true>(op, sc, nullptr, nullptr, nullptr, s)

@@ -458,6 +458,14 @@ constexpr int L1D_MIN_M = 2048;     // above: rows whose split must have Q >= 2
 constexpr int L1D_MAX_P = 4096;     // row length of the four-step row kernel
 constexpr int L1D_MAX_Q = 768;      // line length of the first and last passes
 
+// Rows of up to this many samples run their products in one launch of one CTA
+// (l1d_one_kernel): three launches cost more than the idle SMs.  FP64 on B200,
+// three launches -> one, us waited for: A'A 64 18.2 -> 13.0, 500 23.7 -> 14.3,
+// 2048 23.2 -> 17.2, 4096 25.5 -> 21.4, 6000 26.6 -> 24.6, 8192 27.0 -> 32.5; the
+// plugin's 6N product 500 25.6 -> 17.5, 4096 28.3 -> 28.0, 6000 30.1 -> 33.3;
+// recovery 500 1034 -> 771, 4096 1428 -> 1289, 8192 1151 -> 1315.
+constexpr int L1D_ONE_N = 4096;
+
 // M = P*Q with Q the largest divisor of M not above sqrt(M) (nor L1D_MAX_Q),
 // P = M/Q; false when P exceeds L1D_MAX_P.  Q = 1 (M prime) up to L1D_MIN_M.
 inline bool l1d_split(int M, int* P, int* Q) {
@@ -532,6 +540,7 @@ public:
     C* twP = nullptr;
     C* twQ = nullptr;
     PassCfg f_cfg, p_cfg, q_cfg;    // first lines, rows, last lines (pairs)
+    bool l1_one = false;            // a short row: products in one launch (plan1, row_cfg)
 
     // stream-ordered allocations from this pool on `stream` when set (the
     // handle's), else plain cudaMalloc/cudaFree
@@ -665,6 +674,8 @@ public:
                 return false;
             }
             plan1 = FftPlanDev{};
+            std::string none;
+            l1_one = g.n1 <= L1D_ONE_N && make_row_plan(g.m1, &plan1, &none) && rows_cfg(plan1, 1, 1, PASS_SMEM, &row_cfg);
             return make_row_plan(l1P, &planP, err) && make_fft_plan(l1Q, &planQ, err) && choose_1d(err);
         }
         if (!make_row_plan(g.m1, &plan1, err) || !choose_row(g.n2 * g.n3, &row_cfg, err)) return false;

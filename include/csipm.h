@@ -419,8 +419,8 @@ CSIPM_API int csipm_server_destroy(csipm_server s);
  * last pass with the CG epilogue q = A^T A p + D p, p.q).  Writes up to 8
  * entries: ms_out[k] = average device ms per launch, bytes_out[k] = algorithmic
  * HBM bytes per launch (each array read or written once), name_out (optional,
- * 8 x 32 chars) = kernel role.  *npass receives the pass count (3 in 1D and
- * 2D, 5 in 3D).  x: N, 16-byte aligned.  A CSIPM_MIXED handle times the FP32
+ * 8 x 32 chars) = kernel role.  *npass receives the pass count (1 in 1D up
+ * to 4096 samples, 3 above and in 2D, 5 in 3D).  x: N, 16-byte aligned.  A CSIPM_MIXED handle times the FP32
  * passes of its CG product (x rounded to FP32).  The reference keeps only host-side timers
  * (src/fft_utils.jl:24-25); this has no counterpart there. */
 CSIPM_API int csipm_profile_passes(csipm_handle h, const double* x, int reps, double* ms_out, double* bytes_out,
