@@ -46,8 +46,8 @@ struct BInst {
     __device__ __forceinline__ bool running() const { return ctl->status == IPM_RUNNING; }
 };
 
-// One FFT pass of one instance: its arguments, source and epilogue; the
-// long-row fields serve the four-step 1D passes.
+// One FFT pass of one instance: its arguments, source and epilogue.
+// P and Q are those of the 1D passes.
 template <class Epi>
 struct BPass {
     PassArgs<double> a;
@@ -312,7 +312,8 @@ struct BatchState {
 int batch_kind(csipm_handle h) {
     if (h->g.dim == 3) return PK_3D;
     if (h->g.dim == 2) return PK_2D;
-    return h->g.m1 > L1D_MIN_M ? PK_1DL : PK_1D;   // the split classes of a batch (internal.h)
+    // both run the same three passes; the two classes stay apart as csipm.h says
+    return h->g.m1 > L1D_MIN_M ? PK_1DL : PK_1D;
 }
 
 // Persistent-pass grid: the batch shares one wave of the kernel's CTAs

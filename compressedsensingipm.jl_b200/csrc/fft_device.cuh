@@ -74,7 +74,11 @@ __device__ __forceinline__ void bfly_put(const cplx_t<T>* v, cplx_t<T>* out, con
 // (j, k) lie in shared memory, PRIME_K neighbours at a time (a broadcast read
 // at a fixed offset each; one table of p roots with the index j k mod p kept
 // by additions spent more instructions on indices than on arithmetic); larger
-// primes use the table of roots.
+// primes use the table of roots.  Five pairs a thread divide those of 11, 31 and
+// 41; a last group that is not full computes the rest for nothing.  A'A in FP64 on
+// B200 with 3 / 4 / 5 / 6 pairs, us: 310x410x410 (31, 41) 2190 / 2099 / 1946 / 2040,
+// 984^2 (41) 59 / 54 / 54 / 59, 952^2 (17) 49 / 45 / 46 / 48, 988^2 (19) 56 / 58 / 55 /
+// 53, 936^2 (13) 49 / 50 / 51 / 45, 130^3 (13) 81 / 86 / 102 / 85.
 constexpr int PRIME_K = 5;
 constexpr int PRIME_MAT = 64;
 

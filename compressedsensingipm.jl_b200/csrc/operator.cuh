@@ -3,12 +3,12 @@
 //
 // Layout in HBM: one half spectrum (M1+1) x N2 x N3 of complex values, dim 1
 // fastest, pitch ld1; the mask as one bit per real sample, rows of N1 bits
-// padded to 32-bit words.  Pass structure (3D; 2D drops the dim-3 passes, 1D is
-// a single row pass):
+// padded to 32-bit words.  Pass structure (3D; 2D drops the dim-3 passes; 1D
+// rows take one or three launches, long1d.cuh):
 //
-//   A^T A x :  [gather x -> inverse FFT dim 3] -> [inverse dim 2]
+//   A^T A x :  [gather x -> inverse FFT dim 2] -> [inverse dim 3]
 //              -> [row: C2R dim 1, scale, mask, R2C dim 1]
-//              -> [forward dim 2] -> [forward dim 3 -> scatter + epilogue]
+//              -> [forward dim 3] -> [forward dim 2 -> scatter + epilogue]
 //
 // The beta -> spectrum gather is fused into the first pass and the
 // spectrum -> beta scatter (plus any elementwise epilogue, e.g. the CG's
@@ -88,6 +88,9 @@ __device__ __forceinline__ void pdl_enter() {
 // early (B200, us): 1D 4096 21.6 -> 18.2, 131072 28.7 -> 25.4, 259200 32.2 ->
 // 30.0, 524288 41.0 -> 53.1; 256^2 22.6 -> 17.7, 1024^2 46.6 -> 41.4; 64^3 30.8
 // -> 22.8, 160^3 115 -> 105, 256^3 384 -> 398.
+// Element kernels take one border in every dimension: with the 1D one for them
+// too, 1D recoveries by plain launches lost (FP64, ms, as it is -> with 2^18:
+// 524288 3.61 -> 3.90, 777600 4.67 -> 4.87, 2^20 4.82 -> 4.95).
 inline bool pdl_pays(int dim, long long N) { return N <= (dim == 1 ? 1LL << 18 : 1LL << 22); }
 
 // Not inside a capture: a graph's kernels already follow one another closely,

@@ -7,10 +7,10 @@
 // instruction issue and shared-memory latency at 512 (FP64) threads per SM,
 // then HBM.  Measured on B200 against the former passes (radices up to 8,
 // every stage and load through shared memory, run-time index division, primes
-// as direct sums), A'A product in FP64: 310 x 410 x 410 (primes 31 and 41)
-// 10.64 -> 1.95 ms, the synthesis and analysis of a 1024^2 image 84 -> 51 us,
-// 1D 777600 137 -> 61 us, 1D 4096 26.7 -> 21.8 us; condensed KKT product at
-// 256^3 1.38 -> 0.64 ms; a batch of 16 images of sides 128-256 11.7 -> 8.5 ms.
+// as direct sums), queued one after another in FP64: A'A 310 x 410 x 410 (primes
+// 31 and 41) 10.64 -> 1.96 ms, the synthesis and analysis of a 1024^2 image 85 ->
+// 46 us, A'A 1D 777600 137 -> 58 us; condensed KKT product at 256^3 1.40 -> 0.63
+// ms; a batch of 16 images of sides 128-256 11.7 -> 7.4 ms.
 // 80 registers (768 threads per SM) measured 8-21% slower on the 1D and 2D
 // passes than 128 (512 threads).
 #pragma once
@@ -82,7 +82,11 @@ __device__ __forceinline__ void strided_pass_kernel_body(const PassArgs<T>& a, c
 
 // Threads per CTA at most, and the CTAs per SM the register allocation must
 // allow: a radix-10 butterfly holds 40 (FP64) or 20 (FP32) registers of data and as
-// many of twiddles.
+// many of twiddles.  FP32 at 64 registers (2 CTAs; 24-72 bytes of stack in the
+// strided kernels) against 128 (1 CTA), mixed recoveries on B200, ms: 442x494
+// 2.35 / 2.26, 598x758 5.21 / 4.45, 1000x1022 3.66 / 3.50, 94^3 3.61 / 3.52, 100^3
+// 2.57 / 2.57, 130^3 6.30 / 6.41, 1D 777600 3.45 / 3.51: the border between them
+// lies with the lengths and is not drawn.
 constexpr int PASS_THREADS = 512;
 template <typename T> constexpr int pass_min_ctas() { return sizeof(T) == 8 ? 1 : 2; }
 

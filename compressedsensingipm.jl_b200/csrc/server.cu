@@ -46,8 +46,8 @@ struct Pending {
     Clock::time_point t_submit;
 };
 
-// dimension count, long-row 1D passes (half-length above the one-CTA row
-// pass's limit), missing samples or not
+// dimension count, 1D half-length above 2048 or not (the classes of
+// csipm_solve_batch), missing samples or not
 int batch_class(const csipm_problem& p) {
     const bool long1d = p.dim == 1 && p.size[0] / 2 > csipm::L1D_MIN_M;
     return p.dim * 4 + (long1d ? 2 : 0) + (p.n_missing > 0 ? 1 : 0);
@@ -79,7 +79,7 @@ struct csipm_server_s {
 namespace csipm_internal {
 
 // Device bytes csipm_create allocates for a problem (the handle's vectors,
-// spectra, mask, plane map and reduction workspace), plus the two N-vectors
+// spectra, mask and reduction workspace), plus the two N-vectors
 // the server stages z0 and beta in.
 size_t footprint_bytes(int dim, const int* size, int precision, int64_t n_missing) {
     const long long n1 = size[0], n2 = dim >= 2 ? size[1] : 1, n3 = dim >= 3 ? size[2] : 1;
@@ -90,7 +90,6 @@ size_t footprint_bytes(int dim, const int* size, int precision, int64_t n_missin
     b += 16 * Nh;                                 // FP64 spectrum
     if (precision == CSIPM_MIXED) b += 8 * 4 * N + 8 * Nh;   // FP32 CG vectors and directions + FP32 spectrum
     if (n_missing > 0) b += (size_t)((n1 + 31) / 32) * 4 * (size_t)(n2 * n3) * (precision == CSIPM_MIXED ? 2 : 1);
-    b += 2 * 16 * (size_t)(n2 * n3);              // headroom (twiddle tables of long axes)
     b += 8 * 8 * 65536 + (1 << 20);               // reduction partials, slots, twiddles (upper bound)
     b += 2 * 8 * N;                               // the server's z0 / beta staging
     return b;

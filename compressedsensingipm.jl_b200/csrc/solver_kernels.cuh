@@ -811,17 +811,6 @@ static __global__ void convert_kernel(long long n, const TA* __restrict__ a, TB*
     CSIPM_GRID_LOOP(i, n) b[i] = (TB)a[i];
 }
 
-static __global__ void axpy_kernel(long long n, double alpha, const double* __restrict__ x, double* __restrict__ y) {
-    pdl_enter();
-    CSIPM_GRID_LOOP(i, n) y[i] += alpha * x[i];
-}
-
-// y = x - y  (residual r = rhs - Kx in place on y)
-static __global__ void sub_from_kernel(long long n, const double* __restrict__ x, double* __restrict__ y) {
-    pdl_enter();
-    CSIPM_GRID_LOOP(i, n) y[i] = x[i] - y[i];
-}
-
 // dot products on the device
 static __global__ void dot2_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b,
                             const double* __restrict__ c2, const double* __restrict__ d2, RedWorkspace ws) {
