@@ -484,7 +484,7 @@ def run_ours(args):
     rp_gbs = rp_bytes / rp_ms / 1e6
     roofline = {
         "bound": "hbm",
-        "kernel": "ipm_resdiag_kernel (residual pass: pending step, residual, barrier diagonals, predictor rhs)",
+        "kernel": "ipm_resdiag_kernel (residual pass: pending step, residual, barrier diagonals, start of the predictor CG)",
         "achieved": round(rp_gbs, 1),
         "peak": peak,
         "peak_kind": f"{peak_kind} copy bandwidth (the kernel is timed inside the solve)",
