@@ -101,7 +101,8 @@ typedef struct {
                                   lines / rows per CTA) once per process and keeps the fastest;
                                   with the environment variable CSIPM_TUNE_CACHE naming a file, the
                                   choices persist there (one JSON object per line) and later
-                                  processes start from them; 0: the built-in heuristic */
+                                  processes start from them (choices made for other kernels than
+                                  this library's are passed over); 0: the built-in heuristic */
     double ipm_cg_forcing;     /* csipm_solve: forcing term of the inexact Newton solves.  Iteration k
                                   solves to min(ipm_cg_rtol, max(1e-6, ipm_cg_forcing * gap[k-1]))
                                   with gap[k-1] the previous iteration's relative duality gap, so
